@@ -668,12 +668,6 @@ __global__ void __launch_bounds__(128) k_mem_nodeforce(MembraneArgs A) {
 // sorted position whose bin is >= b, and the nodes in (bin, node) order.  The
 // last CTA of the launch writes the prefix of patch cells over the membranes
 // (the spread kernel's work list).
-// The membrane's nodes in sorted order (global node indices): the spread reads
-// each contribution's stencil weights and force through it.
-__device__ __forceinline__ void write_sorted_nodes(const MembraneArgs &A, const MembraneConst &mc, const int *list) {
-    for (int e = threadIdx.x; e < mc.n_nodes; e += blockDim.x) A.sorted_node[mc.node0 + e] = mc.node0 + list[e];
-}
-
 // Exclusive prefix sum of one int per thread over the CTA, and the CTA's
 // total: a shuffle scan within each warp, the warp totals scanned by warp 0,
 // two barriers (in place of a Hillis-Steele scan over the whole CTA, whose
@@ -887,23 +881,18 @@ __device__ void sort_patch(const MembraneArgs &A, int m, const double *red, bool
     int *cur = in_smem ? cnt : cursor;
     for (int ln = threadIdx.x; ln < mc.n_nodes; ln += blockDim.x) list[atomicAdd(cur + bins[ln], 1)] = ln;
     __syncthreads();
-    // each bin in node-index order; after the placement cur[b] is the end of
-    // bin b, the start of bin b + 1
-    for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
+    // each bin in node-index order: a node's place is the number of smaller indices in its bin
+    // (after the placement cur[b] is the end of bin b, the start of bin b + 1), one thread per node.
+    // Bins are full where a membrane is fine against the grid: an insertion sort by one thread per
+    // bin was quadratic in a serial chain there (49 membranes of radius 1.5 to 4 cells: 57.8 us).
+    for (int ln = threadIdx.x; ln < mc.n_nodes; ln += blockDim.x) {
+        const int b = bins[ln];
         const int lo = b == 0 ? 0 : (in_smem ? cur[b - 1] : __ldcg(cur + b - 1));
         const int hi = in_smem ? cur[b] : __ldcg(cur + b);  // global cursors were moved by atomics
-        for (int i = lo + 1; i < hi; i++) {
-            const int v = list[i];
-            int j = i - 1;
-            while (j >= lo && list[j] > v) {
-                list[j + 1] = list[j];
-                j--;
-            }
-            list[j + 1] = v;
-        }
+        int place = lo;
+        for (int i = lo; i < hi; i++) place += list[i] < ln ? 1 : 0;
+        A.sorted_node[mc.node0 + place] = mc.node0 + ln;
     }
-    __syncthreads();
-    write_sorted_nodes(A, mc, list);
 }
 
 constexpr int kSortThreads = kMembraneThreads;

@@ -133,6 +133,43 @@ def compare_with_oracle(c, steps, fields=True):
     o.close()
 
 
+@pytest.mark.parametrize("level,radius,ibm", [(3, 1.5, "PESKIN4"), (4, 1.5, "HAT2"), (4, 3.0, "PESKIN4")])
+def test_spread_of_full_sort_bins(level, radius, ibm):
+    # membranes fine against the grid: tens of nodes share a stencil bin (642 and 2562 nodes: one and
+    # three per thread of the node sort).  The force field against the sum over the handle's own nodes
+    # and forces: at most 2562 terms a cell, so the sums' rounding is below 2562 eps = 6e-13 of the
+    # sum of magnitudes; and two handles agree bit for bit whatever order the placement took.
+    c = cases.shear_rbc(n=20, level=level, radius_cells=radius, rotate=True,
+                        ibm_stencil=getattr(_abi, "LBFS_IBM_" + ibm))
+    fields = []
+    for _ in range(2):
+        s = make(c)
+        s.step(3)
+        fields.append(s.field(_abi.LBFS_FIELD_FORCE).reshape(-1, 3))
+        x, f = s.nodes(), s.nodes(_abi.LBFS_NODES_FORCE)
+        assert s.status() == 0
+        s.close()
+    assert np.array_equal(fields[0], fields[1])
+    n, r = 20, x / 2.0
+    width = 2 if ibm == "HAT2" else 4
+    base = (np.round(r) - 1 if width == 2 else np.floor(r - 0.5) - 1).astype(int)
+    cells = base[:, :, None] + np.arange(width)
+    d = np.abs(cells + 0.5 - r[:, :, None])
+    near, far = np.minimum(d, 1.0), np.clip(d, 1.0, 2.0)
+    w = 1 - d if width == 2 else np.where(
+        d < 1, (3 - 2 * near + np.sqrt(1 + 4 * near - 4 * near * near)) / 8,
+        np.where(d < 2, (5 - 2 * far - np.sqrt(-7 + 12 * far - 4 * far * far)) / 8, 0.0))
+    want, size = np.zeros((n ** 3, 3)), np.zeros((n ** 3, 3))
+    for i in range(width):
+        for j in range(width):
+            for k in range(width):
+                at = cells[:, 0, i] + n * (cells[:, 1, j] + n * cells[:, 2, k])
+                v = f * (w[:, 0, i] * w[:, 1, j] * w[:, 2, k] / 8.0)[:, None]
+                np.add.at(want, at, v)
+                np.add.at(size, at, np.abs(v))
+    assert np.max(np.abs(fields[0] - want)) <= 1e-12 * size.max()
+
+
 def test_interior_viscosity_l4_vs_oracle():
     # the binned interior-viscosity test (triangles binned by their y-z boxes) against the oracle's
     # test of every triangle: a rotated L4 cell (5120 triangles over many bins), 805 cells inside;
