@@ -218,6 +218,15 @@ def algorithmic_bytes(mesh, phase, fp64=True):
         # parameters: no per-face geometry
         geo = 0 if axis_geometry_uniform(mesh) else 4 * R
         return ni * (8 + 4 * R + geo) + nb * (16 + 29 * R) + nc * (17 * R) + nb * (16 * R)
+    if phase == "fluid_pass":
+        # the fused pass of uniform meshes.  Per cell: state in 4R, viscosity factor R, 1 / volume 8, the
+        # state kept 4R and the cell sums 32 out; per bc face: ids 8, geometry 12R, types/values 8 + 4R,
+        # record 9R, flux out 4R
+        return nc * (40 + 9 * R) + nb * (16 + 29 * R)
+    if phase == "fluid_update":
+        # the update behind it.  Per cell: cell sums 32 and a byte in, volume 8, t1 in/out 64, state out
+        # 4R; per bc face: flux in 4R, the owner's face list 24
+        return nc * (105 + 4 * R) + nb * (24 + 4 * R)
     if phase == "gradients":
         # per cell: stencil 24, folded weights 18R (or their 3-bit codes, 4, on a mesh with at most 8
         # distinct weight vectors), state 4R, gradients out 12R;
@@ -820,13 +829,18 @@ def main():
     phases = {name: phase_sum[i] / K for i, name in enumerate(["membrane", "gradients", "flux", "update"])}
     status = s.status()
 
-    # roofline of the dominant fluid kernel (the membrane kernel overlaps them on a second stream)
-    fluid = {k: v for k, v in phases.items() if k != "membrane"}
+    # roofline of the dominant fluid kernel (the membrane kernel overlaps them on a second stream).  On
+    # uniform meshes gradients and fluxes are one kernel (no gradient phase is recorded)
+    fused = phases["gradients"] == 0.0
+    kernels = ({"flux": ("fluid_pass", "k_uniform_step"), "update": ("fluid_update", "k_cell_update")} if fused else
+               {"gradients": ("gradients", "k_cell_gradients"), "flux": ("flux", "k_face_flux"),
+                "update": ("update", "k_cell_update")})
+    fluid = {k: phases[k] for k in kernels}
     dom = max(fluid, key=fluid.get)
     peaks, peak_kind = measured_peaks()
-    alg = algorithmic_bytes(mesh, dom)
+    alg = algorithmic_bytes(mesh, kernels[dom][0])
     achieved = alg / (fluid[dom] * 1e-3) / 1e9
-    kname = {"flux": "k_face_flux", "gradients": "k_cell_gradients", "update": "k_cell_update"}[dom]
+    kname = kernels[dom][1]
     traffic = read_traffic(kname, f"shear_rbc_{args.n}_fp64")
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "peak_source": peak_kind,
@@ -834,8 +848,8 @@ def main():
                 "timing": "per-kernel CUDA events, second timed pass of K steps with K1 and K2 not pipelined"}
     # every fluid kernel against the same HBM peak (algorithmic bytes / event-timed duration)
     kernel_roofline = {}
-    for ph, kn in (("gradients", "k_cell_gradients"), ("flux", "k_face_flux"), ("update", "k_cell_update")):
-        b_ = algorithmic_bytes(mesh, ph)
+    for ph, (kind, kn) in kernels.items():
+        b_ = algorithmic_bytes(mesh, kind)
         gbs = b_ / (fluid[ph] * 1e-3) / 1e9
         kernel_roofline[kn] = {"algorithmic_bytes": b_, "ms": fluid[ph], "achieved_gbs": gbs,
                                "frac": gbs / peaks["hbm_gbs"],

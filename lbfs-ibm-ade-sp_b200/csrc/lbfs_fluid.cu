@@ -4,46 +4,15 @@
 
 #include <algorithm>
 
+#include "lbfs_face.cuh"
 #include "lbfs_fluid.cuh"
 #include "lbfs_internal.h"
 #include "lbfs_kernels.h"
 
 namespace lbfs {
 
-// ------------------------------------------------------------------ K1 ----
 
-// Ghost-cell macros from the owner state (update_unstructured_bcs,
-// LBFS.cu:1868-1918).  Type 3 (periodic) takes the partner cell's state, as
-// the reference's CPU solver does (Solution::update_unstructured_bcs,
-// Solution.cpp:777-803).  Types outside {1,2,3} / {1,2,3,9,10} are rejected at
-// creation, so every branch here assigns.
-template <typename R>
-__device__ __forceinline__ Vec4<R> ghost_state(const FluidArgs<R> &a, int b, const Vec4<R> &own) {
-    const Vec4<R> bc = a.bc_val[b];
-    Vec4<R> g;
-    const int rt = a.bc_rho_type[b], vt = a.bc_vel_type[b];
-    const Vec4<R> p = (rt == 3 || vt == 3) ? a.state[a.bc_periodic[b]] : own;
-    if (rt == 1) g.rho = bc.rho - (own.rho - bc.rho);
-    else if (rt == 2) g.rho = own.rho;
-    else g.rho = p.rho;
-    if (vt == 3) {
-        g.u = p.u; g.v = p.v; g.w = p.w;
-    } else if (vt == 2) {
-        g.u = own.u; g.v = own.v; g.w = own.w;
-    } else {
-        R ut = bc.u;
-        if (vt == 9) {
-            const BcRec<R> r = a.bc_rec[b];
-            ut = (R)(16 * (double)bc.u * (a.H2 + r.gy) * (a.H2 - r.gy) * (a.H2 + r.gz) * (a.H2 - r.gz) / a.H4);
-        } else if (vt == 10) {
-            ut = a.bc_rec[b].gy * bc.u;
-        }
-        g.u = ut - (own.u - ut);
-        g.v = bc.v - (own.v - bc.v);
-        g.w = bc.w - (own.w - bc.w);
-    }
-    return g;
-}
+// ------------------------------------------------------------------ K1 ----
 
 template <typename R, int TB>
 __global__ void __launch_bounds__(TB, TB == 128 ? 5 : 1) k_cell_gradients(FluidArgs<R> a, int begin, int end) {
@@ -51,585 +20,13 @@ __global__ void __launch_bounds__(TB, TB == 128 ? 5 : 1) k_cell_gradients(FluidA
     const int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= end) return;
     const Vec4<R> own = a.state[i];
-    int st[6];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        const int2 p = __ldg(a.stencil + 3 * i + q);
-        st[2 * q] = p.x;
-        st[2 * q + 1] = p.y;
-    }
-    LsW<R> W;
-    if (a.lsw_code) {  // the weights from the per-mesh table by the cell's six 3-bit codes
-        const unsigned code = __ldg(a.lsw_code + i);
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            const unsigned k = (code >> (3 * q)) & 7u;
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                R v = a.lsw_tab[0][r];
-#pragma unroll
-                for (unsigned t = 1; t < 8; t++) v = (k == t) ? a.lsw_tab[t][r] : v;
-                W.w[3 * q + r] = v;
-            }
-        }
-    } else {
-        W = a.lsw[i];
-    }
     GradRec<R> gr;
-    R *g = gr.g;
-#pragma unroll
-    for (int t = 0; t < 12; t++) g[t] = R(0);
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        const int j = st[q];
-        Vec4<R> s;
-        if (j < a.nc) {
-            s = a.state[j];
-        } else {
-            s = ghost_state(a, j - a.nc, own);
-        }
-        // add_LS_contributions (LBFS.cu:2051-2083) with LHS^-1 folded in
-        const R d[4] = {s.rho - own.rho, s.u - own.u, s.v - own.v, s.w - own.w};
-#pragma unroll
-        for (int m = 0; m < 4; m++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) g[3 * m + r] = g[3 * m + r] + W.w[3 * q + r] * d[m];
-    }
+    cell_gradient(a, i, own, gr.g);
     reinterpret_cast<GradRec<R> *>(a.grad)[i] = gr;
 }
 
 // ------------------------------------------------------------------ K2 ----
 
-// Density offset of the stored state: 0 in FP64 (a compile-time zero, so no
-// add is spent on it), rho0 in the FP32-bulk form.
-template <typename R> __device__ __forceinline__ R rho0_of(const FluidArgs<R> &a) {
-    if constexpr (sizeof(R) == 8) return R(0);
-    else return a.rho0;
-}
-
-// Lattice population divided by its weight, g_k = f_k / w_k, at a reconstructed
-// state L = (rho', u, v, w):  g = rho' + (rho' + rho0) X,
-// X = 3 e.u + q (4.5 (e.u)^2 - 1.5 |u|^2).  The reference's equilibrium
-// w_k rho (1 + X) (populate_feq_lattice_explicit, LBFS.cu:1041-1354; populate_feq,
-// LBFS.cu:940-1036 with the preconditioning factor q) with the weight applied
-// later, once per group of directions that share it.
-template <typename R>
-__device__ __forceinline__ R pop_g(const R (&L)[4], R eu, R rho0, R q) {
-    const R usq = L[1] * L[1] + L[2] * L[2] + L[3] * L[3];
-    const R X = R(3) * eu + q * (R(4.5) * eu * eu - R(1.5) * usq);
-    if constexpr (sizeof(R) == 8) return L[0] + L[0] * X;
-    else return L[0] + (L[0] + rho0) * X;
-}
-
-// FP32-bulk (deviation) form of pop_g at a reconstructed state written as
-// L = p0 + d, p0 the face-centre state and d the direction's small offset
-// from it.  The population's term 3 rho0 e.p0_u is large (the velocity
-// itself) and the same for every direction, so that summing the populations
-// over directions would cancel it and leave its FP32 rounding in the
-// cross-stream moments; it is left out here, and its moments (rho0 p0_u in
-// the first moment, zero in every other) are added once, exactly, by the
-// caller.  The rest is formed from small terms only:
-//   g~ = rho' (1 + X) + rho0 (3 e.d_u + q (4.5 (e.u)^2 - 1.5 |u|^2)).
-// eu = e.u at L, edu = e.d_u.
-__device__ __forceinline__ float pop_dev(const float (&L)[4], float eu, float edu, float rho0, float q) {
-    const float usq = L[1] * L[1] + L[2] * L[2] + L[3] * L[3];
-    const float Q = q * (4.5f * eu * eu - 1.5f * usq);
-    const float X = 3.0f * eu + Q;
-    return (L[0] + L[0] * X) + rho0 * (3.0f * edu + Q);
-}
-
-// Moments of the reconstructed lattice populations that the interface flux
-// needs: rho = sum f, m_c = sum e_c f, d_c = sum_{e_c != 0} f (= sum e_c e_c f),
-// o_xy, o_xz, o_yz = sum e_c e_m f.  Formed from sums and differences of
-// opposite directions (the D3Q15 set is symmetric), then weighted once per
-// group: a few dozen adds instead of one accumulation per direction and moment.
-template <typename R> struct LatMoments {
-    R rho, m[3], d[3], o[3];  // o: xy, xz, yz
-};
-template <typename R> __device__ __forceinline__ R o_of(const LatMoments<R> &M, int c, int q) {
-    // symmetric second moment e_c e_q for c != q
-    return (c + q == 1) ? M.o[0] : ((c + q == 2) ? M.o[1] : M.o[2]);
-}
-
-// Interface equilibrium, BGK relaxation towards the lattice populations and
-// the flux through the face: calculate_flux_at_interface (LBFS.cu:1462-1648)
-// and its axis-aligned forms (LBFS.cu:3648-4092).  The relaxed populations are
-// f_k - tau (f_k - fl_k), f_k the interface equilibrium, so the flux tensor is
-// (1 - tau) F_eq + tau F_fl, F_fl the moments of the lattice populations fl_k.
-// The D3Q15 weights make the equilibrium moments exact closed forms
-// (sum w e = 0, sum w e e = I / 3, sum w e e e e = (dd + dd + dd) / 9):
-//   sum_k e_c f_k = rho u_c = m_c,  sum_k e_c e_q f_k = q_s m_c m_q / rho + d_cq rho' / 3
-// (q_s the preconditioning factor; in the deviation form the d_cq term is
-// rho' / 3).  So the mass flux is m . n exactly, and the momentum flux is
-// formed from the six distinct second moments.  The reference sums the 15
-// equilibria explicitly; the closed form is the same quantity with fewer
-// roundings.  `axis` >= 0: only the face-normal component (axis-aligned faces,
-// n = e_axis); `axis` < 0: all three with the face normal.
-template <typename R>
-__device__ __forceinline__ Vec4<R> interface_flux(const LatMoments<R> &M, R rho0, R tau, R qscale, R area, int axis,
-                                                  R nx, R ny, R nz) {
-    const R rho_i = M.rho + rho0;
-    const R inv = R(1) / rho_i;
-    const R keep = R(1) - tau;
-    const R third = M.rho * R(1.0 / 3.0);
-    // relaxed second moment c, q
-    auto T = [&](int c, int q) -> R {
-        R eq = qscale * (M.m[c] * inv) * M.m[q];
-        R fl;
-        if (c == q) {
-            eq = eq + third;
-            fl = M.d[c];
-        } else {
-            fl = o_of(M, c, q);
-        }
-        return keep * eq + tau * fl;
-    };
-    Vec4<R> out;
-    if (axis >= 0) {
-        out.rho = M.m[axis] * area;
-        out.u = T(axis, 0) * area;
-        out.v = T(axis, 1) * area;
-        out.w = T(axis, 2) * area;
-    } else {
-        const R Txx = T(0, 0), Tyy = T(1, 1), Tzz = T(2, 2), Txy = T(0, 1), Txz = T(0, 2), Tyz = T(1, 2);
-        out.rho = (M.m[0] * nx + M.m[1] * ny + M.m[2] * nz) * area;
-        out.u = (Txx * nx + Txy * ny + Txz * nz) * area;
-        out.v = (Txy * nx + Tyy * ny + Tyz * nz) * area;
-        out.w = (Txz * nx + Tyz * ny + Tzz * nz) * area;
-    }
-    return out;
-}
-
-struct Dir {
-    int ex, ey, ez;
-};
-__device__ __forceinline__ Dir dir_of(int k) { return {c_ex(k), c_ey(k), c_ez(k)}; }
-
-template <typename R> __device__ __forceinline__ void load_grad(const R *g, R (&o)[12]) {
-    const GradRec<R> r = *reinterpret_cast<const GradRec<R> *>(g);
-#pragma unroll
-    for (int t = 0; t < 12; t++) o[t] = r.g[t];
-}
-
-// The five directions of one side of an axis-A face: e_A = s (s = +1 owner
-// side, -1 neighbour side) with (e_B, e_C) in {(0,0), (+,+), (+,-), (-,+), (-,-)}
-// (B < C the other two axes).  populate_lattice_macros_uniform_{x,y,z}
-// (LBFS.cu:2939-3644): the lattice node sits at x_f - e dt and is extrapolated
-// from the side's cell: L = p - dt (e . g).  With a = p - s dt g_A,
-// b = dt g_B, c = dt g_C the four corners are (a -+ b) -+ c.  Returns the
-// side's weighted sums S = sum f, YB = sum e_B f, YC = sum e_C f.
-template <typename R, int A>
-__device__ __forceinline__ void axis_side(const R (&p)[4], const R (&g)[12], R s, R dt, R rho0, R &S, R &YB,
-                                          R &YC) {
-    constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    R av[4], amb[4], apb[4], cv[4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        av[m] = p[m] - s * dt * g[3 * m + A];
-        const R b = dt * g[3 * m + B];
-        cv[m] = dt * g[3 * m + C];
-        amb[m] = av[m] - b;  // e_B = +1
-        apb[m] = av[m] + b;  // e_B = -1
-    }
-    // e = (s e_A, e_B, e_C) in (A, B, C) order; e.u = s u_A + e_B u_B + e_C u_C
-    const R g0 = pop_g<R>(av, s * av[1 + A], rho0, R(1));
-    R Lc[4], gpp, gpm, gmp, gmm;
-#pragma unroll
-    for (int m = 0; m < 4; m++) Lc[m] = amb[m] - cv[m];
-    gpp = pop_g<R>(Lc, s * Lc[1 + A] + Lc[1 + B] + Lc[1 + C], rho0, R(1));
-#pragma unroll
-    for (int m = 0; m < 4; m++) Lc[m] = amb[m] + cv[m];
-    gpm = pop_g<R>(Lc, s * Lc[1 + A] + Lc[1 + B] - Lc[1 + C], rho0, R(1));
-#pragma unroll
-    for (int m = 0; m < 4; m++) Lc[m] = apb[m] - cv[m];
-    gmp = pop_g<R>(Lc, s * Lc[1 + A] - Lc[1 + B] + Lc[1 + C], rho0, R(1));
-#pragma unroll
-    for (int m = 0; m < 4; m++) Lc[m] = apb[m] + cv[m];
-    gmm = pop_g<R>(Lc, s * Lc[1 + A] - Lc[1 + B] - Lc[1 + C], rho0, R(1));
-    const R bp = gpp + gpm, bm = gmp + gmm, cp = gpp - gpm, cm = gmp - gmm;
-    constexpr R w_axis = R(1.0 / 9.0), w_corner = R(1.0 / 72.0);
-    S = w_axis * g0 + w_corner * (bp + bm);
-    YB = w_corner * (bp - bm);
-    YC = w_corner * (cp + cm);
-}
-
-// The same five directions in the deviation form: the side's offsets from
-// the face centre, d = s (hdp - dt g_A) -+ dt g_B -+ dt g_C (hdp half the
-// owner-neighbour difference of the reconstructed states), and L = p0 + d.
-template <int A>
-__device__ __forceinline__ void axis_side_dev(const float (&p0)[4], const float (&hdp)[4], const float (&g)[12],
-                                              float s, float dt, float rho0, float &S, float &YB, float &YC) {
-    constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    float ad[4], amb[4], apb[4], cv[4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        ad[m] = s * (hdp[m] - dt * g[3 * m + A]);
-        const float b = dt * g[3 * m + B];
-        cv[m] = dt * g[3 * m + C];
-        amb[m] = ad[m] - b;
-        apb[m] = ad[m] + b;
-    }
-    float L[4], d[4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) L[m] = p0[m] + ad[m];
-    const float g0 = pop_dev(L, s * L[1 + A], s * ad[1 + A], rho0, 1.0f);
-    float gq[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const float eb = (q < 2) ? 1.0f : -1.0f, ec = (q & 1) ? -1.0f : 1.0f;  // (+,+), (+,-), (-,+), (-,-)
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            d[m] = ((q < 2) ? amb[m] : apb[m]) - ec * cv[m];
-            L[m] = p0[m] + d[m];
-        }
-        gq[q] = pop_dev(L, s * L[1 + A] + eb * L[1 + B] + ec * L[1 + C], s * d[1 + A] + eb * d[1 + B] + ec * d[1 + C],
-                        rho0, 1.0f);
-    }
-    const float bp = gq[0] + gq[1], bm = gq[2] + gq[3], cp = gq[0] - gq[1], cm = gq[2] - gq[3];
-    S = (1.0f / 9.0f) * g0 + (1.0f / 72.0f) * (bp + bm);
-    YB = (1.0f / 72.0f) * (bp - bm);
-    YC = (1.0f / 72.0f) * (cp + cm);
-}
-
-// Axis-aligned interior face of axis A (calc_face_flux_x/_y/_z, LBFS.cu:2283-2569):
-// directions with e_A = +1 extrapolate from the owner, -1 from the neighbour,
-// 0 from the face centre with the distance-weighted gradient.
-template <typename R, int A>
-__device__ __forceinline__ Vec4<R> axis_face_flux(const FluidArgs<R> &a, int f) {
-    constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    const int2 oc = __ldg(a.face_cells + f);
-    AxisFace<R> geo;
-    R wa, wb;
-    if (a.axis_uniform) {
-        geo = {a.axis_geo[A][0], a.axis_geo[A][1], a.axis_geo[A][2], a.axis_geo[A][3]};
-        wa = a.axis_wa[A];
-        wb = a.axis_wb[A];
-    } else {
-        geo = a.axis_face[f];
-        const R ic = R(1) / (geo.t2 - geo.t1);
-        wa = fabs(geo.t2 * ic);
-        wb = fabs(geo.t1 * ic);
-    }
-    const Vec4<R> s1 = a.state[oc.x], s2 = a.state[oc.y];
-    R g1[12], g2[12];
-    load_grad(a.grad + (size_t)12 * oc.x, g1);
-    load_grad(a.grad + (size_t)12 * oc.y, g2);
-    const R rho0 = rho0_of(a);
-    const R dt = geo.dt, t1 = geo.t1, t2 = geo.t2;
-    const R S1[4] = {s1.rho, s1.u, s1.v, s1.w}, S2[4] = {s2.rho, s2.u, s2.v, s2.w};
-    R pi[4], pn[4], p0[4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        pi[m] = S1[m] - t1 * g1[3 * m + A];
-        pn[m] = S2[m] - t2 * g2[3 * m + A];
-        p0[m] = (pi[m] + pn[m]) * R(0.5);
-    }
-    LatMoments<R> M;
-    R Sp, Bp, Cp, Sn, Bn, Cn;
-    if constexpr (sizeof(R) == 8) {
-        axis_side<R, A>(pi, g1, R(1), dt, rho0, Sp, Bp, Cp);
-        axis_side<R, A>(pn, g2, R(-1), dt, rho0, Sn, Bn, Cn);
-    } else {
-        // half the owner-neighbour difference, from the states' difference (exact for close values)
-        R hdp[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) hdp[m] = ((S1[m] - S2[m]) - (t1 * g1[3 * m + A] - t2 * g2[3 * m + A])) * R(0.5);
-        axis_side_dev<A>(p0, hdp, g1, 1.0f, dt, rho0, Sp, Bp, Cp);
-        axis_side_dev<A>(p0, hdp, g2, -1.0f, dt, rho0, Sn, Bn, Cn);
-    }
-    // centre directions (e_A = 0): rest, +-B, +-C, from p0 with gi = wa g1 + wb g2
-    R gz0, gbp, gbm, gcp, gcm;
-    if constexpr (sizeof(R) == 4) {
-        R bv[4], cv[4], L[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            bv[m] = dt * (g1[3 * m + B] * wa + g2[3 * m + B] * wb);
-            cv[m] = dt * (g1[3 * m + C] * wa + g2[3 * m + C] * wb);
-        }
-        gz0 = pop_dev(p0, R(0), R(0), rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] - bv[m];
-        gbp = pop_dev(L, L[1 + B], -bv[1 + B], rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] + bv[m];
-        gbm = pop_dev(L, -L[1 + B], -bv[1 + B], rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] - cv[m];
-        gcp = pop_dev(L, L[1 + C], -cv[1 + C], rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] + cv[m];
-        gcm = pop_dev(L, -L[1 + C], -cv[1 + C], rho0, R(1));
-    } else {
-        R bv[4], cv[4], L[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            bv[m] = dt * (g1[3 * m + B] * wa + g2[3 * m + B] * wb);
-            cv[m] = dt * (g1[3 * m + C] * wa + g2[3 * m + C] * wb);
-        }
-        gz0 = pop_g<R>(p0, R(0), rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] - bv[m];
-        gbp = pop_g<R>(L, L[1 + B], rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] + bv[m];
-        gbm = pop_g<R>(L, -L[1 + B], rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] - cv[m];
-        gcp = pop_g<R>(L, L[1 + C], rho0, R(1));
-#pragma unroll
-        for (int m = 0; m < 4; m++) L[m] = p0[m] + cv[m];
-        gcm = pop_g<R>(L, -L[1 + C], rho0, R(1));
-    }
-    constexpr R w_rest = R(2.0 / 9.0), w_axis = R(1.0 / 9.0);
-    const R Sz = w_rest * gz0 + w_axis * ((gbp + gbm) + (gcp + gcm));
-    const R Bz = w_axis * (gbp - gbm), Cz = w_axis * (gcp - gcm);
-    M.rho = (Sp + Sn) + Sz;
-    M.m[A] = Sp - Sn;
-    M.d[A] = Sp + Sn;
-    M.m[B] = (Bp + Bn) + Bz;
-    M.m[C] = (Cp + Cn) + Cz;
-    M.o[A + B - 1] = Bp - Bn;  // o index of the pair (A, B): xy 0, xz 1, yz 2
-    M.o[A + C - 1] = Cp - Cn;
-    M.d[B] = M.d[C] = M.o[B + C - 1] = R(0);  // not read by the axis-A flux
-    if constexpr (sizeof(R) == 4) {
-        // first moments of the left-out term 3 rho0 e.p0_u (pop_dev)
-#pragma unroll
-        for (int c = 0; c < 3; c++) M.m[c] = M.m[c] + rho0 * p0[1 + c];
-    }
-    const R vf = a.visc_factor[oc.x];
-    const R tau = (a.testcase == 8) ? R(0) : (a.visc * vf * R(3) / dt * a.gamma_inv);
-    return interface_flux<R>(M, rho0, tau, R(1), geo.area, A, 0, 0, 0);
-}
-
-// General face: populate_lattice_macros (LBFS.cu:323-936).  Boundary faces
-// take the boundary branch except the face of the first ghost (LBFS.cu tests
-// neighbour > n_cells), which the host marks per instance in bc_branch.
-// Ghost of boundary face f (ghost cell g = its neighbour): its state
-// (update_unstructured_bcs, LBFS.cu:1843-1928) and its gradients
-// (get_bc_gradients, LBFS.cu:1933-2048): Dirichlet components the difference
-// to the owner over the owner-ghost distance along that direction, the others
-// the owner's gradient without its face-normal part; a periodic component
-// (type 3) the partner cell's gradient (gradients::Get_LS_Gradients,
-// gradients.cpp:428-440).  Formed here, once every cell's gradients exist,
-// and stored in the ghost's records for the fields and the adjoint.
-template <typename R>
-__device__ __forceinline__ void boundary_ghost(const FluidArgs<R> &a, int g, const Vec4<R> &own, const R (&go)[12],
-                                               Vec4<R> &gs, R (&gg)[12]) {
-    const int b = g - a.nc;
-    gs = ghost_state(a, b, own);
-    const BcRec<R> r = a.bc_rec[b];
-    const int rt = a.bc_rho_type[b], vt = a.bc_vel_type[b];
-    const R d[4] = {gs.rho - own.rho, gs.u - own.u, gs.v - own.v, gs.w - own.w};
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const bool dirichlet = (m == 0) ? rt == 1 : (vt != 2 && vt != 3);
-        if (dirichlet) {
-            gg[3 * m + 0] = d[m] / r.dmag * r.dnx;
-            gg[3 * m + 1] = d[m] / r.dmag * r.dny;
-            gg[3 * m + 2] = d[m] / r.dmag * r.dnz;
-        } else {
-            gg[3 * m + 0] = go[3 * m + 0] * r.mx;
-            gg[3 * m + 1] = go[3 * m + 1] * r.my;
-            gg[3 * m + 2] = go[3 * m + 2] * r.mz;
-        }
-    }
-    if (rt == 3 || vt == 3) {
-        R gp[12];
-        load_grad(a.grad + (size_t)12 * a.bc_periodic[b], gp);
-#pragma unroll
-        for (int t = 0; t < 12; t++)
-            if ((t < 3) ? rt == 3 : vt == 3) gg[t] = gp[t];
-    }
-    a.state[g] = gs;
-    GradRec<R> gr;
-#pragma unroll
-    for (int t = 0; t < 12; t++) gr.g[t] = gg[t];
-    reinterpret_cast<GradRec<R> *>(a.grad)[g] = gr;
-}
-
-template <typename R>
-__device__ __forceinline__ Vec4<R> general_face_flux(const FluidArgs<R> &a, int f, bool is_bc) {
-    const int2 oc = __ldg(a.face_cells + f);
-    const GenFace<R> geo = a.gen_face[a.axis_aligned ? f - a.ni : f];
-    const Vec4<R> s1 = a.state[oc.x];
-    const R rho0 = rho0_of(a);
-    Vec4<R> s2;
-    R g1[12], g2[12];
-    load_grad(a.grad + (size_t)12 * oc.x, g1);
-    if (is_bc) {
-        boundary_ghost(a, oc.y, s1, g1, s2, g2);
-    } else {
-        s2 = a.state[oc.y];
-        load_grad(a.grad + (size_t)12 * oc.y, g2);
-    }
-    const R dt = geo.dt;
-    const R S1[4] = {s1.rho, s1.u, s1.v, s1.w}, S2[4] = {s2.rho, s2.u, s2.v, s2.w};
-    R pi[4], pn[4], p0[4];
-    if (geo.bc_branch != R(0)) {
-        const int b = oc.y - a.nc;
-        const Vec4<R> bc = a.bc_val[b];
-        const bool rd = a.bc_rho_type[b] == 1, vd = a.bc_vel_type[b] == 1;
-        const R bcv[4] = {bc.rho, bc.u, bc.v, bc.w};
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const bool dir = (m == 0) ? rd : vd;
-            p0[m] = dir ? bcv[m]
-                        : S1[m] - (geo.t1x * g2[3 * m] + geo.t1y * g2[3 * m + 1] + geo.t1z * g2[3 * m + 2]);
-            pi[m] = p0[m];
-            pn[m] = p0[m];
-        }
-#pragma unroll
-        for (int t = 0; t < 12; t++) g1[t] = g2[t];
-    } else {
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            pi[m] = S1[m] - (geo.t1x * g1[3 * m] + geo.t1y * g1[3 * m + 1] + geo.t1z * g1[3 * m + 2]);
-            pn[m] = S2[m] - (geo.t2x * g2[3 * m] + geo.t2y * g2[3 * m + 1] + geo.t2z * g2[3 * m + 2]);
-            p0[m] = (pi[m] + pn[m]) * R(0.5);
-        }
-    }
-    // FP32 deviation form: offsets from the face centre (pop_dev); hdp is half
-    // the owner-neighbour difference of the reconstructed states
-    R hdp[4] = {R(0), R(0), R(0), R(0)};
-    if constexpr (sizeof(R) == 4) {
-        if (geo.bc_branch == R(0)) {
-#pragma unroll
-            for (int m = 0; m < 4; m++)
-                hdp[m] = ((S1[m] - S2[m]) - ((geo.t1x * g1[3 * m] + geo.t1y * g1[3 * m + 1] + geo.t1z * g1[3 * m + 2]) -
-                                             (geo.t2x * g2[3 * m] + geo.t2y * g2[3 * m + 1] + geo.t2z * g2[3 * m + 2]))) *
-                         R(0.5);
-        }
-    }
-    // Upwind selection by the sign of n.e_k with the threshold 0.001 dt
-    // (LBFS.cu:351-352 override the sin(pi/14) arguments).  Directions come in
-    // opposite pairs (k, k + 1): sum and difference of the pair's populations
-    // feed the moments.
-    const R thr = R(0.001) * dt;
-    const R q = a.recon_q;
-    R g0;
-    if constexpr (sizeof(R) == 4) g0 = pop_dev(p0, R(0), R(0), rho0, q);
-    else g0 = pop_g<R>(p0, R(0), rho0, q);
-    R sax[3], dax[3];          // axis pairs (+e_c, -e_c): sum and difference
-    R sc, mcor[3], ocor[3];    // corner pairs: sum of sums; sum of e_c x difference; of e_c e_q x sum
-#pragma unroll
-    for (int k = 1; k < 15; k += 2) {
-        const Dir e = dir_of(k);  // odd k: e_k; k + 1: -e_k
-        const int ee[3] = {e.ex, e.ey, e.ez};
-        const R s = (k < 7) ? (e.ex ? geo.nx : (e.ey ? geo.ny : geo.nz))
-                            : (R(e.ex) * geo.nx + R(e.ey) * geo.ny + R(e.ez) * geo.nz);
-        // Upwind sides.  With sg = -1 where n.e < -thr and +1 otherwise, the population of
-        // direction sg e comes from the owner and that of -sg e from the neighbour, each
-        // extrapolated along its own direction: Lo = p_owner - sg dt (e . g_owner),
-        // Ln = p_neighbour + sg dt (e . g_neighbour).  Where |n.e| <= thr (cen) both come from
-        // the face centre with the mean gradient C (sg = +1: +e at Lo, -e at Ln).  Only warps
-        // with such a lane take the selects; in the others the side is a sign of dt.
-        const bool neg = s < -thr, cen = !(s > thr) && !neg;
-        const R sg = neg ? R(-1) : R(1);
-        const R sdt = sg * dt;
-        R A[4], B[4];  // e . gradient per component, owner (A) and neighbour (B)
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            bool first = true;
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                if (!ee[d]) continue;
-                const R ga = ee[d] > 0 ? g1[3 * m + d] : -g1[3 * m + d];
-                const R gb = ee[d] > 0 ? g2[3 * m + d] : -g2[3 * m + d];
-                A[m] = first ? ga : A[m] + ga;
-                B[m] = first ? gb : B[m] + gb;
-                first = false;
-            }
-        }
-        R Lo[4], Ln[4], Do[4], Dn[4];
-        if (__any_sync(__activemask(), cen)) {
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const R C = (A[m] + B[m]) * R(0.5);
-                const R Xo = cen ? C : A[m], Xn = cen ? C : B[m];
-                if constexpr (sizeof(R) == 8) {
-                    Lo[m] = (cen ? p0[m] : pi[m]) - sdt * Xo;
-                    Ln[m] = (cen ? p0[m] : pn[m]) + sdt * Xn;
-                } else {
-                    // FP32: offsets from the face centre (+hdp owner, -hdp neighbour, 0 centre)
-                    Do[m] = (cen ? R(0) : hdp[m]) - sdt * Xo;
-                    Dn[m] = (cen ? R(0) : -hdp[m]) + sdt * Xn;
-                    Lo[m] = p0[m] + Do[m];
-                    Ln[m] = p0[m] + Dn[m];
-                }
-            }
-        } else {
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                if constexpr (sizeof(R) == 8) {
-                    Lo[m] = pi[m] - sdt * A[m];
-                    Ln[m] = pn[m] + sdt * B[m];
-                } else {
-                    Do[m] = hdp[m] - sdt * A[m];
-                    Dn[m] = -hdp[m] + sdt * B[m];
-                    Lo[m] = p0[m] + Do[m];
-                    Ln[m] = p0[m] + Dn[m];
-                }
-            }
-        }
-        // e . u at both states (and e . d, FP32); the owner's direction is sg e, the neighbour's -sg e
-        R Eo, En, Edo = R(0), Edn = R(0);
-        {
-            bool first = true;
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                if (!ee[d]) continue;
-                const R uo = ee[d] > 0 ? Lo[1 + d] : -Lo[1 + d], un = ee[d] > 0 ? Ln[1 + d] : -Ln[1 + d];
-                Eo = first ? uo : Eo + uo;
-                En = first ? un : En + un;
-                if constexpr (sizeof(R) == 4) {
-                    const R dO = ee[d] > 0 ? Do[1 + d] : -Do[1 + d], dN = ee[d] > 0 ? Dn[1 + d] : -Dn[1 + d];
-                    Edo = first ? dO : Edo + dO;
-                    Edn = first ? dN : Edn + dN;
-                }
-                first = false;
-            }
-        }
-        R go, gn;
-        if constexpr (sizeof(R) == 4) {
-            go = pop_dev(Lo, sg * Eo, sg * Edo, rho0, q);
-            gn = pop_dev(Ln, -sg * En, -sg * Edn, rho0, q);
-        } else {
-            go = pop_g<R>(Lo, sg * Eo, rho0, q);
-            gn = pop_g<R>(Ln, -sg * En, rho0, q);
-        }
-        // the pair's sum and its (+e) - (-e) difference
-        const R sig = go + gn, del = sg * (go - gn);
-        if (k < 7) {
-            const int c = e.ex ? 0 : (e.ey ? 1 : 2);
-            sax[c] = sig;
-            dax[c] = del;
-        } else if (k == 7) {  // (+,+,+): first corner pair
-            sc = sig;
-#pragma unroll
-            for (int d = 0; d < 3; d++) { mcor[d] = del; ocor[d] = sig; }
-        } else {
-            sc = sc + sig;
-#pragma unroll
-            for (int d = 0; d < 3; d++) mcor[d] = (ee[d] > 0) ? mcor[d] + del : mcor[d] - del;
-            ocor[0] = (ee[0] * ee[1] > 0) ? ocor[0] + sig : ocor[0] - sig;
-            ocor[1] = (ee[0] * ee[2] > 0) ? ocor[1] + sig : ocor[1] - sig;
-            ocor[2] = (ee[1] * ee[2] > 0) ? ocor[2] + sig : ocor[2] - sig;
-        }
-    }
-    constexpr R w_rest = R(2.0 / 9.0), w_axis = R(1.0 / 9.0), w_corner = R(1.0 / 72.0);
-    LatMoments<R> M;
-    M.rho = w_rest * g0 + w_axis * ((sax[0] + sax[1]) + sax[2]) + w_corner * sc;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        M.m[c] = w_axis * dax[c] + w_corner * mcor[c];
-        M.d[c] = w_axis * sax[c] + w_corner * sc;
-        M.o[c] = w_corner * ocor[c];
-        if constexpr (sizeof(R) == 4) M.m[c] = M.m[c] + rho0 * p0[1 + c];  // the term pop_dev leaves out
-    }
-    const R vf = is_bc ? R(1) : a.visc_factor[oc.x];
-    const R tau = (a.testcase == 8) ? R(0) : (a.visc * vf * R(3) / dt * a.gamma_inv);
-    return interface_flux<R>(M, rho0, tau, a.gamma_inv, geo.area, -1, geo.nx, geo.ny, geo.nz);
-}
 
 // Interior faces of an axis-aligned mesh: faces [0, nfx) x, [nfx, nfx+nfy) y,
 // the rest z; warps never mix axes except at the two range boundaries.
@@ -746,7 +143,10 @@ __global__ void __launch_bounds__(256) k_cfl(FluidArgs<R> a) {
 
 // ------------------------------------------------------------------ K3 ----
 
-template <typename R, int TB>
+// GRID: behind the fused step, whose cell sums over the interior faces it
+// reads (32 B instead of six fluxes of 32 / 16 B), adding the boundary faces,
+// whose indices follow the interior ones: the sum order of the gather.
+template <typename R, int TB, bool GRID>
 __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
     __shared__ double sh[4][TB / 32];
     __shared__ bool last_block;
@@ -785,25 +185,58 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
         // 1 / volume: products instead of 24 divisions
         const double iv = a.inv_volume_uniform ? a.inv_volume_all : __ldg(a.cell_inv_volume + i);
         double r[4] = {0, 0, 0, 0};  // rho, u, v, w
-        int cfl[6];
-        if (a.grid_faces) {  // the structured mesh's faces, formed (no dependent load before the fluxes)
-            grid_cell_faces(i, a.grid_n[0], a.grid_n[1], a.grid_n[2], cfl);
-        } else {
+        if constexpr (GRID) {
+            const double4 q = a.grid_res[i];
+            r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
+            const unsigned sides = a.grid_sides[i];
+            if (sides & 1u) {
+                for (int e = 0; e < 6; e++) {
+                    const int f = __ldg(a.cell_faces + 6 * (size_t)i + e) - 1;
+                    if (f < a.ni) continue;
+                    const Vec4<R> fx = a.flux[f];
+                    const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
 #pragma unroll
-            for (int q = 0; q < 3; q++) {
-                const int2 p = __ldg(reinterpret_cast<const int2 *>(a.cell_faces) + 3 * i + q);
-                cfl[2 * q] = p.x;
-                cfl[2 * q + 1] = p.y;
+                    for (int m = 0; m < 4; m++) r[m] = r[m] + (-fv[m] * iv);
+                }
             }
-        }
+            if (sides & 14u) {  // upper faces that another tile formed
+                int sy = a.grid_stride[0], sz = a.grid_stride[1];
+                if (sy == 0) {
+                    const int2 q = a.grid_strides[__ldg(a.grid_instance + i)];
+                    sy = q.x;
+                    sz = q.y;
+                }
+                const double ia = iv * a.grid_area;
 #pragma unroll
-        for (int q = 0; q < 6; q++) {
-            const int e = cfl[q];
-            const int f = (e > 0 ? e : -e) - 1;
-            const Vec4<R> fx = a.flux[f];
-            const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
+                for (int d = 0; d < 3; d++) {
+                    if (!(sides >> (d + 1) & 1u)) continue;
+                    const Vec4<R> fx = a.grid_edge[(size_t)d * a.nc + i + (d == 0 ? 1 : (d == 1 ? sy : sz))];
+                    const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
 #pragma unroll
-            for (int m = 0; m < 4; m++) r[m] = (e > 0) ? r[m] + (-fv[m] * iv) : r[m] + fv[m] * iv;
+                    for (int m = 0; m < 4; m++) r[m] = r[m] + (-fv[m] * ia);
+                }
+            }
+        } else {
+            int cfl[6];
+            if (a.grid_faces) {  // the structured mesh's faces, formed (no dependent load before the fluxes)
+                grid_cell_faces(i, a.grid_n[0], a.grid_n[1], a.grid_n[2], cfl);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    const int2 p = __ldg(reinterpret_cast<const int2 *>(a.cell_faces) + 3 * i + q);
+                    cfl[2 * q] = p.x;
+                    cfl[2 * q + 1] = p.y;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 6; q++) {
+                const int e = cfl[q];
+                const int f = (e > 0 ? e : -e) - 1;
+                const Vec4<R> fx = a.flux[f];
+                const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
+#pragma unroll
+                for (int m = 0; m < 4; m++) r[m] = (e > 0) ? r[m] + (-fv[m] * iv) : r[m] + fv[m] * iv;
+            }
         }
         if (a.closure) {
 #pragma unroll
@@ -1047,11 +480,15 @@ template <typename R> void launch_fluid_flux(const FluidArgs<R> &a, cudaStream_t
     launch_fluid_flux_axis<R>(a, s);
     launch_fluid_flux_general<R>(a, s);
 }
-template <typename R> void launch_fluid_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
+template <typename R, bool GRID> void launch_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
     const int tb = a.tb_update, g = k3_grid(a);
-    if (tb == 128) launch_maybe_pdl(k_cell_update<R, 128>, g, 128, s, pdl, a);
-    else if (tb == 512) launch_maybe_pdl(k_cell_update<R, 512>, g, 512, s, pdl, a);
-    else launch_maybe_pdl(k_cell_update<R, 256>, g, 256, s, pdl, a);
+    if (tb == 128) launch_maybe_pdl(k_cell_update<R, 128, GRID>, g, 128, s, pdl, a);
+    else if (tb == 512) launch_maybe_pdl(k_cell_update<R, 512, GRID>, g, 512, s, pdl, a);
+    else launch_maybe_pdl(k_cell_update<R, 256, GRID>, g, 256, s, pdl, a);
+}
+template <typename R> void launch_fluid_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
+    if (a.grid_res) launch_update<R, true>(a, s, pdl);
+    else launch_update<R, false>(a, s, pdl);
 }
 
 template <typename R> void launch_fluid_cfl(const FluidArgs<R> &a, cudaStream_t s) {

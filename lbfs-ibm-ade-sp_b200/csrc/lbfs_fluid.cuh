@@ -235,6 +235,15 @@ template <typename R> struct FluidArgs {
     // leaves out, sum over the faces of -+ rho0/3 n area / volume (null when
     // every cell closes, where it vanishes)
     const double *closure;       // [3 nc]
+    // after the fused step of structured grids (lbfs_fused.h): the cells' sums over their interior
+    // faces and which cells have boundary faces (null after the separate kernels)
+    const double4 *grid_res;     // [nc] (rho, u, v, w)
+    const unsigned char *grid_sides;  // [nc] GridArgs::sides
+    const Vec4<R> *grid_edge;    // GridArgs::edge, with the face area and the strides along y and z
+    double grid_area;
+    int grid_stride[2];          // of the one instance; 0: grid_strides[grid_instance[cell]]
+    const int2 *grid_strides;
+    const int *grid_instance;
     double4 *t1;                 // [nc] (u, v, w, rho) conservative accumulator, FP64
     double *res_out;             // [4*nc] residuals kept for parity checks (null = not stored)
     // IBM patches (one per membrane), grouped by ensemble instance

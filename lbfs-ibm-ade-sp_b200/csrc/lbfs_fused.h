@@ -1,0 +1,81 @@
+// Plan of the fused fluid step of uniform grids (lbfs_fused.cu).
+//
+// It applies to axis-aligned meshes whose cells form logical grids: each
+// instance's cells are i + nx (j + ny k), every interior face joins two cells one
+// apart along one axis, owner the lower; every missing side of a cell is one
+// boundary face; a cell's gradient stencil is its six neighbours (or ghosts), each
+// with a weight along its axis alone and of one magnitude; every face has one area
+// and one dt and lies dt from both centres (a boundary face's ghost straight across
+// it); a periodic partner is a boundary cell; and gamma is 1.  The generator's uniform
+// meshes and their ensembles meet this; it is checked face by face and cell by
+// cell at create, and any other mesh keeps the separate kernels.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+#include "lbfs_fluid.cuh"
+
+namespace lbfs {
+
+// Blocks per SM the kernel is compiled for: FP64 four of 128 registers, FP32 six of 80.
+template <typename R> struct GridShape { static constexpr int blocks = sizeof(R) == 8 ? 4 : 6; };
+constexpr int kUniformThreads = 128;   // a column each
+constexpr int kUniformPlaneMax = 230;  // cells of a tile's plane with two more below and one above along x and y
+
+struct GridTile {
+    int x0, y0, z0, w, h, d, inst, pad;  // columns [x0, x0 + w) x [y0, y0 + h), planes [z0, z0 + d)
+};
+struct GridInst {
+    int cell0, nx, ny, nz;
+    int side0[6];  // first entry in `side` of the sides -x, +x (j + ny k), -y, +y (i + nx k), -z, +z (i + nx j)
+    int active;    // bit d: some face of side d is not zero-gradient in every component
+    int pad;
+};
+// The ghost of one boundary face as its cell's gradients need it: val the
+// Dirichlet values (velocity profiles of types 9 and 10 evaluated), flags which
+// components take them (the others copy the cell), or the periodic partner's.
+template <typename R> struct alignas(16) GridSide {
+    Vec4<R> val;
+    // bit 0: rho Dirichlet, 1: velocity Dirichlet, 2: rho periodic, 3: velocity periodic, 4: the face takes
+    // the velocity val itself (type 1)
+    int flags, partner;
+};
+// One boundary face: its cell, the cell's strides along y and z, info -- its side d,
+// up to two more missing sides of the cell << 3 and << 6 (7: none) with their
+// boundary faces in more, bit 10: the interior branch (an instance's first ghost);
+// partner: a boundary face of the periodic partner cell.
+struct alignas(16) GridBnd {
+    int cell, sy, sz, info, more[2], partner, pad;
+};
+
+// Multiples of the slope weight w = dt x gradient weight: 3 w, 3 w^2, w / 2, 3 w / 2, 3 w^2 / 4.
+template <typename R> struct GridWeights {
+    R w, w3, ww3, h, h3, hh3;
+};
+
+template <typename R> struct GridArgs {
+    int n_tiles, bnd_blocks;
+    int plane_stride;              // cells of the largest tile's plane
+    int stage_max;                 // threads that may hold a ghost's record
+    const GridTile *tiles;
+    const GridInst *inst;
+    const GridSide<R> *side;       // the boundary faces of every side of every instance
+    const GridBnd *bnd;            // [nb]
+    const GridSide<R> *bnd_side;   // [nb] the boundary faces' records in their own order
+    R bnd_k;                       // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
+    GridWeights<R> cw;
+    R area, dt;                    // of every interior face
+    Vec4<R> *prev;                 // [nc + nb] the state the last step started from
+    double4 *res;                  // [nc] sums of the interior face fluxes (rho, u, v, w)
+    Vec4<R> *edge;                 // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes
+    const unsigned char *sides;    // [nc] bit 0: the cell has boundary faces; bits 1, 2, 3: its upper x, y, z flux is in edge
+};
+
+template <typename R> size_t grid_smem_bytes(const GridArgs<R> &ga);
+template <typename R> cudaError_t grid_prepare();
+// boundary face fluxes and the cells' interior sums of one step
+template <typename R> void launch_grid_step(const FluidArgs<R> &a, const GridArgs<R> &ga, cudaStream_t s);
+
+}  // namespace lbfs

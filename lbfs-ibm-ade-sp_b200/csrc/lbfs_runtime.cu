@@ -23,6 +23,7 @@
 #include "lbfs_adjoint.h"
 #include "lbfs_b200.h"
 #include "lbfs_fluid.cuh"
+#include "lbfs_fused.h"
 #include "lbfs_internal.h"
 #include "lbfs_kernels.h"
 
@@ -56,6 +57,14 @@ struct lbfs_solver {
     // tiles of the face kernel (interior faces ordered by owner within each axis), one table per flux
     // block size 64 / 128 / 256: tiles_h[b] = first face of each axis owned by tile t (3 ints per
     // tile, n_tiles + 1 rows), tile_maxnb[b][t] = largest neighbour of the faces of tiles <= t
+    // fused fluid step of structured grids (lbfs_fused.h): grid64 / grid32 hold its plan when `fused`.
+    // separate: steps take the separate kernels all the same (the adjoint's recording, which reads
+    // every step's gradients).  fields_stale: the last step left no gradients, fluxes or ghosts; they
+    // are formed from the state it started from when asked for.
+    bool fused = false, separate = false, fields_stale = false;
+    GridArgs<double> grid64{};
+    GridArgs<float> grid32{};
+    cudaGraphExec_t graph_separate = nullptr;
     bool tiled = false;
     std::vector<int> tiles_h[3], tile_maxnb[3];
     int *d_tiles[3] = {};
@@ -142,6 +151,7 @@ bool dynamic_dt(const lbfs_params &p) { return p.time_stepping != 0 && p.time_st
 // whenever one of those changes.
 void drop_step_graphs(lbfs_solver *s) {
     if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; s->graph_steps = 0; }
+    if (s->graph_separate) { cudaGraphExecDestroy(s->graph_separate); s->graph_separate = nullptr; }
     if (s->loop_graph) { cudaGraphExecDestroy(s->loop_graph); s->loop_graph = nullptr; }
 }
 
@@ -176,6 +186,9 @@ struct DevBuf {
 template <typename R> FluidArgs<R> &fluid(lbfs_solver *s);
 template <> FluidArgs<double> &fluid<double>(lbfs_solver *s) { return s->f64; }
 template <> FluidArgs<float> &fluid<float>(lbfs_solver *s) { return s->f32; }
+template <typename R> GridArgs<R> &grid(lbfs_solver *s);
+template <> GridArgs<double> &grid<double>(lbfs_solver *s) { return s->grid64; }
+template <> GridArgs<float> &grid<float>(lbfs_solver *s) { return s->grid32; }
 
 int check_mesh(const lbfs_mesh_desc *m) {
     if (!m) return set_error(LBFS_ERR_ARG, "mesh descriptor is null");
@@ -215,6 +228,10 @@ int check_mesh(const lbfs_mesh_desc *m) {
         if (!(m->cell_volume[i] > 0)) return set_error(LBFS_ERR_ARG, "cell volume must be positive");
     return LBFS_OK;
 }
+
+template <typename R>
+int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>> &lsw,
+              const std::vector<AxisFace<R>> &axf, const std::vector<GenFace<R>> &gen, const std::vector<BcRec<R>> &bcr);
 
 template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     FluidArgs<R> &a = fluid<R>(s);
@@ -452,6 +469,8 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
             a.grid_faces = 1;
             for (int d = 0; d < 3; d++) a.grid_n[d] = n3[d];
         }
+    }
+    if (a.axis_aligned && !generic) {
         bool one = nc > 0;
         for (int c = 1; c < nc && one; c++) one = std::memcmp(&inv_vol[c], &inv_vol[0], sizeof(double)) == 0;
         if (one) {
@@ -499,6 +518,296 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     a.n_membranes = 0;
     a.instances = nullptr;
     a.cell_instance = nullptr;
+    return plan_grid<R>(s, m, lsw, axf, gen, bcr);
+}
+
+// Tiles of an instance's grid for the fused step: columns of w x h cells walked
+// over some planes.  w and h minimise the work per cell of a plane -- warps of
+// faces, a block's idle lanes among them, and the loads of the tile with its ring
+// -- over even splits of the axes that fit the block's threads and the plane's
+// shared memory.
+struct TileShape {
+    int w, h;
+};
+TileShape tile_shape(int nx, int ny) {
+    TileShape best{0, 0};
+    double best_cost = 1e300;
+    for (int kx = 1; kx <= nx; kx++) {
+        const int w = (nx + kx - 1) / kx;
+        if (w > kUniformThreads) continue;
+        if (w < 4 && nx > 4) break;
+        for (int ky = 1; ky <= ny; ky++) {
+            const int h = (ny + ky - 1) / ky;
+            if (w * h > kUniformThreads || 2 * (w + h + 4) > kUniformThreads || (w + 3) * (h + 3) > kUniformPlaneMax) continue;
+            if (h < 2 && ny > 2) break;
+            const double plane = 3.4 * ((w * h + 31) / 32) + 0.2 * ((w + 3) * (h + 3) / 32.0);
+            const double cost = plane * ((nx + w - 1) / w) * (double)((ny + h - 1) / h);
+            if (cost < best_cost * (1 - 1e-9)) {
+                best_cost = cost;
+                best = {w, h};
+            }
+        }
+    }
+    return best;
+}
+
+// The fused step's plan: the conditions of lbfs_fused.h over every face and
+// cell, the geometry by direction, and the tiles.  Leaves s->fused false where a
+// condition fails (LBFS_SEPARATE_KERNELS set: always; a diagnostic switch).
+template <typename R>
+int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>> &lsw,
+              const std::vector<AxisFace<R>> &axf, const std::vector<GenFace<R>> &gen, const std::vector<BcRec<R>> &bcr) {
+    FluidArgs<R> &a = fluid<R>(s);
+    GridArgs<R> &ga = grid<R>(s);
+    s->fused = false;
+    if (!a.axis_aligned || a.ni == 0 || std::getenv("LBFS_SEPARATE_KERNELS")) return LBFS_OK;
+    // FP32 keeps the separate kernels: bound by instruction issue in both forms, the fused pass took 22 us
+    // against their 21 at 64^3 (two ducts of 57 x 45 x 33 side by side: 3 % more)
+    if (s->fp32) return LBFS_OK;
+    const int nc = a.nc, ni = a.ni, nb = a.nb;
+    // the instances' grids, and each cell's place in its grid
+    std::vector<GridInst> inst;
+    std::vector<int> place(nc);  // 6 bits: sides on which the cell has no neighbour; instance above
+    long long side_total = 0;
+    for (const lbfs_grid_desc &g : s->grids) {
+        if (!(g.delta_x > 0)) return LBFS_OK;
+        long long n[3];
+        for (int d = 0; d < 3; d++) {
+            n[d] = std::llround(g.length[d] / g.delta_x);
+            if (n[d] < 1 || n[d] > nc) return LBFS_OK;
+        }
+        if (n[0] * n[1] > nc || n[0] * n[1] * n[2] != g.n_cells) return LBFS_OK;
+        GridInst q{};
+        q.cell0 = g.cell0; q.nx = (int)n[0]; q.ny = (int)n[1]; q.nz = (int)n[2];
+        const long long area[3] = {n[1] * n[2], n[0] * n[2], n[0] * n[1]};
+        for (int d = 0; d < 6; d++) {
+            q.side0[d] = (int)side_total;
+            side_total += area[d / 2];
+        }
+        int c = q.cell0;
+        for (int k = 0; k < q.nz; k++)
+            for (int j = 0; j < q.ny; j++)
+                for (int i = 0; i < q.nx; i++, c++)
+                    place[c] = (i == 0) | (i == q.nx - 1) << 1 | (j == 0) << 2 | (j == q.ny - 1) << 3 | (k == 0) << 4 |
+                               (k == q.nz - 1) << 5 | (int)inst.size() << 6;
+        inst.push_back(q);
+    }
+    if (side_total != nb) return LBFS_OK;  // every missing side has one boundary face
+    auto stride = [&](int c, int ax) {
+        const GridInst &q = inst[place[c] >> 6];
+        return ax == 0 ? 1 : (ax == 1 ? q.nx : q.nx * q.ny);
+    };
+    // every interior face joins a cell to its neighbour along one axis
+    std::vector<int> low_face(3 * (size_t)nc, -1);
+    for (int f = 0; f < ni; f++) {
+        const int o = m->owner[f], n = m->neighbour[f];
+        int ax = 0;
+        while (ax < 3 && !(n - o == stride(o, ax) && !(place[o] >> (2 * ax + 1) & 1) && !(place[n] >> (2 * ax) & 1))) ax++;
+        if (ax == 3 || (place[o] >> 6) != (place[n] >> 6) || low_face[(size_t)ax * nc + n] >= 0) return LBFS_OK;
+        if (ax != ((f < a.nfx) ? 0 : ((f < a.nfx + a.nfy) ? 1 : 2))) return LBFS_OK;
+        low_face[(size_t)ax * nc + n] = f;
+    }
+    for (int ax = 0; ax < 3; ax++)
+        for (int c = 0; c < nc; c++)
+            if ((low_face[(size_t)ax * nc + c] < 0) != ((place[c] >> (2 * ax) & 1) != 0)) return LBFS_OK;
+    // the boundary face of every missing side, by the outward normal's largest component
+    std::vector<int> side_bc(nb, -1), side_of(nb);
+    std::vector<unsigned char> sides(nc, 0);
+    for (int b = 0; b < nb; b++) {
+        const int f = ni + b, o = m->owner[f];
+        const double *n = m->face_normal + 3 * (size_t)f;
+        int ax = 0;
+        for (int d = 1; d < 3; d++)
+            if (std::fabs(n[d]) > std::fabs(n[ax])) ax = d;
+        const int d = 2 * ax + (n[ax] > 0 ? 1 : 0);
+        if (!(place[o] >> d & 1)) return LBFS_OK;
+        const GridInst &q = inst[place[o] >> 6];
+        const int l = o - q.cell0, i = l % q.nx, j = (l / q.nx) % q.ny, k = l / (q.nx * q.ny);
+        int &slot = side_bc[q.side0[d] + (ax == 0 ? j + q.ny * k : (ax == 1 ? i + q.nx * k : i + q.nx * j))];
+        if (slot >= 0) return LBFS_OK;
+        slot = b;
+        side_of[b] = d;
+        sides[o] = 1;
+    }
+    // the ghosts as the gradients take them (ghost_state)
+    std::vector<GridSide<R>> side(nb), bnd_side(nb);
+    std::vector<GridBnd> bnd(nb);
+    std::vector<int> face_of(nc, -1);  // a boundary face of the cell
+    for (size_t e = 0; e < side.size(); e++) {
+        const int b = side_bc[e], rt = m->bc_rho_type[b], vt = m->bc_vel_type[b], ghost = nc + b;
+        const double *v = m->bc_values + 4 * (size_t)b;
+        const R gy = (R)m->cell_centroid[3 * (size_t)ghost + 1], gz = (R)m->cell_centroid[3 * (size_t)ghost + 2];
+        GridSide<R> q{};
+        q.val = {(R)v[0], (R)v[1], (R)v[2], (R)(v[3] - (double)a.rho0)};
+        if (vt == 9) q.val.u = (R)(16 * (double)q.val.u * (a.H2 + gy) * (a.H2 - gy) * (a.H2 + gz) * (a.H2 - gz) / a.H4);
+        else if (vt == 10) q.val.u = gy * q.val.u;
+        q.flags = (rt == 1 ? 1 : 0) | (vt == 1 || vt == 9 || vt == 10 ? 2 : 0) | (rt == 3 ? 4 : 0) | (vt == 3 ? 8 : 0) |
+                  (vt == 1 ? 16 : 0);
+        q.partner = rt == 3 || vt == 3 ? m->periodic_node[b] : 0;
+        side[e] = q;
+        if (q.flags) inst[place[m->owner[ni + b]] >> 6].active |= 1 << side_of[b];
+        bnd_side[b] = q;
+        // its cell's other missing sides
+        const int o = m->owner[ni + b], l = o - inst[place[o] >> 6].cell0;
+        const GridInst &g = inst[place[o] >> 6];
+        const int i = l % g.nx, j = (l / g.nx) % g.ny, k = l / (g.nx * g.ny);
+        GridBnd &r = bnd[b];
+        r = {o, g.nx, g.nx * g.ny, side_of[b], {0, 0}, 0, 0};
+        int others = 0;
+        for (int d = 0; d < 6; d++) {
+            if (d == side_of[b] || !(place[o] >> d & 1)) continue;
+            if (others == 2) return LBFS_OK;  // a grid one cell thick
+            r.info |= d << (3 + 3 * others);
+            r.more[others++] = side_bc[g.side0[d] + (d < 2 ? j + g.ny * k : (d < 4 ? i + g.nx * k : i + g.nx * j))];
+        }
+        for (; others < 2; others++) r.info |= 7 << (3 + 3 * others);
+        face_of[o] = b;
+    }
+    for (int b = 0; b < nb; b++) {
+        if (!(bnd_side[b].flags & 12)) continue;
+        bnd[b].partner = face_of[bnd_side[b].partner];
+        if (bnd[b].partner < 0) return LBFS_OK;
+    }
+    // every boundary face like the interior ones, its ghost straight across it
+    if (a.gamma_inv != R(1) || a.recon_q != R(1)) return LBFS_OK;
+    for (int b = 0; b < nb; b++) {
+        const GenFace<R> &f = gen[b];
+        const BcRec<R> &r = bcr[b];
+        const int ax = side_of[b] / 2;
+        const R sn = (side_of[b] & 1) ? R(1) : R(-1);
+        const R nv[3] = {f.nx, f.ny, f.nz}, t1[3] = {f.t1x, f.t1y, f.t1z}, t2[3] = {f.t2x, f.t2y, f.t2z};
+        const R dn[3] = {r.dnx, r.dny, r.dnz}, mv[3] = {r.mx, r.my, r.mz};
+        if (f.area != axf[0].area || f.dt != axf[0].dt || r.dmag != bcr[0].dmag) return LBFS_OK;
+        for (int q = 0; q < 3; q++) {
+            const R e = q == ax ? sn : R(0);
+            if (nv[q] != e || dn[q] != e || t1[q] != -f.dt * e || t2[q] != f.dt * e || mv[q] != (q == ax ? R(0) : R(1)))
+                return LBFS_OK;
+        }
+        if (f.bc_branch == R(0)) bnd[b].info |= 1024;
+    }
+    // every gradient stencil is the six neighbours, weighted along their axes alone by one magnitude
+    // (ref: a lower neighbour's weight)
+    R ref = R(0);
+    for (int c = 0; c < nc; c++) {
+        int seen = 0;
+        for (int q = 0; q < 6; q++) {
+            const int j = m->gradient_stencil[6 * (size_t)c + q];
+            int d = 0;
+            if (j >= nc) {
+                if (m->owner[ni + j - nc] != c) return LBFS_OK;
+                d = side_of[j - nc];
+            } else {
+                while (d < 6 && !(!(place[c] >> d & 1) && j - c == ((d & 1) ? stride(c, d / 2) : -stride(c, d / 2)))) d++;
+            }
+            if (d == 6 || (seen >> d & 1)) return LBFS_OK;
+            seen |= 1 << d;
+            const R *v = lsw[c].w + 3 * q;
+            if (c == 0 && q == 0) ref = (d & 1) ? -v[d / 2] : v[d / 2];
+            for (int r = 0; r < 3; r++)
+                if (v[r] != (r == d / 2 ? ((d & 1) ? -ref : ref) : R(0))) return LBFS_OK;
+        }
+    }
+    // every interior face has one area and dt and lies dt from both centres
+    ga.area = axf[0].area;
+    ga.dt = axf[0].dt;
+    for (int f = 0; f < ni; f++)
+        if (axf[f].area != ga.area || axf[f].dt != ga.dt || axf[f].t1 != -ga.dt || axf[f].t2 != ga.dt) return LBFS_OK;
+    const R c = -ref * ga.dt;
+    ga.cw = {c, R(3) * c, R(3) * c * c, R(0.5) * c, R(1.5) * c, R(0.75) * c * c};
+    ga.bnd_k = nb > 0 ? ga.dt / (bcr[0].dmag * c) : R(0);
+    int rc;
+    // the tiles, with one walk length d for all instances.  A block's time is d planes and a start of 1.2
+    // (clock stamps inside the kernel), a plane's about 3000 cycles and 1300 (FP64) or 1100 (FP32) for each
+    // block on its SM.  Grids of at most one wave: the longest block at that occupancy; larger ones: the
+    // blocks' throughput and a third of a block for the last wave.  64^3 FP64: 45 us at the chosen d = 4,
+    // 47 at 3, 54 at 8; 128^3: 203 at 8, 206 at 4, 213 at 16.
+    std::vector<TileShape> shape;
+    for (const GridInst &q : inst) {
+        const TileShape t = tile_shape(q.nx, q.ny);
+        if (t.w == 0) return LBFS_OK;
+        shape.push_back(t);
+    }
+    const int per_sm = GridShape<R>::blocks;
+    auto plane_time = [](int blocks) { return 3000.0 + (sizeof(R) == 8 ? 1300.0 : 1100.0) * blocks; };
+    int depth = 1;
+    double best = 1e300;
+    for (int d = 1; d <= 64; d++) {
+        double planes = 0.0, longest = 0.0, blocks = 0.0;
+        for (size_t q = 0; q < inst.size(); q++) {
+            const int walks = (inst[q].nz + d - 1) / d, even = (inst[q].nz + walks - 1) / walks;
+            const double n = (double)((inst[q].nx + shape[q].w - 1) / shape[q].w) * ((inst[q].ny + shape[q].h - 1) / shape[q].h) * walks;
+            blocks += n;
+            planes += n * (even + 1.2);
+            longest = std::max(longest, even + 1.2);
+        }
+        const int on_sm = (int)std::ceil(blocks / 148.0);
+        const double t = on_sm <= per_sm ? longest * plane_time(on_sm)
+                                         : planes / 148.0 * plane_time(per_sm) / per_sm + 0.35 * longest * plane_time(per_sm);
+        if (t < best * (1 - 1e-9)) {
+            best = t;
+            depth = d;
+        }
+    }
+    std::vector<GridTile> tiles;
+    int P = 0, G = 0;
+    for (size_t q = 0; q < inst.size(); q++) {
+        const GridInst &g = inst[q];
+        const int w0 = shape[q].w, h0 = shape[q].h, walks = (g.nz + depth - 1) / depth, dz = (g.nz + walks - 1) / walks;
+        for (int z = 0; z < g.nz; z += dz)
+            for (int y = 0; y < g.ny; y += h0)
+                for (int x = 0; x < g.nx; x += w0) {
+                    const GridTile t = {x, y, z, std::min(w0, g.nx - x), std::min(h0, g.ny - y), std::min(dz, g.nz - z), (int)q, 0};
+                    tiles.push_back(t);
+                    for (int k = t.z0; k < t.z0 + t.d; k++)  // upper faces that other tiles form
+                        for (int j = t.y0; j < t.y0 + t.h; j++)
+                            for (int i = t.x0; i < t.x0 + t.w; i++) {
+                                const int e = (i == t.x0 + t.w - 1 && i < g.nx - 1) << 1 |
+                                              (j == t.y0 + t.h - 1 && j < g.ny - 1) << 2 |
+                                              (k == t.z0 + t.d - 1 && k < g.nz - 1) << 3;
+                                if (e) sides[g.cell0 + i + g.nx * (j + g.ny * k)] |= (unsigned char)e;
+                            }
+                    P = std::max(P, (t.w + 3) * (t.h + 3));
+                    G = std::max(G, 2 * (t.w + t.h + 4));
+                }
+    }
+    GridTile *d_tiles;
+    GridInst *d_inst;
+    GridSide<R> *d_side;
+    GridBnd *d_bnd;
+    GridSide<R> *d_bside;
+    unsigned char *d_sides;
+    double4 *d_res;
+    Vec4<R> *d_prev;
+    if ((rc = s->upload(&d_tiles, tiles)) || (rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) ||
+        (rc = s->upload(&d_bnd, bnd)) || (rc = s->upload(&d_bside, bnd_side)) ||
+        (rc = s->upload(&d_sides, sides)) || (rc = s->alloc(&d_res, nc)) || (rc = s->alloc(&d_prev, (size_t)nc + nb)))
+        return rc;
+    if ((rc = s->alloc(&ga.edge, 3 * (size_t)nc))) return rc;
+    a.grid_edge = ga.edge;
+    a.grid_area = (double)ga.area;
+    a.grid_stride[0] = inst.size() == 1 ? inst[0].nx : 0;
+    a.grid_stride[1] = inst.size() == 1 ? inst[0].nx * inst[0].ny : 0;
+    if (inst.size() > 1) {
+        std::vector<int2> st;
+        std::vector<int> which(nc);
+        for (const GridInst &q : inst) st.push_back(make_int2(q.nx, q.nx * q.ny));
+        for (int i = 0; i < nc; i++) which[i] = place[i] >> 6;
+        int2 *d_st;
+        int *d_which;
+        if ((rc = s->upload(&d_st, st)) || (rc = s->upload(&d_which, which))) return rc;
+        a.grid_strides = d_st;
+        a.grid_instance = d_which;
+    }
+    ga.tiles = d_tiles; ga.inst = d_inst; ga.side = d_side; ga.bnd = d_bnd; ga.bnd_side = d_bside; ga.sides = d_sides; ga.res = d_res; ga.prev = d_prev;
+    ga.n_tiles = (int)tiles.size();
+    ga.bnd_blocks = (nb + kUniformThreads - 1) / kUniformThreads;
+    ga.plane_stride = P;
+    ga.stage_max = G;
+    if (grid_prepare<R>() != cudaSuccess) {
+        cudaGetLastError();
+        return LBFS_OK;
+    }
+    s->fused = true;
     return LBFS_OK;
 }
 
@@ -903,8 +1212,9 @@ void set_chunks(lbfs_solver *s, int K) {
     const bool aa = s->fp32 ? s->f32.axis_aligned : s->f64.axis_aligned;
     const int tb = s->fp32 ? (aa ? s->f32.tb_flux : s->f32.tb_gen) : (aa ? s->f64.tb_flux : s->f64.tb_gen);
     const std::vector<int> &mx = s->tile_maxnb[tb == 64 ? 0 : (tb == 256 ? 2 : 1)];
-    // gradients and interior fluxes (K each), boundary fluxes, update; membrane kernels; CFL
-    s->launches_per_step = 2 * K + 2 + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
+    // fused step: fluid pass and update; else gradients and interior fluxes (K each), boundary fluxes,
+    // update; membrane kernels; CFL
+    s->launches_per_step = (s->fused ? 2 : 2 * K + 2) + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
     s->chunk_cell.assign(K + 1, 0);
     s->chunk_faces.assign(K, FaceRanges{});
     for (int c = 0; c <= K; c++) s->chunk_cell[c] = (int)((long long)s->nc * c / K);
@@ -1048,7 +1358,91 @@ int enqueue_k1_k2(lbfs_solver *s, FluidArgs<R> &a, int *n, bool spread_here,
     return LBFS_OK;
 }
 
+// Joins the membrane stream to a capture behind the launch completion of the
+// handle's stream's last kernel (every block has begun).
+int fork_behind_launch(lbfs_solver *s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t nd = 0;
+    LBFS_CUDA(cudaStreamGetCaptureInfo_v3(s->stream, &st, nullptr, nullptr, &deps, &edges, &nd));
+    cudaGraphNode_t k1 = nullptr;
+    cudaGraphNodeType type;
+    if (st == cudaStreamCaptureStatusActive && nd == 1 && cudaGraphNodeGetType(deps[0], &type) == cudaSuccess &&
+        type == cudaGraphNodeTypeKernel)
+        k1 = deps[0];
+    LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
+    LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
+    if (k1) {  // otherwise the membrane stream stays behind the kernel's end
+        cudaGraphEdgeData e = {};
+        e.from_port = cudaGraphKernelNodePortLaunchCompletion;
+        e.type = cudaGraphDependencyTypeProgrammatic;
+        LBFS_CUDA(cudaStreamUpdateCaptureDependencies_v2(s->stream2, &k1, &e, 1, cudaStreamSetCaptureDependencies));
+    }
+    return LBFS_OK;
+}
+
+// A step through the fused fluid pass: the membrane chain, spread included, on
+// its own stream beside the pass (or behind its launch completion, launch shape
+// membrane_after_k1), then the update.  An interior-viscosity update goes
+// between the two, in sequence.
+template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
+    const GridArgs<R> &ga = grid<R>(s);
+    FluidArgs<R> a = fluid<R>(s);
+    a.grid_res = ga.res;
+    a.grid_sides = ga.sides;
+    int n = 0;
+    for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = false;
+    if (s->profiling) LBFS_CUDA(record_event(s->ev_phase[5][0], s->stream));
+    if (a.time_stepping != 0 && a.time_stepping != LBFS_DT_CONSTANT) {
+        launch_fluid_cfl<R>(a, s->stream);
+        n += 1;
+    }
+    auto pass = [&]() {
+        PhaseMark m(s, 2, s->stream);
+        launch_grid_step<R>(a, ga, s->stream);
+        n += 1;
+    };
+    if (s->n_membranes == 0) {
+        pass();
+    } else if (visc_update) {
+        { PhaseMark m(s, 0, s->stream); n += launch_membrane(s->ma, s->stream); }
+        { PhaseMark m(s, 4, s->stream); launch_interior_viscosity(s->va, s->stream); }
+        n += 2;
+        pass();
+    } else {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        LBFS_CUDA(cudaStreamIsCapturing(s->stream, &cap));
+        const bool behind = s->membrane_after_k1 && cap == cudaStreamCaptureStatusActive && !s->kernel_events;
+        if (behind) {
+            pass();
+            int rc = fork_behind_launch(s);
+            if (rc) return rc;
+        } else {
+            LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
+            LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
+        }
+        {
+            PhaseMark m(s, 0, s->stream2);
+            n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted);
+        }
+        LBFS_CUDA(cudaEventRecord(s->ev_join, s->stream2));
+        if (!behind) pass();
+        LBFS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_join, 0));
+    }
+    { PhaseMark m(s, 3, s->stream); launch_fluid_update<R>(a, s->stream, !s->kernel_events); }
+    n += 1;
+    if (s->profiling) {
+        LBFS_CUDA(record_event(s->ev_phase[5][1], s->stream));
+        s->phase_recorded[5] = true;
+    }
+    LBFS_CUDA(cudaGetLastError());
+    if (launches) *launches = n;
+    return LBFS_OK;
+}
+
 template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *launches) {
+    if (s->fused && !s->separate) return enqueue_fused_step<R>(s, visc_update, launches);
     FluidArgs<R> &a = fluid<R>(s);
     int n = 0;
     for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = false;
@@ -1085,25 +1479,8 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
                 // the advection kernel reads nothing the gradients write and does not wait on its
                 // programmatic predecessor), so its kernels are placed behind the gradients' last wave.
                 const std::function<int()> after_k1 = [&]() -> int {
-                    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-                    const cudaGraphNode_t *deps = nullptr;
-                    const cudaGraphEdgeData *edges = nullptr;
-                    size_t nd = 0;
-                    LBFS_CUDA(cudaStreamGetCaptureInfo_v3(s->stream, &st, nullptr, nullptr, &deps, &edges, &nd));
-                    cudaGraphNode_t k1 = nullptr;
-                    cudaGraphNodeType type;
-                    if (st == cudaStreamCaptureStatusActive && nd == 1 &&
-                        cudaGraphNodeGetType(deps[0], &type) == cudaSuccess && type == cudaGraphNodeTypeKernel)
-                        k1 = deps[0];
-                    LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
-                    LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
-                    if (k1) {  // otherwise the membrane stream stays behind the gradient kernel's end
-                        cudaGraphEdgeData e = {};
-                        e.from_port = cudaGraphKernelNodePortLaunchCompletion;
-                        e.type = cudaGraphDependencyTypeProgrammatic;
-                        LBFS_CUDA(cudaStreamUpdateCaptureDependencies_v2(s->stream2, &k1, &e, 1,
-                                                                         cudaStreamSetCaptureDependencies));
-                    }
+                    const int r = fork_behind_launch(s);
+                    if (r) return r;
                     return membranes();
                 };
                 rc = enqueue_k1_k2<R>(s, a, &n, spread_here, &after_k1);
@@ -1132,6 +1509,28 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
     return LBFS_OK;
 }
 
+// Gradients, face fluxes and ghosts of the last fused step, formed by the
+// separate kernels from the state it started from; on the handle's stream.
+template <typename R> int form_fields(lbfs_solver *s) {
+    FluidArgs<R> a = fluid<R>(s);
+    a.state = grid<R>(s).prev;
+    launch_fluid_gradients<R>(a, s->stream);
+    launch_fluid_flux<R>(a, s->stream);
+    LBFS_CUDA(cudaGetLastError());
+    LBFS_CUDA(cudaMemcpyAsync(fluid<R>(s).state + s->nc, a.state + s->nc, sizeof(Vec4<R>) * (size_t)s->nb,
+                              cudaMemcpyDeviceToDevice, s->stream));
+    return LBFS_OK;
+}
+int ensure_fields(lbfs_solver *s) {
+    if (!s->fields_stale) return LBFS_OK;
+    int rc = s->fp32 ? form_fields<float>(s) : form_fields<double>(s);
+    if (rc) return rc;
+    s->fields_stale = false;
+    return LBFS_OK;
+}
+// after one or more steps
+void note_steps(lbfs_solver *s) { s->fields_stale = s->fused && !s->separate; }
+
 int enqueue(lbfs_solver *s, bool visc_update, int *launches) {
     return s->fp32 ? enqueue_step<float>(s, visc_update, launches) : enqueue_step<double>(s, visc_update, launches);
 }
@@ -1152,8 +1551,7 @@ int after_step(lbfs_solver *s) {
 }
 
 void free_all(lbfs_solver *s) {
-    if (s->graph) cudaGraphExecDestroy(s->graph);
-    if (s->loop_graph) cudaGraphExecDestroy(s->loop_graph);
+    drop_step_graphs(s);
     for (int p = 0; p < kPhases; p++)
         for (int e = 0; e < 2; e++)
             if (s->ev_phase[p][e]) cudaEventDestroy(s->ev_phase[p][e]);
@@ -1345,6 +1743,7 @@ extern "C" int lbfs_step(lbfs_solver *s, int32_t n_steps) {
     for (int k = 0; k < n_steps; k++) {
         int n = 0;
         int rc = enqueue(s, visc_due(s, s->t), &n);
+        note_steps(s);
         if (rc || (rc = after_step(s))) return rc;
         s->t++;
     }
@@ -1354,7 +1753,8 @@ extern "C" int lbfs_step(lbfs_solver *s, int32_t n_steps) {
 extern "C" int lbfs_step_graph(lbfs_solver *s, int32_t n_steps) {
     if (!s || n_steps < 0) return set_error(LBFS_ERR_ARG, "bad arguments");
     LBFS_CUDA(cudaSetDevice(s->device));
-    if (!s->graph) {
+    cudaGraphExec_t &graph = s->separate ? s->graph_separate : s->graph;
+    if (!graph) {
         cudaGraph_t g = nullptr;
         LBFS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
         int n = 0;
@@ -1367,7 +1767,7 @@ extern "C" int lbfs_step_graph(lbfs_solver *s, int32_t n_steps) {
         }
         // keep the membrane kernels' launch priority inside the graph (without
         // the flag every node runs at the priority of the stream it is launched into)
-        e = cudaGraphInstantiate(&s->graph, g, cudaGraphInstantiateFlagUseNodePriority);
+        e = cudaGraphInstantiate(&graph, g, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return set_error(LBFS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
         s->graph_steps = 1;
@@ -1378,9 +1778,10 @@ extern "C" int lbfs_step_graph(lbfs_solver *s, int32_t n_steps) {
             int rc = enqueue(s, true, nullptr);
             if (rc) return rc;
         } else {
-            LBFS_CUDA(cudaGraphLaunch(s->graph, s->stream));
+            LBFS_CUDA(cudaGraphLaunch(graph, s->stream));
             for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = s->graph_phase_recorded[p];
         }
+        note_steps(s);
         if (int rc = after_step(s)) return rc;
         s->t++;
     }
@@ -1467,6 +1868,7 @@ extern "C" int lbfs_step_until(lbfs_solver *s, int32_t max_steps, double toleran
             LBFS_CUDA(cudaGraphLaunch(s->loop_graph, s->stream));
             LBFS_CUDA(cudaMemcpyAsync(&u, s->d_until, sizeof u, cudaMemcpyDeviceToHost, s->stream));
             LBFS_CUDA(cudaStreamSynchronize(s->stream));
+            note_steps(s);
             s->t += u.count;
             done += u.count;
             for (int k = 0; k < 4; k++) res[k] = u.res[k];
@@ -1676,6 +2078,8 @@ template <typename R> int get_field_t(lbfs_solver *s, int which, double *out) {
 extern "C" int lbfs_get_field(lbfs_solver *s, int32_t which, double *out) {
     if (!s || !out) return set_error(LBFS_ERR_ARG, "null argument");
     LBFS_CUDA(cudaSetDevice(s->device));
+    if (which == LBFS_FIELD_GRADIENTS || which == LBFS_FIELD_FACE_FLUX || which == LBFS_FIELD_GHOST)
+        if (int rc = ensure_fields(s)) return rc;
     LBFS_CUDA(cudaStreamSynchronize(s->stream));
     return s->fp32 ? get_field_t<float>(s, which, out) : get_field_t<double>(s, which, out);
 }
@@ -2054,6 +2458,13 @@ extern "C" int lbfs_adjoint(lbfs_solver *s, int32_t n_steps, int32_t checkpoint_
     int rc = adj_prepare(s);
     if (rc) return rc;
     if (M > 0 && (rc = adjm_prepare(s))) return rc;
+    // the reverse sweep reads every step's gradients and ghosts: the separate kernels
+    struct Separate {
+        lbfs_solver *s;
+        explicit Separate(lbfs_solver *s_) : s(s_) { s->separate = true; }
+        ~Separate() { s->separate = false; }
+    } separate(s);
+    if ((rc = ensure_fields(s))) return rc;
     FluidArgs<double> &a = s->f64;
     MembraneArgs &ma = s->ma;
     AdjointArgs &j = s->adj;
@@ -2475,6 +2886,7 @@ extern "C" int lbfs_checkpoint_save(lbfs_solver *s, void *buf, uint64_t bytes) {
     if (rc) return rc;
     if (!buf || bytes < need) return set_error(LBFS_ERR_ARG, "checkpoint buffer too small (lbfs_checkpoint_size)");
     LBFS_CUDA(cudaSetDevice(s->device));
+    if ((rc = ensure_fields(s))) return rc;  // the ghosts are part of the state
     LBFS_CUDA(cudaStreamSynchronize(s->stream));
     const unsigned int *flags = s->fp32 ? s->f32.flags : s->f64.flags;
     CkHeader h{};
@@ -2508,6 +2920,7 @@ extern "C" int lbfs_checkpoint_load(lbfs_solver *s, const void *buf, uint64_t by
         h.n_membranes != s->n_membranes || h.total_nodes != s->total_nodes || h.total_springs != s->total_springs)
         return set_error(LBFS_ERR_ARG, "checkpoint of a different mesh, membrane set or precision");
     LBFS_CUDA(cudaSetDevice(s->device));
+    if ((rc = ensure_fields(s))) return rc;  // they follow the viscosity field, which the load replaces
     LBFS_CUDA(cudaStreamSynchronize(s->stream));
     const char *o = (const char *)buf + sizeof(h);
     for (const CkPart &p : ck_parts(s)) {
@@ -2531,6 +2944,7 @@ namespace {
 // miss.  The state (the checkpoint parts, the counter and the status word)
 // is put back afterwards.
 int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) {
+    if (int r = ensure_fields(s)) return r;  // of the caller's last step
     LBFS_CUDA(cudaStreamSynchronize(s->stream));
     const std::vector<CkPart> parts = ck_parts(s);
     size_t total = 0;
@@ -2635,6 +3049,7 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
     const int r2 = copy_all(false);
     if (!rc) rc = r2;
     s->t = t0;
+    if (s->fused) s->fields_stale = false;
     drop_graph(s);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
