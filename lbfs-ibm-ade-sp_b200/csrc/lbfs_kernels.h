@@ -8,7 +8,10 @@
 
 namespace lbfs {
 
-constexpr int kK3MaxBlocks = 148 * 8;      // default grid cap of the cell update (grid-stride)
+// Default grid cap of the cell update (grid-stride): its 256-thread blocks (62 registers) at once.  Twice as
+// many, in two waves: step 56.4 against 54.3 us at 64^3 and 284 against 279 at 128^3 FP64 with a membrane,
+// 135.2 against 132.1 jittered at 72^3; three an SM 54.5, 293 and 135.0.
+constexpr int kK3MaxBlocks = 148 * 4;
 constexpr int kSpreadMaxBlocks = 148 * 8;  // default spread grid cap (grid-stride over the tiles)
 constexpr int kK3PatchCache = 32;          // membranes whose patches the cell update caches per block
 constexpr int kK3BlocksLimit = LBFS_MAX_UPDATE_BLOCKS;  // partial-sum slots allocated for the update
