@@ -118,7 +118,7 @@ bool membrane_cluster_fits(int max_nodes);
 // events are given); returns the launch count.  without_spread: everything
 // but the spread, which the caller launches (launch_membrane_spread).
 int launch_membrane(const MembraneArgs &a, cudaStream_t s, cudaStream_t s_side = nullptr,
-                    cudaEvent_t ev_advected = nullptr, cudaEvent_t ev_sorted = nullptr, bool without_spread = false);
+                    cudaEvent_t ev_advected = nullptr, cudaEvent_t ev_sorted = nullptr, bool without_spread = false, cudaGraphNode_t *advect = nullptr);
 
 // Per membrane, the y-z binning of its triangles for the interior test: bins
 // of size >= every triangle's y-z extent and >= 4 delta_h over the membrane's

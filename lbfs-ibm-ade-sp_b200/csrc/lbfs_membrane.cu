@@ -1476,7 +1476,7 @@ void launch_hi(void (*kernel)(Args...), dim3 grid, dim3 block, size_t smem, cuda
 }  // namespace
 
 int launch_membrane(const MembraneArgs &a, cudaStream_t s, cudaStream_t s_side, cudaEvent_t ev_advected,
-                    cudaEvent_t ev_sorted, bool without_spread) {
+                    cudaEvent_t ev_sorted, bool without_spread, cudaGraphNode_t *advect) {
     const size_t smem = sort_smem_bytes(a.sort_capacity);
     const dim3 spring_grid((a.max_springs + 127) / 128, a.n_membranes);
     if (a.mode == kModeReference) {  // stress-free reference pass
@@ -1491,6 +1491,15 @@ int launch_membrane(const MembraneArgs &a, cudaStream_t s, cudaStream_t s_side, 
     const int blocks = (a.total_nodes * 32 + 255) / 256;
     if (a.state_is_float) launch_hi(k_mem_advect<float>, dim3(blocks), dim3(256), 0, s, a);
     else launch_hi(k_mem_advect<double>, dim3(blocks), dim3(256), 0, s, a);
+    if (advect) {  // its node, when the stream is being captured
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        const cudaGraphNode_t *deps = nullptr;
+        const cudaGraphEdgeData *edges = nullptr;
+        size_t nd = 0;
+        if (cudaStreamGetCaptureInfo_v3(s, &st, nullptr, nullptr, &deps, &edges, &nd) == cudaSuccess &&
+            st == cudaStreamCaptureStatusActive && nd == 1)
+            *advect = deps[0];
+    }
     const dim3 spread_grid(a.spread_blocks);
     if (a.force_cluster == 8 || a.force_cluster == 16) {
         // totals, sort, spring and node forces as one cluster per membrane, then the spread

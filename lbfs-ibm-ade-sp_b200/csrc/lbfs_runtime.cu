@@ -90,6 +90,15 @@ struct lbfs_solver {
     long long t = 0;  // time-step counter (the reference's loop index)
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
+    // several steps as one graph, once calls of the same length have repeated (lbfs_step_graph)
+    struct StepRun {
+        cudaGraphExec_t graph = nullptr;
+        int steps = 0;        // of the graph
+        int asked = 0;        // of the last calls
+        long long taken = 0;  // by them
+        bool failed = false;
+    };
+    StepRun run, run_separate;
     // lbfs_step_until: one graph whose while node repeats the step and a convergence check
     cudaGraphExec_t loop_graph = nullptr;
     bool loop_unavailable = false;  // the loop graph could not be built (steps go one at a time)
@@ -150,6 +159,10 @@ bool dynamic_dt(const lbfs_params &p) { return p.time_stepping != 0 && p.time_st
 // The cached graphs of a step hold the launch shape, the stream and the kernel arguments: dropped
 // whenever one of those changes.
 void drop_step_graphs(lbfs_solver *s) {
+    for (lbfs_solver::StepRun *r : {&s->run, &s->run_separate}) {
+        if (r->graph) cudaGraphExecDestroy(r->graph);
+        *r = lbfs_solver::StepRun{};
+    }
     if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; s->graph_steps = 0; }
     if (s->graph_separate) { cudaGraphExecDestroy(s->graph_separate); s->graph_separate = nullptr; }
     if (s->loop_graph) { cudaGraphExecDestroy(s->loop_graph); s->loop_graph = nullptr; }
@@ -1358,6 +1371,20 @@ int enqueue_k1_k2(lbfs_solver *s, FluidArgs<R> &a, int *n, bool spread_here,
     return LBFS_OK;
 }
 
+// In a capture: the next launch on the handle's stream begins only when every block
+// of the advection kernel has, so that the fluid's blocks do not take its place and
+// the membrane chain behind it starts late (between the steps of one graph they are
+// released together; us per step without / with: 29.1 / 27.3 on 45x37x29 cells, 51.4
+// / 50.7 at 64^3, 117 / 113 for twelve grids with 49 membranes).
+int order_behind_advect(lbfs_solver *s, cudaGraphNode_t advect) {
+    if (!advect) return LBFS_OK;
+    cudaGraphEdgeData e = {};
+    e.from_port = cudaGraphKernelNodePortLaunchCompletion;
+    e.type = cudaGraphDependencyTypeProgrammatic;
+    LBFS_CUDA(cudaStreamUpdateCaptureDependencies_v2(s->stream, &advect, &e, 1, cudaStreamAddCaptureDependencies));
+    return LBFS_OK;
+}
+
 // Joins the membrane stream to a capture behind the launch completion of the
 // handle's stream's last kernel (every block has begun).
 int fork_behind_launch(lbfs_solver *s) {
@@ -1413,6 +1440,7 @@ template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, i
     } else {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         LBFS_CUDA(cudaStreamIsCapturing(s->stream, &cap));
+        cudaGraphNode_t advect = nullptr;
         const bool behind = s->membrane_after_k1 && cap == cudaStreamCaptureStatusActive && !s->kernel_events;
         if (behind) {
             pass();
@@ -1424,10 +1452,13 @@ template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, i
         }
         {
             PhaseMark m(s, 0, s->stream2);
-            n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted);
+            n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted, false, &advect);
         }
         LBFS_CUDA(cudaEventRecord(s->ev_join, s->stream2));
-        if (!behind) pass();
+        if (!behind) {
+            if (int rc = order_behind_advect(s, advect)) return rc;
+            pass();
+        }
         LBFS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_join, 0));
     }
     { PhaseMark m(s, 3, s->stream); launch_fluid_update<R>(a, s->stream, !s->kernel_events); }
@@ -1461,10 +1492,11 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
             n += 3;
         } else {
             const bool spread_here = spread_with_faces<R>(s, a);
+            cudaGraphNode_t advect = nullptr;
             auto membranes = [&]() -> int {
                 {
                     PhaseMark m(s, 0, s->stream2);
-                    n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted, spread_here);
+                    n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted, spread_here, &advect);
                 }
                 LBFS_CUDA(cudaEventRecord(s->ev_join, s->stream2));
                 return LBFS_OK;
@@ -1488,6 +1520,9 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
                 LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
                 LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
                 if ((rc = membranes())) return rc;
+                // (gradient blocks that the SMs hold beside the membranes' take no one's place: 44.5 us a
+                // step without, 46.7 with, on 64,000 imported cells)
+                if (s->nc > 2 * 148 * a.tb_grad && (rc = order_behind_advect(s, advect))) return rc;
                 rc = enqueue_k1_k2<R>(s, a, &n, spread_here);
             }
             if (rc) return rc;
@@ -1750,30 +1785,86 @@ extern "C" int lbfs_step(lbfs_solver *s, int32_t n_steps) {
     return LBFS_OK;
 }
 
+namespace {
+// The regular step `steps` times as one graph.
+int build_step_graph(lbfs_solver *s, int steps, cudaGraphExec_t *graph) {
+    cudaGraph_t g = nullptr;
+    LBFS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = LBFS_OK;
+    for (int k = 0; k < steps && !rc; k++) {
+        int n = 0;
+        rc = enqueue(s, false, &n);
+    }
+    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    if (rc || e != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);  // a capture that ended but whose enqueue failed
+        if (rc) return rc;
+        return set_error(LBFS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    }
+    // keep the membrane kernels' launch priority inside the graph (without
+    // the flag every node runs at the priority of the stream it is launched into)
+    e = cudaGraphInstantiate(graph, g, cudaGraphInstantiateFlagUseNodePriority);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        *graph = nullptr;
+        return set_error(LBFS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+    }
+    return LBFS_OK;
+}
+
+// Steps of one graph launch: those of a call, up to kRunSteps.  Between two graphs
+// the GPU is idle for 2 to 5 us, between two steps of one graph it is not (us per
+// step, one step / up to 16 a graph: 16.5 / 14.2 on 32^3 cells, 31-34 / 27.4 on
+// 45x37x29 with a membrane, 46.3 / 44.5 on an imported mesh of 64,000 cells; 267 /
+// 269 at 128^3, where it is nothing).  A graph costs its capture and instantiation,
+// some 50 us a step, so it is made only when calls of one length have taken
+// kRunAfter steps, which is when it would have paid for itself.
+constexpr int kRunSteps = 16;
+constexpr long long kRunAfter = 256;
+
+void plan_step_run(lbfs_solver *s, lbfs_solver::StepRun *r, int n_steps) {
+    const int asked = std::min(n_steps, kRunSteps);
+    if (asked != r->asked) {
+        r->asked = asked;
+        r->taken = 0;
+    }
+    if (asked < 2 || asked == r->steps || r->failed || s->profiling || (r->taken += n_steps) <= kRunAfter) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;  // the caller may be capturing this call
+    if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
+    cudaGraphExec_t g = nullptr;
+    if (build_step_graph(s, asked, &g) != LBFS_OK) {  // one step at a time as before
+        cudaGetLastError();
+        r->failed = true;
+        return;
+    }
+    if (r->graph) cudaGraphExecDestroy(r->graph);
+    r->graph = g;
+    r->steps = asked;
+}
+}  // namespace
+
 extern "C" int lbfs_step_graph(lbfs_solver *s, int32_t n_steps) {
     if (!s || n_steps < 0) return set_error(LBFS_ERR_ARG, "bad arguments");
     LBFS_CUDA(cudaSetDevice(s->device));
     cudaGraphExec_t &graph = s->separate ? s->graph_separate : s->graph;
     if (!graph) {
-        cudaGraph_t g = nullptr;
-        LBFS_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        int n = 0;
-        int rc = enqueue(s, false, &n);
-        cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-        if (rc || e != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);  // a capture that ended but whose enqueue failed
-            if (rc) return rc;
-            return set_error(LBFS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-        }
-        // keep the membrane kernels' launch priority inside the graph (without
-        // the flag every node runs at the priority of the stream it is launched into)
-        e = cudaGraphInstantiate(&graph, g, cudaGraphInstantiateFlagUseNodePriority);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return set_error(LBFS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+        if (int rc = build_step_graph(s, 1, &graph)) return rc;
         s->graph_steps = 1;
         for (int p = 0; p < kPhases; p++) s->graph_phase_recorded[p] = s->phase_recorded[p];
     }
+    lbfs_solver::StepRun &run = s->separate ? s->run_separate : s->run;
+    plan_step_run(s, &run, n_steps);
     for (int k = 0; k < n_steps; k++) {
+        bool together = run.graph && !s->profiling && n_steps - k >= run.steps;
+        for (int q = 0; together && q < run.steps; q++) together = !visc_due(s, s->t + q) && !wrap_due(s, s->t + q);
+        if (together) {
+            LBFS_CUDA(cudaGraphLaunch(run.graph, s->stream));
+            for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = s->graph_phase_recorded[p];
+            note_steps(s);
+            s->t += run.steps;
+            k += run.steps - 1;
+            continue;
+        }
         if (visc_due(s, s->t)) {
             int rc = enqueue(s, true, nullptr);
             if (rc) return rc;

@@ -386,6 +386,34 @@ def test_membranes_behind_the_gradient_launch_are_bit_identical(precision, clust
     assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
 
 
+@pytest.mark.parametrize("n,precision,shape,period", [(32, 0, {}, 10000), (32, 1, {}, 10000), (32, 0, {}, 23),
+                                                     (32, 0, {"membrane_cluster": 8, "membrane_after_k1": 1}, 10000),
+                                                     (44, 1, {}, 10000)],
+                         ids=["fp64", "fp32", "viscosity_every_23", "fp64_cluster8_after_k1", "fp32_44"])
+def test_calls_of_several_steps_match_single_steps(n, precision, shape, period):
+    """Repeated calls of one length run their steps as one graph (a handle makes it after 256 steps of such
+    calls, of at most 16 steps); lengths that change, a rest shorter than the graph and the steps that stay
+    single (interior viscosity) go one graph a step.  The kernels and their order are the same, so states,
+    nodes and residual norms are those of single steps, bit for bit."""
+    c = cases.shear_rbc(n=n, level=2, radius_cells=5.0, precision=precision)
+    c.params.viscosity_period = period
+    calls = [10] * 30 + [23] * 2 + [7] * 40 + [40] * 8 + [1]
+    a, b = make(c), make(c)
+    for h in (a, b):
+        if shape:
+            h.set_launch_shape(**shape)
+    for k in calls:
+        a.step(k, graph=True)
+    for _ in range(sum(calls)):
+        b.step(1, graph=True)
+    assert a.status() == b.status()
+    for x, y in zip(a.state(), b.state()):
+        assert np.array_equal(x, y)
+    assert np.array_equal(a.nodes(), b.nodes()) and np.array_equal(a.residuals(), b.residuals())
+    a.close()
+    b.close()
+
+
 @pytest.mark.parametrize("precision,shape,period", [(0, {}, 10000), (1, {}, 10000),
                                                    (0, {"membrane_cluster": 8, "membrane_after_k1": 1}, 10000),
                                                    (0, {}, 7)],
