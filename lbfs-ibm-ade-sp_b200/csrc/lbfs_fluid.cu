@@ -70,9 +70,11 @@ __global__ void __launch_bounds__(TB, (sizeof(R) == 4 ? 1024 : 640) / TB) k_face
 // takes the faces owned by the TB cells of tile tile0 + b, in up to three
 // face ranges ordered by owner (the generator's x, y, z faces; an imported
 // mesh's internal faces, which OpenFOAM orders by owner, form one range).
-// FP64 at 128 registers (16 warps per SM; at 96 it spills 1.4 KB a thread), FP32 at 64 (32 warps
-// per SM, 44 B spilled; 6 % faster than at 80 registers and 24 warps).
-template <typename R, int TB>
+// FP64 at 128 registers (16 warps per SM), FP32 at 64 (32 warps per SM).  CONE: three ranges, so that a
+// warp's faces are of one axis (general_face_flux); an imported mesh's one range mixes them and would
+// only pay for the votes (44.4 / 44.9 us a step on 64,000 cells; its faces taken axis by axis through
+// an index list: 48.5).
+template <typename R, int TB, bool CONE>
 __global__ void __launch_bounds__(TB, (sizeof(R) == 4 ? 1024 : 512) / TB) k_face_flux_general_tiles(FluidArgs<R> a, int tile0) {
     pdl_trigger();
     pdl_wait();  // the gradients
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(TB, (sizeof(R) == 4 ? 1024 : 512) / TB) k_face
 #pragma unroll 1
     for (int r = 0; r < 3; r++) {
         const int f0 = __ldg(tp + r), f1 = __ldg(tp + 3 + r);
-        for (int f = f0 + (int)threadIdx.x; f < f1; f += TB) a.flux[f] = general_face_flux<R>(a, f, false);
+        for (int f = f0 + (int)threadIdx.x; f < f1; f += TB) a.flux[f] = general_face_flux<R, CONE>(a, f, false);
     }
 }
 
@@ -91,7 +93,7 @@ template <typename R, int TB>
 __global__ void __launch_bounds__(TB) k_face_flux_general(FluidArgs<R> a, int first) {
     const int f = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= a.nf) return;
-    a.flux[f] = general_face_flux<R>(a, f, f >= a.ni);
+    a.flux[f] = general_face_flux<R, false>(a, f, f >= a.ni);
 }
 
 // ----------------------------------------------------------------- CFL ----
@@ -419,14 +421,22 @@ void launch_maybe_pdl(void (*kernel)(KArgs...), int g, int tb, cudaStream_t s, b
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+template <typename R, bool CONE>
+void launch_general_tiles(const FluidArgs<R> &a, int g, int tile0, cudaStream_t s, bool pdl) {
+    if (a.tb_gen == 64) launch_maybe_pdl(k_face_flux_general_tiles<R, 64, CONE>, g, 64, s, pdl, a, tile0);
+    else if (a.tb_gen == 256) launch_maybe_pdl(k_face_flux_general_tiles<R, 256, CONE>, g, 256, s, pdl, a, tile0);
+    else launch_maybe_pdl(k_face_flux_general_tiles<R, 128, CONE>, g, 128, s, pdl, a, tile0);
+}
+
 template <typename R>
 void launch_fluid_flux_tiles(const FluidArgs<R> &a, int tile0, int tile1, cudaStream_t s, bool pdl) {
     const int g = tile1 - tile0;
     if (g <= 0) return;
     if (!a.axis_aligned) {
-        if (a.tb_gen == 64) launch_maybe_pdl(k_face_flux_general_tiles<R, 64>, g, 64, s, pdl, a, tile0);
-        else if (a.tb_gen == 256) launch_maybe_pdl(k_face_flux_general_tiles<R, 256>, g, 256, s, pdl, a, tile0);
-        else launch_maybe_pdl(k_face_flux_general_tiles<R, 128>, g, 128, s, pdl, a, tile0);
+        if (a.nfx >= 0 && a.nfy >= 0 && a.nfz >= 0 && (long long)a.nfx + a.nfy + a.nfz == a.ni)
+            launch_general_tiles<R, true>(a, g, tile0, s, pdl);
+        else
+            launch_general_tiles<R, false>(a, g, tile0, s, pdl);
         return;
     }
     if (a.tb_flux == 64) launch_maybe_pdl(k_face_flux_tiles<R, 64>, g, 64, s, pdl, a, tile0);

@@ -75,6 +75,35 @@ def test_jittered_channel_with_red_cell_matches_oracle():
     assert rel_err(nodes, o.nodes()) <= FP64_RTOL
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [(9, 7, 5), (131, 2, 3), (2, 3, 70)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("jitter", [0.02, 0.24])
+def test_faces_within_an_axis_cone_match_oracle(jitter, size):
+    """Interior faces whose normals a warp finds within one axis' cone take the closed form of the corner
+    sums and choose the sides of the tangential directions by the normal's signs: with 2 % jitter some
+    lie near the threshold, with 24 % (where n_A - |n_B| - |n_C| comes down to 0.39) few.  The sizes end
+    inside a tile of 128 cells, a few cells over one and within a warp.  The oracle sums the directions
+    one by one: other roundings only (FP64 parity bound)."""
+    from dataclasses import replace
+    from lbfs_b200 import GpuSolver, cases
+    from oracle_lbfs import OracleSolver
+    c = cases.poiseuille(n=size[0], ny=size[1], nz=size[2])
+    c.params = replace(c.params, gamma_inv=0.5, preconditioning=1)
+    m = _mesh(jitter, n=size)
+    m.set_boundaries(c.bcs)
+    rng = np.random.default_rng(3)
+    state = [c.rho] + [0.01 * rng.uniform(-1, 1, m.n_cells) for _ in range(3)]
+    with GpuSolver(m, c.params) as s:
+        s.set_state(*state)
+        s.step(5, graph=True)
+        got = s.state()
+    o = OracleSolver(m, c.params, [])
+    o.set_state(*state)
+    o.step(5)
+    for a, b in zip(got, o.state()):
+        assert rel_err(a, b) <= FP64_RTOL
+
+
 def test_jittered_box_at_rest_stays_at_rest():
     """With the faces' vector areas closing around every cell, a fluid at rest
     in a closed jittered box feels no net pressure force (oracle, CPU)."""
