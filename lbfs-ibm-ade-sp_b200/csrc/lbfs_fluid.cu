@@ -314,15 +314,16 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
         if (lane == 0) sh[m][warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int m = 0; m < 4; m++) {
+    if (warp == 0) {
+        if (lane < 4) {
             double v = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += sh[m][w];
-            a.partials[4 * blockIdx.x + m] = v;
+#pragma unroll
+            for (int w = 0; w < TB / 32; w++) v += sh[lane][w];
+            a.partials[4 * blockIdx.x + lane] = v;
+            __threadfence();
         }
-        __threadfence();
-        const unsigned int prev = atomicAdd(a.ticket, 1u);
-        last_block = (prev == gridDim.x - 1);
+        __syncwarp();
+        if (lane == 0) last_block = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (last_block) {

@@ -527,7 +527,9 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     LBFS_CUDA(cudaMemset(d_rsum, 0, 4 * sizeof(double)));
     a.partials = d_partials; a.residual_sums = d_rsum; a.ticket = d_ticket; a.flags = d_flags;
     a.res_out = nullptr;
-    a.tb_grad = 256; a.tb_flux = 128; a.tb_gen = 128; a.tb_update = 256; a.update_blocks = kK3MaxBlocks;
+    // gradients: 128 threads at 102 registers, five blocks an SM, against two of 256 at 106 (us per step: periodic
+    // 57x45x33 FP32 19.6 / 20.7, twelve grids 109.1 / 111.3, jittered 128^3 FP32 337.6 / 346.1; 72^3 FP64 the same)
+    a.tb_grad = 128; a.tb_flux = 128; a.tb_gen = 128; a.tb_update = 256; a.update_blocks = kK3MaxBlocks;
     a.n_membranes = 0;
     a.instances = nullptr;
     a.cell_instance = nullptr;
@@ -1520,9 +1522,9 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
                 LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
                 LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
                 if ((rc = membranes())) return rc;
-                // (gradient blocks that the SMs hold beside the membranes' take no one's place: 44.5 us a
-                // step without, 46.7 with, on 64,000 imported cells)
-                if (s->nc > 2 * 148 * a.tb_grad && (rc = order_behind_advect(s, advect))) return rc;
+                // (gradient blocks that the SMs hold at once take no one's place: 44.5 us a step without, 46.7
+                // with, on 64,000 imported cells)
+                if (s->nc > 2 * 148 * 256 && (rc = order_behind_advect(s, advect))) return rc;
                 rc = enqueue_k1_k2<R>(s, a, &n, spread_here);
             }
             if (rc) return rc;
