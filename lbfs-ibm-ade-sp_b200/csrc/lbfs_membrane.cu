@@ -886,12 +886,27 @@ __device__ void sort_patch(const MembraneArgs &A, int m, const double *red, bool
     // Bins are full where a membrane is fine against the grid: an insertion sort by one thread per
     // bin was quadratic in a serial chain there (49 membranes of radius 1.5 to 4 cells: 57.8 us).
     for (int ln = threadIdx.x; ln < mc.n_nodes; ln += blockDim.x) {
+        const size_t n = mc.node0 + ln;
+        const int base = __ldcg(A.node_base + 3 * n);  // in flight beside the count
+        double2 w[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+            w[q] = (q & 1) && S == 2 ? make_double2(0.0, 0.0)
+                                     : __ldcg(reinterpret_cast<const double2 *>(A.node_w + 12 * n) + q);
         const int b = bins[ln];
         const int lo = b == 0 ? 0 : (in_smem ? cur[b - 1] : __ldcg(cur + b - 1));
         const int hi = in_smem ? cur[b] : __ldcg(cur + b);  // global cursors were moved by atomics
         int place = lo;
         for (int i = lo; i < hi; i++) place += list[i] < ln ? 1 : 0;
-        A.sorted_node[mc.node0 + place] = mc.node0 + ln;
+        const size_t e = mc.node0 + place, N = A.total_nodes;
+        A.sorted_node[e] = (int)n;
+        A.sorted_base[e] = base;
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+            if ((q & 1) && S == 2) continue;  // two weights an axis
+            A.sorted_w[2 * q * N + e] = w[q].x;
+            A.sorted_w[(2 * q + 1) * N + e] = w[q].y;
+        }
     }
 }
 
@@ -1095,11 +1110,12 @@ size_t step_smem_bytes(int sort_capacity, int max_nodes) {
 // of bins (rows in (z, y) order, each row a contiguous range of the sorted
 // nodes); lane q of the warp takes contributions q, q + 32, ... of that list,
 // then the warp adds the lanes in a fixed tree.  All nodes of a row share the
-// stencil's y and z offsets, and a node's record carries its first x cell, so
-// the loads of one contribution do not wait on each other.  Bound by the latency of
-// those lookups, most of it in cells that few nodes reach (a warp per row of cells
-// that takes its nodes one after the other: 180 us a step for twelve grids with 49
-// membranes against 120).
+// stencil's y and z offsets; their weights and first x cells come from copies in
+// sorted order, so that neighbouring lanes share sectors and only the forces are
+// gathered.  Bound by those sectors where a membrane is fine against its grid (62
+// contributions a cell for the 49 membranes of twelve grids: 109.3 us a step with every
+// node's record gathered, 103.6 with the copies), else by the lookups' latency.  A
+// warp per row of cells that takes its nodes one after the other: 180 us.
 template <int S>
 __global__ void __launch_bounds__(256) k_mem_spread(MembraneArgs A) {
     pdl_wait();
@@ -1152,7 +1168,9 @@ __global__ void __launch_bounds__(256) k_mem_spread(MembraneArgs A) {
             if (lane >= o) end += x;
         }
         const int count = __shfl_sync(0xffffffffu, end, S * S - 1);
-        const int *sorted = A.sorted_node + mc.node0;
+        const int *sorted = A.sorted_node + mc.node0, *base = A.sorted_base + mc.node0;
+        const double *weight = A.sorted_w + mc.node0;
+        const size_t N = A.total_nodes;
 
         double inv3 = 1 / mc.gdx / mc.gdx / mc.gdx;
         if (A.ibm_stencil == LBFS_IBM_VANDERMONDE4) {
@@ -1175,10 +1193,10 @@ __global__ void __launch_bounds__(256) k_mem_spread(MembraneArgs A) {
             if (q < count) {
                 const int e = r_lo + q - (r_end - r_len);
                 const int node = __ldg(sorted + e);
-                const double *w = A.node_w + 12 * (size_t)node;
                 const double3 F = make_double3(__ldg(A.fx + node), __ldg(A.fy + node), __ldg(A.fz + node));
-                const double wy = __ldg(w + 4 + S - 1 - r % S), wz = __ldg(w + 8 + S - 1 - r / S);
-                const double wx = __ldg(w + ci - __ldg(A.node_base + 3 * (size_t)node));
+                const double wy = __ldg(weight + (4 + S - 1 - r % S) * N + e);
+                const double wz = __ldg(weight + (8 + S - 1 - r / S) * N + e);
+                const double wx = __ldg(weight + (size_t)(ci - __ldg(base + e)) * N + e);
                 const double w3 = wx * wy * wz;
                 f[0] += F.x * w3;
                 f[1] += F.y * w3;

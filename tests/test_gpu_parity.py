@@ -170,6 +170,30 @@ def test_spread_of_full_sort_bins(level, radius, ibm):
     assert np.max(np.abs(fields[0] - want)) <= 1e-12 * size.max()
 
 
+@pytest.mark.parametrize("count", [32, 33])
+def test_many_membranes_vs_oracle(count, monkeypatch):
+    # the separate kernels' spread follows the boundary faces up to 32 membranes and the node forces beyond;
+    # the state after four graph steps against the oracle (FP64 parity bound)
+    monkeypatch.setenv("LBFS_SEPARATE_KERNELS", "1")
+    from lbfs_b200 import red_cell
+    c = cases.shear_rbc(n=20, level=1, radius_cells=2.0, ibm_stencil=_abi.LBFS_IBM_PESKIN4)
+    first = c.membranes[0]
+    moduli = {k: getattr(first, k) for k in ("volume_modulus", "local_area_modulus", "global_area_modulus",
+                                             "shear_modulus", "global_bending_modulus", "wlc_ratio",
+                                             "internal_viscosity_ratio")}
+    centres = np.random.default_rng(4).uniform(0.3, 0.7, (count, 3)) * c.mesh.X
+    c.membranes = [red_cell(1, 4.0, tuple(x), **moduli) for x in centres]
+    s, o = make(c), make(c, OracleSolver)
+    s.step(4, graph=True)
+    o.step(4)
+    for x, y in zip(s.state(), o.state()):
+        assert rel_err(x, y) < FP64_RTOL
+    assert rel_err(s.nodes(), o.nodes()) < FP64_RTOL
+    assert s.status() == 0
+    s.close()
+    o.close()
+
+
 def test_interior_viscosity_l4_vs_oracle():
     # the binned interior-viscosity test (triangles binned by their y-z boxes) against the oracle's
     # test of every triangle: a rotated L4 cell (5120 triangles over many bins), 805 cells inside;
