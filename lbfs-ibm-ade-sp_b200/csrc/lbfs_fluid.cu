@@ -145,6 +145,30 @@ __global__ void __launch_bounds__(256) k_cfl(FluidArgs<R> a) {
 
 // ------------------------------------------------------------------ K3 ----
 
+// The convergence test of the reference's loop (Solver_gpu.cu:1206-1208:
+// convergence_residual.max_error() < tolerance) on the step's residual norms,
+// formed as lbfs_get_residuals forms them, and the drop-in's divergence test
+// (non-finite state or density out of range); sets the while node's condition.
+// Lanes 0 to 3 of one warp bring the sums.  In the update's last block: a kernel of
+// its own behind it cost 0.8 to 1.2 us a step of the loop (32^3 18.6 / 17.8 us,
+// 45x37x29 with a membrane 31.5 / 30.3).
+template <typename R> __device__ __forceinline__ void until_check(const FluidArgs<R> &a, double sum, int lane) {
+    UntilState *u = a.until.u;
+    const double r = sqrt(sum / (double)a.nc) / (lane == 0 ? a.until.ref_rho : a.until.ref_mom);
+    if (lane < 4) u->res[lane] = r;
+    const double r0 = __shfl_sync(0xffffffffu, r, 0), r1 = __shfl_sync(0xffffffffu, r, 1);
+    const double r2 = __shfl_sync(0xffffffffu, r, 2), r3 = __shfl_sync(0xffffffffu, r, 3);
+    if (lane != 0) return;
+    const double m01 = r0 < r1 ? r1 : r0, m23 = r2 < r3 ? r3 : r2;  // std::max
+    const double mx = m01 < m23 ? m23 : m01;
+    const bool converged = mx < u->tol;
+    const bool diverged = (__ldcg(a.flags) & (LBFS_FLAG_NONFINITE | LBFS_FLAG_RHO_RANGE)) != 0u;
+    const int c = u->count + 1;
+    u->count = c;
+    u->stop = converged ? 1 : (diverged ? 2 : 0);
+    cudaGraphSetConditional(a.until.handle, (!converged && !diverged && c < u->limit) ? 1u : 0u);
+}
+
 // GRID: behind the fused step, whose cell sums over the interior faces it
 // reads (32 B instead of six fluxes of 32 / 16 B), adding the boundary faces,
 // whose indices follow the interior ones: the sum order of the gather.
@@ -343,12 +367,15 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
             if (lane == 0) sh[m][warp] = v;
         }
         __syncthreads();
-        if (threadIdx.x < 4) {
+        if (warp == 0) {
             double v = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += sh[threadIdx.x][w];
-            a.residual_sums[threadIdx.x] = v;
+            if (lane < 4) {
+                for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += sh[lane][w];
+                a.residual_sums[lane] = v;
+            }
+            if (lane == 0) *a.ticket = 0u;
+            if (a.until.u) until_check(a, v, lane);
         }
-        if (threadIdx.x == 0) *a.ticket = 0u;
     }
 }
 

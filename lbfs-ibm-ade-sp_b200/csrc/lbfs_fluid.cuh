@@ -172,6 +172,21 @@ __host__ __device__ inline void grid_cell_faces(int c, int nx, int ny, int nz, i
     for (int q = 0; q < 6; q++) cf[q] = sg[q] * (f[q] + 1);
 }
 
+// Device record of lbfs_step_until's loop: steps taken in this launch, their limit, the tolerance,
+// the last step's residual norms and why the loop stopped (0 limit, 1 converged, 2 diverged).
+struct UntilState {
+    int count, limit, stop, pad;
+    double tol;
+    double res[4];
+};
+
+// Where the step is the body of that loop: the update's last block makes the test (u null otherwise).
+struct UntilArgs {
+    UntilState *u;
+    cudaGraphConditionalHandle handle;
+    double ref_rho, ref_mom;
+};
+
 template <typename R> struct FluidArgs {
     int nc, nf, ni, nb, nfx, nfy, nfz, axis_aligned;
     int testcase;
@@ -257,6 +272,7 @@ template <typename R> struct FluidArgs {
     unsigned int *ticket;
     double *residual_sums;       // [4] sum of squares of the last step
     unsigned int *flags;
+    UntilArgs until;
     // launch shape (read by the host launchers only; lbfs_autotune picks it)
     int tb_grad, tb_flux, tb_gen, tb_update, update_blocks;
     // time stepping other than constant (get_cfl_device, LBFS.cu:2868-2932)

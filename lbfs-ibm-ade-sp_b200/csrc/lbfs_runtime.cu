@@ -102,7 +102,7 @@ struct lbfs_solver {
     // lbfs_step_until: one graph whose while node repeats the step and a convergence check
     cudaGraphExec_t loop_graph = nullptr;
     bool loop_unavailable = false;  // the loop graph could not be built (steps go one at a time)
-    struct UntilState *d_until = nullptr;
+    UntilState *d_until = nullptr;
     int launches_per_step = 0;
     // per-kernel timing: start/stop events per phase (membrane, gradients, flux, update, viscosity)
     bool profiling = false;    // step events (level >= 1)
@@ -143,14 +143,6 @@ struct lbfs_solver {
     }
 };
 
-// Device record of lbfs_step_until's loop: steps taken in this launch, their limit, the tolerance,
-// the last step's residual norms and why the loop stopped (0 limit, 1 converged, 2 diverged).
-struct UntilState {
-    int count, limit, stop, pad;
-    double tol;
-    double res[4];
-};
-
 namespace {
 
 // time stepping other than constant (lbfs_params.time_stepping 1, 3, 4)
@@ -166,28 +158,6 @@ void drop_step_graphs(lbfs_solver *s) {
     if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; s->graph_steps = 0; }
     if (s->graph_separate) { cudaGraphExecDestroy(s->graph_separate); s->graph_separate = nullptr; }
     if (s->loop_graph) { cudaGraphExecDestroy(s->loop_graph); s->loop_graph = nullptr; }
-}
-
-// The convergence test of the reference's loop (Solver_gpu.cu:1206-1208:
-// convergence_residual.max_error() < tolerance) on the step's residual norms,
-// formed as lbfs_get_residuals forms them, and the drop-in's divergence test
-// (non-finite state or density out of range); sets the while node's condition.
-__global__ void k_until_check(cudaGraphConditionalHandle h, UntilState *u, const double *sums, const unsigned int *flags,
-                              double nc, double ref_rho, double ref_mom) {
-    if (threadIdx.x != 0) return;
-    double r[4];
-    for (int k = 0; k < 4; k++) {
-        r[k] = sqrt(sums[k] / nc) / (k == 0 ? ref_rho : ref_mom);
-        u->res[k] = r[k];
-    }
-    const double m01 = r[0] < r[1] ? r[1] : r[0], m23 = r[2] < r[3] ? r[3] : r[2];  // std::max
-    const double mx = m01 < m23 ? m23 : m01;
-    const bool converged = mx < u->tol;
-    const bool diverged = (*flags & (LBFS_FLAG_NONFINITE | LBFS_FLAG_RHO_RANGE)) != 0u;
-    const int c = u->count + 1;
-    u->count = c;
-    u->stop = converged ? 1 : (diverged ? 2 : 0);
-    cudaGraphSetConditional(h, (!converged && !diverged && c < u->limit) ? 1u : 0u);
 }
 
 // Device buffer freed when it leaves scope (temporary storage).
@@ -1886,7 +1856,7 @@ extern "C" int lbfs_step_graph(lbfs_solver *s, int32_t n_steps) {
 
 namespace {
 // The loop graph of lbfs_step_until: a while node whose body is one regular step (as the step graph
-// captures it) followed by k_until_check.  Returns LBFS_OK with s->loop_unavailable set when the
+// captures it) whose update ends with the convergence test.  Returns LBFS_OK with s->loop_unavailable set when the
 // driver refuses the body (the caller then steps one graph at a time).
 int build_loop_graph(lbfs_solver *s) {
     if (!s->d_until) {
@@ -1918,14 +1888,14 @@ int build_loop_graph(lbfs_solver *s) {
         s->loop_unavailable = true;
         return LBFS_OK;
     }
+    auto until = [&](UntilState *u) {
+        for (UntilArgs *t : {&s->f64.until, &s->f32.until})
+            *t = {u, h, s->params.ref_rho, s->params.ref_rho * s->params.max_velocity};
+    };
     int n = 0;
+    until(s->d_until);
     int rc = enqueue(s, false, &n);
-    if (!rc) {
-        const double ref_mom = s->params.ref_rho * s->params.max_velocity;
-        k_until_check<<<1, 32, 0, s->stream>>>(h, s->d_until, s->fp32 ? s->f32.residual_sums : s->f64.residual_sums,
-                                               s->fp32 ? s->f32.flags : s->f64.flags, (double)s->nc, s->params.ref_rho,
-                                               ref_mom);
-    }
+    until(nullptr);
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(s->stream, &captured);
     if (rc) {
