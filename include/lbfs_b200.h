@@ -203,7 +203,8 @@ int lbfs_get_state(lbfs_solver *s, double *rho, double *u, double *v, double *w)
 /* Advance n_steps time steps (one iteration of Solver_gpu.cu:749-1046 each).
  * Enqueued on the solver's stream; returns without waiting. */
 int lbfs_step(lbfs_solver *s, int32_t n_steps);
-/* Same, with the per-step work replayed from a CUDA graph captured on first use. */
+/* Same, with the per-step work replayed from a CUDA graph captured on first use; calls of one
+ * length that repeat (256 steps of them) replay up to 16 regular steps per graph. */
 int lbfs_step_graph(lbfs_solver *s, int32_t n_steps);
 int lbfs_synchronize(lbfs_solver *s);
 /* The reference's time loop with its convergence test (Solver_gpu.cu:1206-1208:
