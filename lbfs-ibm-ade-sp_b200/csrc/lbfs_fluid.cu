@@ -170,8 +170,8 @@ template <typename R> __device__ __forceinline__ void until_check(const FluidArg
 }
 
 // GRID: behind the fused step, whose cell sums over the interior faces it
-// reads (32 B instead of six fluxes of 32 / 16 B), adding the boundary faces,
-// whose indices follow the interior ones: the sum order of the gather.
+// reads (32 B instead of six fluxes of 32 / 16 B).  It subtracts the upper faces
+// that other tiles formed, z, x, y, scales the sum and adds the boundary faces.
 template <typename R, int TB, bool GRID>
 __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
     __shared__ double sh[4][TB / 32];
@@ -216,6 +216,26 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
             const double4 q = a.grid_res[i];
             r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
             const unsigned sides = a.grid_sides[i];
+            if (sides & 14u) {  // upper faces that another tile formed: z first, as a walk subtracts it
+                int sy = a.grid_stride[0], sz = a.grid_stride[1];
+                if (sy == 0) {
+                    const int2 q = a.grid_strides[__ldg(a.grid_instance + i)];
+                    sy = q.x;
+                    sz = q.y;
+                }
+#pragma unroll
+                for (int e = 0; e < 3; e++) {
+                    const int d = (e + 2) % 3;
+                    if (!(sides >> (d + 1) & 1u)) continue;
+                    const Vec4<R> fx = a.grid_edge[(size_t)d * a.nc + i + (d == 0 ? 1 : (d == 1 ? sy : sz))];
+                    const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
+#pragma unroll
+                    for (int m = 0; m < 4; m++) r[m] = r[m] - fv[m];
+                }
+            }
+            const double ia = iv * a.grid_area;
+#pragma unroll
+            for (int m = 0; m < 4; m++) r[m] = __dmul_rn(r[m], ia);  // not contracted with what follows, whatever that is
             if (sides & 1u) {
                 for (int e = 0; e < 6; e++) {
                     const int f = __ldg(a.cell_faces + 6 * (size_t)i + e) - 1;
@@ -224,23 +244,6 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
                     const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
 #pragma unroll
                     for (int m = 0; m < 4; m++) r[m] = r[m] + (-fv[m] * iv);
-                }
-            }
-            if (sides & 14u) {  // upper faces that another tile formed
-                int sy = a.grid_stride[0], sz = a.grid_stride[1];
-                if (sy == 0) {
-                    const int2 q = a.grid_strides[__ldg(a.grid_instance + i)];
-                    sy = q.x;
-                    sz = q.y;
-                }
-                const double ia = iv * a.grid_area;
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    if (!(sides >> (d + 1) & 1u)) continue;
-                    const Vec4<R> fx = a.grid_edge[(size_t)d * a.nc + i + (d == 0 ? 1 : (d == 1 ? sy : sz))];
-                    const double fv[4] = {(double)fx.rho, (double)fx.u, (double)fx.v, (double)fx.w};
-#pragma unroll
-                    for (int m = 0; m < 4; m++) r[m] = r[m] + (-fv[m] * ia);
                 }
             }
         } else {

@@ -60,7 +60,10 @@ template <typename R> __device__ __forceinline__ int bnd_before(const GridArgs<R
 // the three low faces of its cells, so all lanes work on every face; the high
 // faces of a tile and the upper ones of a walk are another block's low ones, which
 // it also leaves in ga.edge for the update to subtract (forming them here too, by a
-// warp of their own, cost a fifth: 265 against 203 us at 128^3 FP64).  Ghosts are
+// warp of their own, cost a fifth: 265 against 203 us at 128^3 FP64).  A walk
+// subtracts a cell's upper z flux last and scales nothing, and the update goes on
+// from there: the order of a cell's sum does not depend on where its walk ends,
+// which follows from all grids of the handle.  Ghosts are
 // cells of the ring: copied from the cell beside them (zero gradient) and, where
 // they are not, set from the side's record after the copy's arrival by the thread
 // that issued it.  Bound by FP64 issue inside the walk (of its cycles about three
@@ -635,16 +638,12 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
                 if (ly + 1 < t.h) v = v - (double)fy[m * TB + tid + t.w];
                 sum[m * TB + tid] = v;
             }
-            if (k > t.z0) {  // the cell below is complete
-                const double iv = __ldg(a.cell_inv_volume + c - nxy) * (double)ga.area;
-                ga.res[c - nxy] = make_double4(below_sum[0] * iv, below_sum[1] * iv, below_sum[2] * iv, below_sum[3] * iv);
-            }
+            if (k > t.z0)  // the cell below is complete
+                ga.res[c - nxy] = make_double4(below_sum[0], below_sum[1], below_sum[2], below_sum[3]);
         }
     }
     if (own) {  // the last cell's upper face belongs to the walk above (or there is none)
-        const int c = c00 + nxy * (z_end - 1);
-        const double iv = __ldg(a.cell_inv_volume + c) * (double)ga.area;
-        ga.res[c] = make_double4(sum[tid] * iv, sum[TB + tid] * iv, sum[2 * TB + tid] * iv, sum[3 * TB + tid] * iv);
+        ga.res[c00 + nxy * (z_end - 1)] = make_double4(sum[tid], sum[TB + tid], sum[2 * TB + tid], sum[3 * TB + tid]);
     }
 }
 

@@ -68,7 +68,7 @@ template <typename R> struct GridArgs {
     GridWeights<R> cw;
     R area, dt;                    // of every interior face
     Vec4<R> *prev;                 // [nc + nb] the state the last step started from
-    double4 *res;                  // [nc] sums of the interior face fluxes (rho, u, v, w)
+    double4 *res;                  // [nc] sums of the interior face fluxes per unit area, those in edge left out
     Vec4<R> *edge;                 // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes
     const unsigned char *sides;    // [nc] bit 0: the cell has boundary faces; bits 1, 2, 3: its upper x, y, z flux is in edge
 };

@@ -1,0 +1,76 @@
+"""The order of a cell's sums on uniform FP64 grids does not depend on how the fused pass cuts its tiles.
+
+The pass walks tiles of columns over some planes; how long the walks are follows from all instances of a
+handle together.  A cell whose upper neighbour lies in another walk takes that face's flux in the update
+instead of inside the walk.  An instance of an ensemble and a slab of a mesh must evolve bit for bit as
+they do in a handle of their own, so both places keep one order of sums.  The sizes are walked over
+different lengths by the handles compared (more than one plane each), and at spacing 1.5 the ratio of
+area and volume is no power of two, so that another place of the scaling shows in the last bits.
+"""
+import numpy as np
+import pytest
+
+from lbfs_b200 import GpuSolver, StepParams, build_uniform_mesh
+from lbfs_b200.ensemble import concatenate
+from lbfs_b200.slabs import SlabSolver, build_slab_mesh, slab_bounds, step_local
+
+pytestmark = pytest.mark.gpu
+
+WALL, OPEN = (2, 1, 1.0, 0.0, 0.0, 0.0), (2, 2, 1.0, 0.0, 0.0, 0.0)
+MOVING = (2, 1, 1.0, 0.01, 0.002, -0.003)
+BCS = {"left": OPEN, "right": OPEN, "bottom": WALL, "top": MOVING, "back": WALL, "front": MOVING}
+# a force that does not fit in few bits, so that sums of the same terms in another order differ
+PARAMS = StepParams(visc=0.1, delta_t=0.35, channel_diameter=64.0, body_force=(1e-5 / 3, -1e-6 / 7, 1e-6 / 11),
+                    ref_rho=1.0, max_velocity=0.01, rho0=1.0, visc_factor_initial=1.0, testcase=2, viscosity_period=0)
+
+
+def _box(n, spacing):
+    m = build_uniform_mesh(*(spacing * k for k in n), 0.5 * spacing, visc=PARAMS.visc)
+    m.set_boundaries(BCS)
+    return m
+
+
+def _state(n_cells, seed):
+    rng = np.random.default_rng(seed)
+    return [rng.uniform(0.99, 1.01, n_cells)] + [rng.uniform(-0.01, 0.01, n_cells) for _ in range(3)]
+
+
+def _run(mesh, state, steps=4):
+    with GpuSolver(mesh, PARAMS) as s:
+        s.set_state(*state)
+        s.step(steps, graph=True)
+        assert s.launches_per_step() == 2  # the fused pass and the update
+        assert s.status() == 0
+        return s.state()
+
+
+@pytest.mark.parametrize("spacing", [2.0, 1.5])
+@pytest.mark.parametrize("sizes", [((40, 40, 40), (44, 44, 44)), ((48, 47, 45), (40, 41, 66), (63, 50, 49))],
+                         ids=["40_44", "three"])
+def test_instances_equal_handles_of_their_own(sizes, spacing):
+    meshes = [_box(n, spacing) for n in sizes]
+    states = [_state(m.n_cells, 5 + k) for k, m in enumerate(meshes)]
+    e = concatenate(meshes)
+    got = _run(e, [np.concatenate(q) for q in zip(*states)])
+    for k, (m, st) in enumerate(zip(meshes, states)):
+        for a, b in zip(got, _run(m, st)):
+            assert np.array_equal(e.split(a)[k], b), k
+
+
+@pytest.mark.parametrize("spacing", [2.0, 1.5])
+def test_slabs_equal_the_whole_mesh(spacing):
+    n, nz = 64, 128
+    mesh = _box((n, n, nz), spacing)
+    state = _state(mesh.n_cells, 3)
+    want = _run(mesh, state)
+    bounds = slab_bounds(nz, 2)
+    slabs = []
+    for r in range(2):
+        slab = build_slab_mesh(n * spacing, n * spacing, nz * spacing, 0.5 * spacing, bounds, r, bcs=BCS, visc=PARAMS.visc)
+        slabs.append(SlabSolver(slab, PARAMS))
+        slabs[-1].set_state(*state)
+    step_local(slabs, 4, "cuda:0")
+    for s, (z0, z1) in zip(slabs, bounds):
+        for a, b in zip(s.owned_state(), want):
+            assert np.array_equal(a, b[z0 * n * n:z1 * n * n])
+        s.solver.close()
