@@ -91,7 +91,7 @@ struct MembraneArgs {
     double *node_w;              // [12 total_nodes] 1D stencil weights per axis (4 slots) at the current positions
     int *sorted_node;            // [total_nodes] each membrane's nodes in (bin, node) order, from node0
     int *sorted_base;            // [total_nodes] their first x cells and [12][total_nodes] their weights in that
-    double *sorted_w;            // order: the spread's lanes take neighbours in it (sort_patch)
+    double *sorted_w;            // order, for the spread (null: it gathers them by node)
     // LBFS_IBM_VANDERMONDE4 (rectilinear meshes, one instance): per axis the
     // vertex coordinates [n + 1] and the centroid coordinate of each cell row [n]
     // (centroid[i].x, centroid[j nx].y, centroid[k nx ny].z), and the cell volumes

@@ -885,20 +885,47 @@ __device__ void sort_patch(const MembraneArgs &A, int m, const double *red, bool
     // (after the placement cur[b] is the end of bin b, the start of bin b + 1), one thread per node.
     // Bins are full where a membrane is fine against the grid: an insertion sort by one thread per
     // bin was quadratic in a serial chain there (49 membranes of radius 1.5 to 4 cells: 57.8 us).
+    // Four nodes per round where nothing is copied (a membrane of 2562 nodes in the cluster step's 128
+    // threads).
+    auto range_of = [&](int b, int &lo, int &hi) {
+        lo = b == 0 ? 0 : (in_smem ? cur[b - 1] : __ldcg(cur + b - 1));
+        hi = in_smem ? cur[b] : __ldcg(cur + b);  // global cursors were moved by atomics
+    };
+    if (A.sorted_w == nullptr) {
+        for (int l0 = threadIdx.x; l0 < mc.n_nodes; l0 += 4 * blockDim.x) {
+            int lo[4], hi[4], place[4], most = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int ln = l0 + k * blockDim.x;
+                lo[k] = hi[k] = 0;
+                if (ln < mc.n_nodes) range_of(bins[ln], lo[k], hi[k]);
+                place[k] = lo[k];
+                most = max(most, hi[k] - lo[k]);
+            }
+            for (int i = 0; i < most; i++)
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (lo[k] + i < hi[k]) place[k] += list[lo[k] + i] < l0 + k * (int)blockDim.x ? 1 : 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int ln = l0 + k * blockDim.x;
+                if (ln < mc.n_nodes) A.sorted_node[mc.node0 + place[k]] = mc.node0 + ln;
+            }
+        }
+        return;
+    }
     for (int ln = threadIdx.x; ln < mc.n_nodes; ln += blockDim.x) {
-        const size_t n = mc.node0 + ln;
+        const size_t n = mc.node0 + ln, N = A.total_nodes;
         const int base = __ldcg(A.node_base + 3 * n);  // in flight beside the count
         double2 w[6];
 #pragma unroll
         for (int q = 0; q < 6; q++)
             w[q] = (q & 1) && S == 2 ? make_double2(0.0, 0.0)
                                      : __ldcg(reinterpret_cast<const double2 *>(A.node_w + 12 * n) + q);
-        const int b = bins[ln];
-        const int lo = b == 0 ? 0 : (in_smem ? cur[b - 1] : __ldcg(cur + b - 1));
-        const int hi = in_smem ? cur[b] : __ldcg(cur + b);  // global cursors were moved by atomics
-        int place = lo;
-        for (int i = lo; i < hi; i++) place += list[i] < ln ? 1 : 0;
-        const size_t e = mc.node0 + place, N = A.total_nodes;
+        int lo, hi;
+        range_of(bins[ln], lo, hi);
+        size_t e = mc.node0 + lo;
+        for (int i = lo; i < hi; i++) e += list[i] < ln ? 1 : 0;
         A.sorted_node[e] = (int)n;
         A.sorted_base[e] = base;
 #pragma unroll
@@ -1110,13 +1137,14 @@ size_t step_smem_bytes(int sort_capacity, int max_nodes) {
 // of bins (rows in (z, y) order, each row a contiguous range of the sorted
 // nodes); lane q of the warp takes contributions q, q + 32, ... of that list,
 // then the warp adds the lanes in a fixed tree.  All nodes of a row share the
-// stencil's y and z offsets; their weights and first x cells come from copies in
-// sorted order, so that neighbouring lanes share sectors and only the forces are
-// gathered.  Bound by those sectors where a membrane is fine against its grid (62
-// contributions a cell for the 49 membranes of twelve grids: 109.3 us a step with every
-// node's record gathered, 103.6 with the copies), else by the lookups' latency.  A
-// warp per row of cells that takes its nodes one after the other: 180 us.
-template <int S>
+// stencil's y and z offsets, and a node's record carries its first x cell, so the
+// loads of one contribution do not wait on each other.  COPIES (sorted_copies): the
+// weights and first x cells come from copies in sorted order, so that neighbouring
+// lanes share sectors and only the forces are gathered.  Bound by those sectors where
+// many membranes are fine against their grids (62 contributions a cell for the 49
+// membranes of twelve grids), else by the lookups' latency.  A warp per row of cells
+// that takes its nodes one after the other: 180 us.
+template <int S, bool COPIES>
 __global__ void __launch_bounds__(256) k_mem_spread(MembraneArgs A) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -1168,9 +1196,7 @@ __global__ void __launch_bounds__(256) k_mem_spread(MembraneArgs A) {
             if (lane >= o) end += x;
         }
         const int count = __shfl_sync(0xffffffffu, end, S * S - 1);
-        const int *sorted = A.sorted_node + mc.node0, *base = A.sorted_base + mc.node0;
-        const double *weight = A.sorted_w + mc.node0;
-        const size_t N = A.total_nodes;
+        const int *sorted = A.sorted_node + mc.node0;
 
         double inv3 = 1 / mc.gdx / mc.gdx / mc.gdx;
         if (A.ibm_stencil == LBFS_IBM_VANDERMONDE4) {
@@ -1194,9 +1220,11 @@ __global__ void __launch_bounds__(256) k_mem_spread(MembraneArgs A) {
                 const int e = r_lo + q - (r_end - r_len);
                 const int node = __ldg(sorted + e);
                 const double3 F = make_double3(__ldg(A.fx + node), __ldg(A.fy + node), __ldg(A.fz + node));
-                const double wy = __ldg(weight + (4 + S - 1 - r % S) * N + e);
-                const double wz = __ldg(weight + (8 + S - 1 - r / S) * N + e);
-                const double wx = __ldg(weight + (size_t)(ci - __ldg(base + e)) * N + e);
+                // weight k of the node at w[k * stride]
+                const size_t at = COPIES ? (size_t)(mc.node0 + e) : (size_t)node, stride = COPIES ? (size_t)A.total_nodes : 1;
+                const double *w = COPIES ? A.sorted_w + at : A.node_w + 12 * at;
+                const double wy = __ldg(w + (4 + S - 1 - r % S) * stride), wz = __ldg(w + (8 + S - 1 - r / S) * stride);
+                const double wx = __ldg(w + (ci - __ldg(COPIES ? A.sorted_base + at : A.node_base + 3 * at)) * stride);
                 const double w3 = wx * wy * wz;
                 f[0] += F.x * w3;
                 f[1] += F.y * w3;
@@ -1526,7 +1554,6 @@ int launch_membrane(const MembraneArgs &a, cudaStream_t s, cudaStream_t s_side, 
             st == cudaStreamCaptureStatusActive && nd == 1)
             *advect = deps[0];
     }
-    const dim3 spread_grid(a.spread_blocks);
     if (a.force_cluster == 8 || a.force_cluster == 16) {
         // totals, sort, spring and node forces as one cluster per membrane, then the spread
         const size_t fs = step_smem_bytes(a.sort_capacity, a.max_nodes);
@@ -1534,8 +1561,7 @@ int launch_membrane(const MembraneArgs &a, cudaStream_t s, cudaStream_t s_side, 
         if (a.force_cluster == 16) launch_hi(k_mem_step<16, kStepThreads>, grid, block, fs, s, a, 16, true);
         else launch_hi(k_mem_step<8, kStepThreads>, grid, block, fs, s, a, 8, true);
         if (without_spread) return 2;
-        if (stencil_width(a.ibm_stencil) == 4) launch_hi(k_mem_spread<4>, spread_grid, dim3(256), 0, s, a, 0, true);
-        else launch_hi(k_mem_spread<2>, spread_grid, dim3(256), 0, s, a, 0, true);
+        launch_membrane_spread(a, s, true);
         return 3;
     }
     // the node sort needs only the advected positions: side stream
@@ -1554,8 +1580,7 @@ int launch_membrane(const MembraneArgs &a, cudaStream_t s, cudaStream_t s_side, 
     // the spread reads the sorted node list and the node forces
     if (side) cudaStreamWaitEvent(s, ev_sorted, 0);
     if (without_spread) return n - 1;
-    if (stencil_width(a.ibm_stencil) == 4) launch_hi(k_mem_spread<4>, spread_grid, dim3(256), 0, s, a);
-    else launch_hi(k_mem_spread<2>, spread_grid, dim3(256), 0, s, a);
+    launch_membrane_spread(a, s, false);
     return n;
 }
 
@@ -1589,9 +1614,10 @@ void launch_membrane_wrap(const MembraneArgs &a, cudaStream_t s) {
 }
 
 void launch_membrane_spread(const MembraneArgs &a, cudaStream_t s, bool programmatic) {
-    const dim3 grid(a.spread_blocks);
-    if (stencil_width(a.ibm_stencil) == 4) launch_hi(k_mem_spread<4>, grid, dim3(256), 0, s, a, 0, programmatic);
-    else launch_hi(k_mem_spread<2>, grid, dim3(256), 0, s, a, 0, programmatic);
+    const bool copies = a.sorted_w != nullptr;
+    void (*k)(MembraneArgs) = stencil_width(a.ibm_stencil) == 4 ? (copies ? k_mem_spread<4, true> : k_mem_spread<4, false>)
+                                                                : (copies ? k_mem_spread<2, true> : k_mem_spread<2, false>);
+    launch_hi(k, dim3(a.spread_blocks), dim3(256), 0, s, a, 0, programmatic);
 }
 
 void launch_interior_viscosity(const ViscArgs &a, cudaStream_t s) {

@@ -116,6 +116,7 @@ struct lbfs_solver {
     std::vector<lbfs_grid_desc> grids;
     std::vector<InstanceGrid> inst;
     long long total_patch = 0;  // cells of all IBM patch slices
+    double *sorted_w = nullptr;  // the node sort's weight copies (sorted_copies), ma.sorted_w where it makes them
     // discrete adjoint: persistent buffers (allocated on first use)
     AdjointArgs adj{};
     bool adj_ready = false;
@@ -912,6 +913,17 @@ int setup_instances(lbfs_solver *s, const lbfs_mesh_desc *m) {
     return LBFS_OK;
 }
 
+// Whether the node sort leaves the nodes' weights in sorted order for the spread.  One block a
+// membrane copies them: nothing while it has a thread per node, else some 3 us per 1000 nodes of the
+// largest membrane (64^3 with one membrane of 2562 nodes: 68.2 us a step with the copies, 59.9
+// without; of 10242 nodes 154 / 92; 48^3 with one of 642 nodes 34.7 / 34.9).  The spread gains by the
+// nodes of all membranes (64^3, radius 3 cells, 2562 nodes each, with / without: two 81.8 / 75.8,
+// three 86.9 / 88.0, four 92.0 / 94.4, eight 110 / 121; radius 6: three 81.3 / 78.1, four 88.4 /
+// 85.3; 2-point stencil, four 71.8 / 72.4, eight 88.7 / 90.3).  Not in the cluster step, whose sort
+// has 128 threads (64^3 with 642 nodes: 60.8 / 56.1; 48^3 with 2562: 87.9 / 80.8).  Either way the
+// sums are the same.
+bool sorted_copies(int total_nodes, int max_nodes) { return max_nodes <= kMembraneThreads || total_nodes / 4 >= max_nodes; }
+
 int setup_membranes(lbfs_solver *s, const lbfs_mesh_desc *m, const lbfs_rbc_desc *rbc, int n_rbc) {
     const lbfs_params &p = s->params;
     MembraneArgs &ma = s->ma;
@@ -1033,6 +1045,7 @@ int setup_membranes(lbfs_solver *s, const lbfs_mesh_desc *m, const lbfs_rbc_desc
     }
     ma.total_nodes = N;
     ma.total_springs = S;
+    const bool copies = sorted_copies(N, maxn);
     MembraneConst *d_mc; MembraneScalars *d_ms; int *d_tri, *d_spr, *d_inc, *d_incs, *d_smem, *d_nmem;
     InstanceGrid *d_inst; int *d_cinst = nullptr;
     if ((rc = s->upload(&d_inst, s->inst)) || (rc = s->upload(&d_nmem, node_mem)) ||
@@ -1053,12 +1066,13 @@ int setup_membranes(lbfs_solver *s, const lbfs_mesh_desc *m, const lbfs_rbc_desc
         (rc = s->alloc(&ma.bin_cursor, (size_t)total_patch + n_rbc)) ||
         (rc = s->alloc(&ma.cell_start, (size_t)n_rbc + 1)) || (rc = s->alloc(&ma.sort_ticket, 1)) ||
         (rc = s->upload(&ma.sorted_node, identity)) ||
-        (rc = s->alloc(&ma.sorted_base, N)) || (rc = s->alloc(&ma.sorted_w, 12 * (size_t)N)) ||
+        (copies && ((rc = s->alloc(&ma.sorted_base, N)) || (rc = s->alloc(&s->sorted_w, 12 * (size_t)N)))) ||
         (rc = s->alloc(&ma.node_base, 3 * (size_t)N)) ||
         (rc = s->alloc(&ma.node_w, 12 * (size_t)N)) ||
         (rc = s->alloc(&ma.mad_partials, (size_t)n_rbc * kMaxSpringBlocks)) ||
         (rc = s->alloc(&ma.mad_ticket, (size_t)n_rbc)))
         return rc;
+    ma.sorted_w = s->sorted_w;
     LBFS_CUDA(cudaMemset(ma.mad_ticket, 0, sizeof(unsigned int) * n_rbc));
     LBFS_CUDA(cudaMemset(ma.sort_ticket, 0, sizeof(unsigned int)));
     LBFS_CUDA(cudaMemset(ma.cell_start, 0, sizeof(int) * (n_rbc + 1)));
@@ -2266,6 +2280,7 @@ template <typename R> void shape_to_args(lbfs_solver *s, const lbfs_launch_shape
     a.tb_update = sh.update_threads; a.update_blocks = sh.update_blocks;
     s->ma.spread_blocks = sh.spread_blocks;
     s->ma.force_cluster = sh.membrane_cluster;
+    s->ma.sorted_w = sh.membrane_cluster ? nullptr : s->sorted_w;
     s->membrane_after_k1 = sh.membrane_after_k1 != 0;
     set_chunks(s, sh.flux_chunks);
 }
@@ -2425,11 +2440,14 @@ int adjm_prepare(lbfs_solver *s) {
     std::vector<int> identity(N);
     for (int n = 0; n < N; n++) identity[n] = n;
     MembraneScalars *ms2;
+    mb.sorted_base = nullptr;
+    mb.sorted_w = nullptr;
+    const bool copies = sorted_copies(N, ma.max_nodes);
     if ((rc = s->alloc(&ms2, M)) ||
         (rc = s->alloc(&mb.bin_start, (size_t)s->total_patch + M)) || (rc = s->alloc(&mb.cell_start, (size_t)M + 1)) ||
         (rc = s->alloc(&mb.bin_cursor, (size_t)s->total_patch + M)) ||
         (rc = s->alloc(&mb.sort_ticket, 1)) || (rc = s->upload(&mb.sorted_node, identity)) ||
-        (rc = s->alloc(&mb.sorted_base, N)) || (rc = s->alloc(&mb.sorted_w, 12 * (size_t)N)) ||
+        (copies && ((rc = s->alloc(&mb.sorted_base, N)) || (rc = s->alloc(&mb.sorted_w, 12 * (size_t)N)))) ||
         (rc = s->alloc(&mb.fx, N)) || (rc = s->alloc(&mb.fy, N)) || (rc = s->alloc(&mb.fz, N)) ||
         (rc = s->alloc(&mb.patch_force, 3 * (size_t)s->total_patch)) ||
         (rc = s->alloc(&mb.node_base, 3 * (size_t)N)) || (rc = s->alloc(&mb.node_w, 12 * (size_t)N)))

@@ -209,3 +209,36 @@ def test_batched_fp32_bulk_within_bound_of_fp64():
     assert a.status() == 0 and b.status() == 0
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("stencil", ["PESKIN4", "HAT2"])
+def test_spread_form_does_not_change_bits(stencil):
+    """A handle of several large membranes spreads from copies of the stencil weights in sorted order, a
+    handle of one gathers them node by node (and one of a small membrane copies): the same sums.  Six
+    instances with a red cell each, one of them small, against handles of their own."""
+    from dataclasses import replace
+
+    from lbfs_b200 import GpuSolver, _abi, cases
+    from lbfs_b200.ensemble import concatenate
+    members = [cases.shear_channel(20, 1, 4 if k else 2, 1.5 + 0.5 * k, seed=k,
+                                   ibm_stencil=getattr(_abi, "LBFS_IBM_" + stencil)) for k in range(6)]
+    mesh = concatenate([m.mesh for m in members])
+    cells = [replace(m.membranes[0], instance=k) for k, m in enumerate(members)]
+
+    def run(mesh, membranes, state):
+        with GpuSolver(mesh, members[0].params, membranes) as s:
+            s.set_state(*state)
+            s.step(6, graph=True)
+            assert s.status() == 0
+            return s.state(), s.nodes(), s.nodes(_abi.LBFS_NODES_FORCE)
+
+    state, nodes, force = run(mesh, cells, [np.concatenate(q) for q in zip(*((m.rho, m.u, m.v, m.w) for m in members))])
+    first = 0
+    for k, m in enumerate(members):
+        own = run(m.mesh, m.membranes, (m.rho, m.u, m.v, m.w))
+        for a, b in zip(state, own[0]):
+            assert np.array_equal(mesh.split(a)[k], b), k
+        n = len(own[1])
+        assert np.array_equal(nodes[first:first + n], own[1]) and np.array_equal(force[first:first + n], own[2]), k
+        first += n
