@@ -319,7 +319,8 @@ typedef struct lbfs_launch_shape {
     int32_t membrane_after_k1;      /* 1: in a captured step the membrane kernels start once every block
                                        of the gradient kernel has begun (a programmatic edge from its
                                        launch-completion port) instead of beside it from the step's
-                                       start; 0: from the step's start.  Order only: results unchanged */
+                                       start; 0: from the step's start.  Order only: results unchanged.
+                                       Without effect where gradients and fluxes are one kernel */
     double time_us[5];              /* autotune: [0] mean step time of the chosen shape (us) */
 } lbfs_launch_shape;
 int lbfs_get_launch_shape(lbfs_solver *s, lbfs_launch_shape *shape);

@@ -1399,9 +1399,11 @@ int fork_behind_launch(lbfs_solver *s) {
 }
 
 // A step through the fused fluid pass: the membrane chain, spread included, on
-// its own stream beside the pass (or behind its launch completion, launch shape
-// membrane_after_k1), then the update.  An interior-viscosity update goes
-// between the two, in sequence.
+// its own stream beside the pass, then the update.  An interior-viscosity update
+// goes between the two, in sequence.  The launch shape's membrane_after_k1 has no
+// gradient kernel to follow here: behind the pass, whose blocks hold every
+// register of an SM until they end, the chain came late (us per step, behind /
+// beside: 44.6 / 36.5 on 48^3 with 162 nodes, 64.8 / 55.5 at 64^3 with 642).
 template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
     const GridArgs<R> &ga = grid<R>(s);
     FluidArgs<R> a = fluid<R>(s);
@@ -1427,27 +1429,16 @@ template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, i
         n += 2;
         pass();
     } else {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        LBFS_CUDA(cudaStreamIsCapturing(s->stream, &cap));
         cudaGraphNode_t advect = nullptr;
-        const bool behind = s->membrane_after_k1 && cap == cudaStreamCaptureStatusActive && !s->kernel_events;
-        if (behind) {
-            pass();
-            int rc = fork_behind_launch(s);
-            if (rc) return rc;
-        } else {
-            LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
-            LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
-        }
+        LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
+        LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
         {
             PhaseMark m(s, 0, s->stream2);
             n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted, false, &advect);
         }
         LBFS_CUDA(cudaEventRecord(s->ev_join, s->stream2));
-        if (!behind) {
-            if (int rc = order_behind_advect(s, advect)) return rc;
-            pass();
-        }
+        if (int rc = order_behind_advect(s, advect)) return rc;
+        pass();
         LBFS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_join, 0));
     }
     { PhaseMark m(s, 3, s->stream); launch_fluid_update<R>(a, s->stream, !s->kernel_events); }
