@@ -587,7 +587,8 @@ __device__ __forceinline__ Vec4<R> general_flux(const FluidArgs<R> &a, const Gen
 // The same flux for an interior face whose normal lies within its axis' cone, n_A -
 // |n_B| - |n_C| > 0.001 dt: every direction with e_A = +1 then comes from the owner
 // and every one with e_A = -1 from the neighbour, so the two sides take the closed
-// form of the axis-aligned faces and only the pairs +-e_B, +-e_C choose by n's signs.
+// form of the axis-aligned faces and only the pairs +-e_B, +-e_C choose by n's signs
+// (us per step without / with: 128.6 / 118.4 jittered at 72^3 FP64, 367 / 346 at 128^3 FP32).
 template <typename R, int A>
 __device__ __forceinline__ Vec4<R> cone_flux(const FluidArgs<R> &args, const GenFace<R> &geo, const Vec4<R> &s1,
                                              const Vec4<R> &s2, const R (&g1)[12], const R (&g2)[12], R vf) {
@@ -685,10 +686,8 @@ __device__ __forceinline__ Vec4<R> cone_flux(const FluidArgs<R> &args, const Gen
     return interface_flux<R>(M, rho0, tau, args.gamma_inv, geo.area, -1, nv[0], nv[1], nv[2]);
 }
 
-// CONE: interior faces that a warp takes axis by axis; where all of a warp's faces lie
-// within the cone of one axis they take cone_flux (us per step without / with: 128.6 /
-// 118.4 jittered at 72^3 FP64, 367 / 346 at 128^3 FP32).
-template <typename R, bool CONE>
+// CONE: the axis whose cone the (interior) face's normal lies in, -1: none is known.
+template <typename R, int CONE>
 __device__ __forceinline__ Vec4<R> general_face_flux(const FluidArgs<R> &a, int f, bool is_bc) {
     const int2 oc = __ldg(a.face_cells + f);
     const GenFace<R> geo = a.gen_face[a.axis_aligned ? f - a.ni : f];
@@ -709,14 +708,7 @@ __device__ __forceinline__ Vec4<R> general_face_flux(const FluidArgs<R> &a, int 
     } else {
         s2 = a.state[oc.y];
         load_grad(a.grad + (size_t)12 * oc.y, g2);
-        if constexpr (CONE) {
-            const unsigned lanes = __activemask();
-            const R vf = a.visc_factor[oc.x], thr = R(0.001) * geo.dt;
-            const R ax = fabs(geo.nx), ay = fabs(geo.ny), az = fabs(geo.nz);
-            if (__all_sync(lanes, geo.nx - ay - az > thr)) return cone_flux<R, 0>(a, geo, s1, s2, g1, g2, vf);
-            if (__all_sync(lanes, geo.ny - ax - az > thr)) return cone_flux<R, 1>(a, geo, s1, s2, g1, g2, vf);
-            if (__all_sync(lanes, geo.nz - ax - ay > thr)) return cone_flux<R, 2>(a, geo, s1, s2, g1, g2, vf);
-        }
+        if constexpr (CONE >= 0) return cone_flux<R, CONE>(a, geo, s1, s2, g1, g2, a.visc_factor[oc.x]);
     }
     return general_flux<R>(a, geo, s1, s2, g1, g2, oc.y - a.nc, is_bc ? R(1) : a.visc_factor[oc.x]);
 }

@@ -70,19 +70,28 @@ __global__ void __launch_bounds__(TB, (sizeof(R) == 4 ? 1024 : 640) / TB) k_face
 // takes the faces owned by the TB cells of tile tile0 + b, in up to three
 // face ranges ordered by owner (the generator's x, y, z faces; an imported
 // mesh's internal faces, which OpenFOAM orders by owner, form one range).
-// FP64 at 128 registers (16 warps per SM), FP32 at 64 (32 warps per SM).  CONE: three ranges, so that a
-// warp's faces are of one axis (general_face_flux); an imported mesh's one range mixes them and would
-// only pay for the votes (44.4 / 44.9 us a step on 64,000 cells; its faces taken axis by axis through
-// an index list: 48.5).
+// FP64 at 128 registers (16 warps per SM), FP32 at 64 (32 warps per SM).  CONE: the
+// faces of the three ranges lie within the cones of x, y and z (FluidArgs::cone), a
+// property of the whole mesh: which form a face takes depends on no other face of its
+// warp, so results do not depend on the block size.  An imported mesh's one range
+// mixes the axes (its faces taken axis by axis through an index list: 48.5 us a step on
+// 64,000 cells, 44.4 without).
 template <typename R, int TB, bool CONE>
 __global__ void __launch_bounds__(TB, (sizeof(R) == 4 ? 1024 : 512) / TB) k_face_flux_general_tiles(FluidArgs<R> a, int tile0) {
     pdl_trigger();
     pdl_wait();  // the gradients
     const int *tp = a.flux_tiles + 3 * (tile0 + (int)blockIdx.x);
+    if constexpr (CONE) {
+        const int t = (int)threadIdx.x;
+        for (int f = __ldg(tp) + t, f1 = __ldg(tp + 3); f < f1; f += TB) a.flux[f] = general_face_flux<R, 0>(a, f, false);
+        for (int f = __ldg(tp + 1) + t, f1 = __ldg(tp + 4); f < f1; f += TB) a.flux[f] = general_face_flux<R, 1>(a, f, false);
+        for (int f = __ldg(tp + 2) + t, f1 = __ldg(tp + 5); f < f1; f += TB) a.flux[f] = general_face_flux<R, 2>(a, f, false);
+    } else {
 #pragma unroll 1
-    for (int r = 0; r < 3; r++) {
-        const int f0 = __ldg(tp + r), f1 = __ldg(tp + 3 + r);
-        for (int f = f0 + (int)threadIdx.x; f < f1; f += TB) a.flux[f] = general_face_flux<R, CONE>(a, f, false);
+        for (int r = 0; r < 3; r++) {
+            const int f0 = __ldg(tp + r), f1 = __ldg(tp + 3 + r);
+            for (int f = f0 + (int)threadIdx.x; f < f1; f += TB) a.flux[f] = general_face_flux<R, -1>(a, f, false);
+        }
     }
 }
 
@@ -93,7 +102,7 @@ template <typename R, int TB>
 __global__ void __launch_bounds__(TB) k_face_flux_general(FluidArgs<R> a, int first) {
     const int f = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= a.nf) return;
-    a.flux[f] = general_face_flux<R, false>(a, f, f >= a.ni);
+    a.flux[f] = general_face_flux<R, -1>(a, f, f >= a.ni);
 }
 
 // ----------------------------------------------------------------- CFL ----
@@ -464,10 +473,8 @@ void launch_fluid_flux_tiles(const FluidArgs<R> &a, int tile0, int tile1, cudaSt
     const int g = tile1 - tile0;
     if (g <= 0) return;
     if (!a.axis_aligned) {
-        if (a.nfx >= 0 && a.nfy >= 0 && a.nfz >= 0 && (long long)a.nfx + a.nfy + a.nfz == a.ni)
-            launch_general_tiles<R, true>(a, g, tile0, s, pdl);
-        else
-            launch_general_tiles<R, false>(a, g, tile0, s, pdl);
+        if (a.cone) launch_general_tiles<R, true>(a, g, tile0, s, pdl);
+        else launch_general_tiles<R, false>(a, g, tile0, s, pdl);
         return;
     }
     if (a.tb_flux == 64) launch_maybe_pdl(k_face_flux_tiles<R, 64>, g, 64, s, pdl, a, tile0);

@@ -189,6 +189,7 @@ struct UntilArgs {
 
 template <typename R> struct FluidArgs {
     int nc, nf, ni, nb, nfx, nfy, nfz, axis_aligned;
+    int cone;  // general faces in three ranges, every normal within its axis' cone, n_A - |n_B| - |n_C| > 0.001 dt
     int testcase;
     R rho0;          // density offset of the stored state (0 in FP64)
     R gamma_inv, visc;

@@ -351,6 +351,14 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
         g.bc_branch = (R)((f >= ni && !first_ghost[f - ni]) ? 1 : 0);
         gen[f - gf0] = g;
     }
+    // the generator's jittered meshes: every interior face within the cone of its range's axis
+    a.cone = !a.axis_aligned && ni > 0 && a.nfx >= 0 && a.nfy >= 0 && a.nfz >= 0 && (long long)a.nfx + a.nfy + a.nfz == ni;
+    for (int f = 0; f < ni && a.cone; f++) {
+        const GenFace<R> &g = gen[f];
+        const R n[3] = {g.nx, g.ny, g.nz};
+        const int A = (f < a.nfx) ? 0 : ((f < a.nfx + a.nfy) ? 1 : 2), B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
+        a.cone = n[A] - std::fabs(n[B]) - std::fabs(n[C]) > R(0.001) * g.dt;
+    }
     // K3: signed face list per cell, faces in increasing index order
     std::vector<int> cf(6 * (size_t)nc, 0), cnt(nc, 0);
     for (int f = 0; f < nf; f++) {

@@ -104,6 +104,42 @@ def test_faces_within_an_axis_cone_match_oracle(jitter, size):
         assert rel_err(a, b) <= FP64_RTOL
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+def test_general_flux_form_does_not_depend_on_the_block_size(precision):
+    """A mesh with some interior faces outside their axis' cone: the flux of a face must not depend on
+    which faces share its warp, so states agree bit for bit over block sizes 64, 128 and 256 (tiles of
+    that many cells), and with the oracle to the parity bound."""
+    from lbfs_b200 import GpuSolver, cases
+    from oracle_lbfs import OracleSolver
+    size = (21, 9, 7)
+    c = cases.poiseuille(n=size[0], ny=size[1], nz=size[2], precision=precision)
+    m = _mesh(0.1, n=size)
+    m.set_boundaries(c.bcs)
+    rng = np.random.default_rng(8)
+    tilted = rng.random(m.n_interior) < 0.2
+    n = m.face_normal.reshape(-1, 3)
+    n[:m.n_interior][tilted] += rng.uniform(-0.8, 0.8, (int(tilted.sum()), 3))
+    n /= np.linalg.norm(n, axis=1)[:, None]
+    state = [c.rho] + [0.01 * rng.uniform(-1, 1, m.n_cells) for _ in range(3)]
+    got = []
+    for threads in (64, 128, 256):
+        with GpuSolver(m, c.params) as s:
+            s.set_launch_shape(general_flux_threads=threads)
+            s.set_state(*state)
+            s.step(5, graph=True)
+            got.append(s.state())
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert np.array_equal(a, b)
+    if precision == 0:
+        o = OracleSolver(m, c.params, [])
+        o.set_state(*state)
+        o.step(5)
+        for a, b in zip(got[0], o.state()):
+            assert rel_err(a, b) <= FP64_RTOL
+
+
 def test_jittered_box_at_rest_stays_at_rest():
     """With the faces' vector areas closing around every cell, a fluid at rest
     in a closed jittered box feels no net pressure force (oracle, CPU)."""
