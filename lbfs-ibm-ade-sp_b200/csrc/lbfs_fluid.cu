@@ -535,8 +535,10 @@ template <typename R, bool GRID> void launch_update(const FluidArgs<R> &a, cudaS
     else launch_maybe_pdl(k_cell_update<R, 256, GRID>, g, 256, s, pdl, a);
 }
 template <typename R> void launch_fluid_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
-    if (a.grid_res) launch_update<R, true>(a, s, pdl);
-    else launch_update<R, false>(a, s, pdl);
+    if constexpr (sizeof(R) == 8) {
+        if (a.grid_res) return launch_update<R, true>(a, s, pdl);
+    }
+    launch_update<R, false>(a, s, pdl);
 }
 
 template <typename R> void launch_fluid_cfl(const FluidArgs<R> &a, cudaStream_t s) {

@@ -26,19 +26,19 @@
 namespace lbfs {
 namespace {
 
-template <typename R> __device__ __forceinline__ R relaxation(const FluidArgs<R> &a, R vf, R dt) {
-    return (a.testcase == 8) ? R(0) : (a.visc * vf * R(3) / dt * a.gamma_inv);
+__device__ __forceinline__ double relaxation(const FluidArgs<double> &a, double vf, double dt) {
+    return (a.testcase == 8) ? 0.0 : (a.vi3.0 * vf * 3.0 / dt * a.gamma_inv);
 }
 
 // The ghost of a cell (state s: rho, u, v, w) across a side with record gs, in place of s.
-template <typename R> __device__ __forceinline__ void side_ghost(const FluidArgs<R> &a, const GridSide<R> &gs, R (&s)[4]) {
-    const R v[4] = {gs.val.rho, gs.val.u, gs.val.v, gs.val.w};
+__device__ __forceinline__ void side_ghost(const FluidArgs<double> &a, const GridSide &gs, double (&s)[4]) {
+    const double v[4] = {gs.val.rho, gs.val.u, gs.val.v, gs.val.w};
 #pragma unroll
     for (int m = 0; m < 4; m++)
         if (gs.flags & (m == 0 ? 1 : 2)) s[m] = v[m] - (s[m] - v[m]);
     if (gs.flags & 12) {
-        const Vec4<R> q = a.state[gs.partner];
-        const R qv[4] = {q.rho, q.u, q.v, q.w};
+        const Vec4<double> q = a.state[gs.partner];
+        const double qv[4] = {q.rho, q.u, q.v, q.w};
 #pragma unroll
         for (int m = 0; m < 4; m++)
             if (gs.flags & (m == 0 ? 4 : 8)) s[m] = qv[m];
@@ -48,7 +48,7 @@ template <typename R> __device__ __forceinline__ void side_ghost(const FluidArgs
 // Boundary blocks among the first `block` blocks of the launch: spread evenly, so
 // that each runs beside a tile's block (all of them first were one latency-bound
 // wave before the tiles: 40 us of 275 at 128^3).
-template <typename R> __device__ __forceinline__ int bnd_before(const GridArgs<R> &ga, unsigned block) {
+__device__ __forceinline__ int bnd_before(const GridArgs &ga, unsigned block) {
     return (int)((unsigned long long)block * (unsigned)ga.bnd_blocks / (unsigned)(ga.bnd_blocks + ga.n_tiles));
 }
 
@@ -73,54 +73,41 @@ template <typename R> __device__ __forceinline__ int bnd_before(const GridArgs<R
 // SM) took 362 us: their loads were waited for.
 constexpr int kSlots = 4;
 
-template <typename R> struct Half;  // 16-byte pieces of a state record
-template <> struct Half<double> { using type = double2; static constexpr int n = 2; };
-template <> struct Half<float> { using type = float4; static constexpr int n = 1; };
-
 __device__ __forceinline__ void copy16(void *smem, const void *g) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(g) : "memory");
 }
-template <int BYTES> __device__ __forceinline__ void copy_small(void *smem, const void *g) {
+__device__ __forceinline__ void copy8(void *smem, const void *g) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(a), "l"(g), "n"(BYTES) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(g) : "memory");
 }
 
-template <typename R> struct State4 {
-    R s[4];  // rho, u, v, w
+struct State4 {
+    double s[4];  // rho, u, v, w
 };
 
-// The staged planes: the halves of slot t's states at h[(Half::n t + half) Q + position].
-template <typename R> struct Planes {
-    typename Half<R>::type *h;
+// The staged planes: the halves of slot t's states at h[(2 t + half) Q + position].
+struct Planes {
+    double2 *h;
     int Q;
-    __device__ __forceinline__ void get(int at, R (&s)[4]) const {  // at = Half::n slot Q + position; rho, u, v, w
-        if constexpr (sizeof(R) == 8) {
-            const double2 p = h[at], q = h[at + Q];
-            s[1] = p.x; s[2] = p.y; s[3] = q.x; s[0] = q.y;
-        } else {
-            const float4 p = h[at];
-            s[1] = p.x; s[2] = p.y; s[3] = p.z; s[0] = p.w;
-        }
+    __device__ __forceinline__ void get(int at, double (&s)[4]) const {  // at = 2 slot Q + position; rho, u, v, w
+        const double2 p = h[at], q = h[at + Q];
+        s[1] = p.x; s[2] = p.y; s[3] = q.x; s[0] = q.y;
     }
-    __device__ __forceinline__ State4<R> at(int i) const {
-        State4<R> q;
+    __device__ __forceinline__ State4 at(int i) const {
+        State4 q;
         get(i, q.s);
         return q;
     }
-    __device__ __forceinline__ void put(int at, const R (&s)[4]) const {
-        if constexpr (sizeof(R) == 8) {
-            h[at] = make_double2(s[1], s[2]);
-            h[at + Q] = make_double2(s[3], s[0]);
-        } else {
-            h[at] = make_float4(s[1], s[2], s[3], s[0]);
-        }
+    __device__ __forceinline__ void put(int at, const double (&s)[4]) const {
+        h[at] = make_double2(s[1], s[2]);
+        h[at + Q] = make_double2(s[3], s[0]);
     }
 };
 
 // A cell's state and its neighbours' differences along each axis (upper - lower).
-template <typename R> struct CellSlopes {
-    R s[4], d[3][4];
+struct CellSlopes {
+    double s[4], d[3][4];
 };
 
 // Lattice moments of one side of a face.  Its nodes in the directions e = (s e_A,
@@ -136,118 +123,81 @@ template <typename R> struct CellSlopes {
 // The slopes' weight w (dt x gradient weight, its multiples in GridWeights) is
 // applied to sums and not to the twelve differences.  rho, a: the cell's density
 // and v; db, dc: its neighbours' differences along B and C (velocities not scaled).
-// FP32 (rho the deviation from rho0): in the velocities themselves, from the small
-// terms X = 3 e.u + 4.5 (e.u)^2 - 1.5 |u|^2 alone; the term 3 rho0 e.p of the face
-// centre's velocity is left out as in pop_dev and added once by the caller, the
-// rest of the linear term coming from ad = a - p.
-template <typename R> struct SideSums {
-    R S, YB, YC, ga0;
+struct SideSums {
+    double S, YB, YC, ga0;
 };
-template <typename R, int A, int SGN>
-__device__ __forceinline__ SideSums<R> uniform_side(R rho, const R (&a)[3], const R (&db)[4], const R (&dc)[4],
-                                                    const GridWeights<R> &g, const R (&ad)[3], R rho0) {
+template <int A, int SGN>
+__device__ __forceinline__ SideSums uniform_side(double rho, const double (&a)[3], const double (&db)[4],
+                                                 const double (&dc)[4], const GridWeights &g) {
     constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    constexpr R s = R(SGN);
-    const R lin = sizeof(R) == 8 ? g.w3 : g.w;
-    const R be = SGN > 0 ? a[B] - lin * db[1 + A] : a[B] + lin * db[1 + A];
-    const R ga = SGN > 0 ? a[C] - lin * dc[1 + A] : a[C] + lin * dc[1 + A];
-    const R de = -lin * (db[1 + C] + dc[1 + B]);
-    const R sl = db[1 + B] + dc[1 + C];
-    const R aa = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-    const R nn = (db[1] * db[1] + db[2] * db[2] + db[3] * db[3]) + (dc[1] * dc[1] + dc[2] * dc[2] + dc[3] * dc[3]);
-    const R ab = a[0] * db[1] + a[1] * db[2] + a[2] * db[3];
-    const R ac = a[0] * dc[1] + a[1] * dc[2] + a[2] * dc[3];
-    const R bc = db[1] * dc[1] + db[2] * dc[2] + db[3] * dc[3];
-    const R b0 = g.w * db[0], c0 = g.w * dc[0];
-    SideSums<R> r;
-    if constexpr (sizeof(R) == 8) {
-        const R ea = R(1) + s * a[A];
-        const R al = ea - g.w3 * sl;
-        const R Ka = R(1) - R(1.0 / 3.0) * aa;
-        const R q0 = R(0.5) * ((Ka + al * al + be * be) + (ga * ga + de * de - g.ww3 * nn));
-        const R XB = g.w * ab + (al * be + ga * de), XC = g.w * ac + (al * ga + be * de);
-        const R XBC = (al * de + be * ga) - g.ww3 * bc;
-        r.S = rho * q0 - b0 * XB - c0 * XC;
-        r.YB = rho * XB - b0 * q0 - c0 * XBC;
-        r.YC = rho * XC - c0 * q0 - b0 * XBC;
-        r.ga0 = rho * (Ka + ea * ea);
-    } else {
-        const R al = s * a[A] - g.w * sl;
-        const R E0 = R(4.5) * (al * al + be * be + ga * ga + de * de) - (R(1.5) * aa + (R(0.5) * g.ww3) * nn);
-        const R EB = R(9) * (al * be + ga * de) + g.w3 * ab, EC = R(9) * (al * ga + be * de) + g.w3 * ac;
-        const R XBC = R(3) * de + (R(9) * (al * de + be * ga) - g.ww3 * bc);
-        const R X0 = R(3) * al + E0, XB = R(3) * be + EB, XC = R(3) * ga + EC;
-        // without the face centre's e.p: from a - p
-        const R X0d = R(3) * (s * ad[A] - g.w * sl) + E0;
-        const R XBd = R(3) * (SGN > 0 ? ad[B] - g.w * db[1 + A] : ad[B] + g.w * db[1 + A]) + EB;
-        const R XCd = R(3) * (SGN > 0 ? ad[C] - g.w * dc[1 + A] : ad[C] + g.w * dc[1 + A]) + EC;
-        r.S = rho + (rho * X0 - b0 * XB - c0 * XC + rho0 * X0d);
-        r.YB = (rho * XB - b0 * X0 - c0 * XBC + rho0 * XBd) - b0;
-        r.YC = (rho * XC - c0 * X0 - b0 * XBC + rho0 * XCd) - c0;
-        const R Ea = R(4.5) * (a[A] * a[A]) - R(1.5) * aa;
-        r.ga0 = R(2) * (rho + (rho * (R(3) * (s * a[A]) + Ea) + rho0 * (R(3) * (s * ad[A]) + Ea)));
-    }
+    constexpr double s = SGN;
+    const double be = SGN > 0 ? a[B] - g.w3 * db[1 + A] : a[B] + g.w3 * db[1 + A];
+    const double ga = SGN > 0 ? a[C] - g.w3 * dc[1 + A] : a[C] + g.w3 * dc[1 + A];
+    const double de = -g.w3 * (db[1 + C] + dc[1 + B]);
+    const double sl = db[1 + B] + dc[1 + C];
+    const double aa = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+    const double nn = (db[1] * db[1] + db[2] * db[2] + db[3] * db[3]) + (dc[1] * dc[1] + dc[2] * dc[2] + dc[3] * dc[3]);
+    const double ab = a[0] * db[1] + a[1] * db[2] + a[2] * db[3];
+    const double ac = a[0] * dc[1] + a[1] * dc[2] + a[2] * dc[3];
+    const double bc = db[1] * dc[1] + db[2] * dc[2] + db[3] * dc[3];
+    const double b0 = g.w * db[0], c0 = g.w * dc[0];
+    SideSums r;
+    const double ea = 1.0 + s * a[A];
+    const double al = ea - g.w3 * sl;
+    const double Ka = 1.0 - (1.0 / 3.0) * aa;
+    const double q0 = 0.5 * ((Ka + al * al + be * be) + (ga * ga + de * de - g.ww3 * nn));
+    const double XB = g.w * ab + (al * be + ga * de), XC = g.w * ac + (al * ga + be * de);
+    const double XBC = (al * de + be * ga) - g.ww3 * bc;
+    r.S = rho * q0 - b0 * XB - c0 * XC;
+    r.YB = rho * XB - b0 * q0 - c0 * XBC;
+    r.YC = rho * XC - c0 * q0 - b0 * XBC;
+    r.ga0 = rho * (Ka + ea * ea);
     return r;
 }
 
 // Half the sum and half the difference of the populations (over their weight) of
 // the opposite directions +-e_X at the face centre, in the same variables: rho, p
-// its density and v (FP32: u), K = 1 - |v|^2 / 3 (FP32: -1.5 |u|^2); ds the sum of both cells'
-// differences along X, w / 2 times which is the displacement (L = p -+ b).
-template <typename R, int X>
-__device__ __forceinline__ void uniform_pair(R rho, const R (&p)[3], R K, const R (&ds)[4], const GridWeights<R> &g,
-                                             R rho0, R &sum, R &dif) {
-    const R bb = ds[1] * ds[1] + ds[2] * ds[2] + ds[3] * ds[3];
-    const R pb = p[0] * ds[1] + p[1] * ds[2] + p[2] * ds[3];
-    const R b0 = g.h * ds[0], px = p[X];
-    if constexpr (sizeof(R) == 8) {
-        const R c = R(1) - g.h3 * ds[1 + X];
-        const R q0 = R(0.5) * ((K + c * c) + (px * px - g.hh3 * bb));
-        const R odd = g.h * pb + c * px;
-        sum = rho * q0 - b0 * odd;
-        dif = rho * odd - b0 * q0;
-    } else {
-        const R bx = g.h * ds[1 + X];
-        const R even = (K + R(4.5) * (px * px + bx * bx) - (R(0.5) * g.hh3) * bb) - R(3) * bx;
-        const R odd2 = g.h3 * pb - R(9) * (bx * px);
-        const R odd = odd2 + R(3) * px;
-        sum = rho + (rho * even - b0 * odd + rho0 * even);
-        dif = (rho * odd - b0 * even + rho0 * odd2) - b0;
-    }
+// its density and v, K = 1 - |v|^2 / 3; ds the sum of both cells' differences along
+// X, w / 2 times which is the displacement (L = p -+ b).
+template <int X>
+__device__ __forceinline__ void uniform_pair(double rho, const double (&p)[3], double K, const double (&ds)[4],
+                                             const GridWeights &g, double &sum, double &dif) {
+    const double bb = ds[1] * ds[1] + ds[2] * ds[2] + ds[3] * ds[3];
+    const double pb = p[0] * ds[1] + p[1] * ds[2] + p[2] * ds[3];
+    const double b0 = g.h * ds[0], px = p[X];
+    const double c = 1.0 - g.h3 * ds[1 + X];
+    const double q0 = 0.5 * ((K + c * c) + (px * px - g.hh3 * bb));
+    const double odd = g.h * pb + c * px;
+    sum = rho * q0 - b0 * odd;
+    dif = rho * odd - b0 * q0;
 }
 
 // Flux per unit area (rho, u, v, w) through an axis-A face: its density p0 and v at
 // the centre, the sums of both cells' differences along B and C and the sides' sums.
-template <typename R, int A>
-__device__ __forceinline__ Vec4<R> face_flux(const FluidArgs<R> &args, const GridWeights<R> &g, R p0, const R (&p)[3],
-                                             const R (&bs)[4], const R (&cs)[4], const SideSums<R> &o,
-                                             const SideSums<R> &n, R tau) {
+template <int A>
+__device__ __forceinline__ Vec4<double> face_flux(const GridWeights &g, double p0, const double (&p)[3],
+                                                  const double (&bs)[4], const double (&cs)[4], const SideSums &o,
+                                                  const SideSums &n, double tau) {
     constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    const R rho0 = rho0_of(args);
     // the rest and tangential directions from the face centre
-    const R pp = (sizeof(R) == 8 ? R(-1.0 / 3.0) : R(-1.5)) * (p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
-    const R K = sizeof(R) == 8 ? R(1) + pp : pp;
-    R sB, dB, sC, dC;
-    uniform_pair<R, B>(p0, p, K, bs, g, rho0, sB, dB);
-    uniform_pair<R, C>(p0, p, K, cs, g, rho0, sC, dC);
-    const R gz0 = sizeof(R) == 8 ? p0 * (R(1) + R(0.5) * pp) : p0 + (p0 + rho0) * pp;
-    constexpr R w0 = R(2.0 / 9.0), wh = R(1.0 / 18.0);
+    const double pp = (-1.0 / 3.0) * (p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+    const double K = 1.0 + pp;
+    double sB, dB, sC, dC;
+    uniform_pair<B>(p0, p, K, bs, g, sB, dB);
+    uniform_pair<C>(p0, p, K, cs, g, sC, dC);
+    const double gz0 = p0 * (1.0 + 0.5 * pp);
+    constexpr double w0 = 2.0 / 9.0, wh = 1.0 / 18.0;
     // moments, relaxation and the axis-A flux (interface_flux): with u = m_A / rho the relaxed second
     // moments are (1 - tau) (u m_q + d_Aq rho / 3) + tau F_q
-    const R So = wh * (o.ga0 + o.S), Sn = wh * (n.ga0 + n.S);  // 1/9 of ga0 / 2, four corners of 1/72
-    const R rho = (So + Sn) + w0 * (gz0 + (sB + sC));
-    R mA = So - Sn, mB = wh * (o.YB + n.YB) + w0 * dB, mC = wh * (o.YC + n.YC) + w0 * dC;
-    if constexpr (sizeof(R) == 4) {  // the term 3 rho0 e.p left out of the populations
-        mA = mA + rho0 * p[A];
-        mB = mB + rho0 * p[B];
-        mC = mC + rho0 * p[C];
-    }
-    const R keep = R(1) - tau;
-    const R ku = keep * (mA / (rho + rho0)), th = tau * wh;
-    Vec4<R> r;
+    const double So = wh * (o.ga0 + o.S), Sn = wh * (n.ga0 + n.S);  // 1/9 of ga0 / 2, four corners of 1/72
+    const double rho = (So + Sn) + w0 * (gz0 + (sB + sC));
+    const double mA = So - Sn, mB = wh * (o.YB + n.YB) + w0 * dB, mC = wh * (o.YC + n.YC) + w0 * dC;
+    const double keep = 1.0 - tau;
+    const double ku = keep * (mA / rho), th = tau * wh;
+    Vec4<double> r;
     r.rho = mA;
-    const R fA = ku * mA + (keep * R(1.0 / 3.0)) * rho + tau * (So + Sn);
-    const R fB = ku * mB + th * (o.YB - n.YB), fC = ku * mC + th * (o.YC - n.YC);
+    const double fA = ku * mA + (keep * (1.0 / 3.0)) * rho + tau * (So + Sn);
+    const double fB = ku * mB + th * (o.YB - n.YB), fC = ku * mC + th * (o.YC - n.YC);
     r.u = A == 0 ? fA : fB;
     r.v = A == 1 ? fA : (A == 0 ? fB : fC);
     r.w = A == 2 ? fA : fC;
@@ -257,40 +207,23 @@ __device__ __forceinline__ Vec4<R> face_flux(const FluidArgs<R> &args, const Gri
 // Flux per unit area (rho, u, v, w) through the low axis-A face of the cell hi:
 // the lower cell at lo, its lower neighbour's state lm and its neighbours lbm, lbp
 // along B and lcm, lcp along C.
-template <typename R, int A>
-__device__ __forceinline__ Vec4<R> uniform_flux(const FluidArgs<R> &args, const GridArgs<R> &ga, const Planes<R> &pl,
-                                                const CellSlopes<R> &hi, int lo, const State4<R> &lm, int lbm, int lbp, int lcm,
-                                                int lcp, R tau) {
+template <int A>
+__device__ __forceinline__ Vec4<double> uniform_flux(const GridArgs &ga, const Planes &pl, const CellSlopes &hi, int lo,
+                                                     const State4 &lm, int lbm, int lbp, int lcm, int lcp, double tau) {
     constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    const R rho0 = rho0_of(args);
-    const GridWeights<R> &g = ga.cw;
-    R s1[4], p0, p[3], ad1[3] = {R(0), R(0), R(0)}, ad2[3] = {R(0), R(0), R(0)};
+    const GridWeights &g = ga.cw;
+    double s1[4], p0, p[3];
     pl.get(lo, s1);
     {
-        const R(&q)[4] = lm.s;
-        if constexpr (sizeof(R) == 8) {
-            p0 = R(0.5) * (s1[0] + hi.s[0]) + g.h * ((hi.s[0] - q[0]) - hi.d[A][0]);
+        const double(&q)[4] = lm.s;
+        p0 = 0.5 * (s1[0] + hi.s[0]) + g.h * ((hi.s[0] - q[0]) - hi.d[A][0]);
 #pragma unroll
-            for (int m = 0; m < 3; m++)
-                p[m] = R(1.5) * (s1[1 + m] + hi.s[1 + m]) + g.h3 * ((hi.s[1 + m] - q[1 + m]) - hi.d[A][1 + m]);
-        } else {
-            // p = s1 - (s1 - p): the difference is small and formed from differences, so that p, whose
-            // term in the first moments is the largest, is rounded once (0.5 (s1 + s2) + h twice: 5 %
-            // more error in the cross-stream components)
-            p0 = s1[0] - (R(0.5) * (s1[0] - hi.s[0]) - g.h * ((hi.s[0] - q[0]) - hi.d[A][0]));
-#pragma unroll
-            for (int m = 0; m < 3; m++) {
-                const R h = g.h * ((hi.s[1 + m] - q[1 + m]) - hi.d[A][1 + m]);
-                const R hd = R(0.5) * (s1[1 + m] - hi.s[1 + m]);
-                ad1[m] = hd - h;
-                ad2[m] = -(hd + h);
-                p[m] = s1[1 + m] - ad1[m];
-            }
-        }
+        for (int m = 0; m < 3; m++)
+            p[m] = 1.5 * (s1[1 + m] + hi.s[1 + m]) + g.h3 * ((hi.s[1 + m] - q[1 + m]) - hi.d[A][1 + m]);
     }
-    R b[4], c[4];
+    double b[4], c[4];
     {
-        R q0[4], q1[4];
+        double q0[4], q1[4];
         pl.get(lbm, q0);
         pl.get(lbp, q1);
 #pragma unroll
@@ -300,15 +233,14 @@ __device__ __forceinline__ Vec4<R> uniform_flux(const FluidArgs<R> &args, const 
 #pragma unroll
         for (int m = 0; m < 4; m++) c[m] = q1[m] - q0[m];
     }
-    constexpr R sc = sizeof(R) == 8 ? R(3) : R(1);
-    const R v1[3] = {sc * s1[1], sc * s1[2], sc * s1[3]};
-    const SideSums<R> o = uniform_side<R, A, 1>(s1[0], v1, b, c, g, ad1, rho0);
-    const R v2[3] = {sc * hi.s[1], sc * hi.s[2], sc * hi.s[3]};
-    const SideSums<R> n = uniform_side<R, A, -1>(hi.s[0], v2, hi.d[B], hi.d[C], g, ad2, rho0);
-    R bs[4], cs[4];
+    const double v1[3] = {3.0 * s1[1], 3.0 * s1[2], 3.0 * s1[3]};
+    const SideSums o = uniform_side<A, 1>(s1[0], v1, b, c, g);
+    const double v2[3] = {3.0 * hi.s[1], 3.0 * hi.s[2], 3.0 * hi.s[3]};
+    const SideSums n = uniform_side<A, -1>(hi.s[0], v2, hi.d[B], hi.d[C], g);
+    double bs[4], cs[4];
 #pragma unroll
     for (int m = 0; m < 4; m++) { bs[m] = b[m] + hi.d[B][m]; cs[m] = c[m] + hi.d[C][m]; }
-    return face_flux<R, A>(args, g, p0, p, bs, cs, o, n, tau);
+    return face_flux<A>(g, p0, p, bs, cs, o, n, tau);
 }
 
 // ---- boundary faces ----------------------------------------------------------------
@@ -324,16 +256,15 @@ __device__ __forceinline__ Vec4<R> uniform_flux(const FluidArgs<R> &args, const 
 // faces were 30 us of the pass at 128^3 FP64 and half of it on 48,000 cells.
 
 // Differences (upper - lower) along x, y, z around the cell of boundary face f.
-template <typename R>
-__device__ __forceinline__ void boundary_slopes(const FluidArgs<R> &a, const GridArgs<R> &ga, const GridBnd &f,
-                                                const GridSide<R> &rec, const R (&own)[4], R (&d)[3][4]) {
+__device__ __forceinline__ void boundary_slopes(const FluidArgs<double> &a, const GridArgs &ga, const GridBnd &f,
+                                                const GridSide &rec, const double (&own)[4], double (&d)[3][4]) {
     const unsigned at[3] = {(unsigned)f.info & 7u, (unsigned)(f.info >> 3) & 7u, (unsigned)(f.info >> 6) & 7u};
     const unsigned miss = 1u << at[0] | 1u << at[1] | 1u << at[2];  // bit 7: none
-    const Vec4<R> *st = a.state + f.cell;
+    const Vec4<double> *st = a.state + f.cell;
     const int step[3] = {1, f.sy, f.sz};
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        const Vec4<R> lo = st[(miss >> (2 * q) & 1u) ? 0 : -step[q]], hi = st[(miss >> (2 * q + 1) & 1u) ? 0 : step[q]];
+        const Vec4<double> lo = st[(miss >> (2 * q) & 1u) ? 0 : -step[q]], hi = st[(miss >> (2 * q + 1) & 1u) ? 0 : step[q]];
         d[q][0] = hi.rho - lo.rho;
         d[q][1] = hi.u - lo.u;
         d[q][2] = hi.v - lo.v;
@@ -342,9 +273,9 @@ __device__ __forceinline__ void boundary_slopes(const FluidArgs<R> &a, const Gri
 #pragma unroll
     for (int e = 0; e < 3; e++) {
         if (at[e] > 5u) continue;
-        R gs[4] = {own[0], own[1], own[2], own[3]};
+        double gs[4] = {own[0], own[1], own[2], own[3]};
         side_ghost(a, e == 0 ? rec : ga.bnd_side[f.more[e - 1]], gs);
-        const R sg = (at[e] & 1u) ? R(1) : R(-1);
+        const double sg = (at[e] & 1u) ? 1.0 : -1.0;
 #pragma unroll
         for (int q = 0; q < 3; q++)
 #pragma unroll
@@ -353,94 +284,86 @@ __device__ __forceinline__ void boundary_slopes(const FluidArgs<R> &a, const Gri
     }
 }
 
-template <typename R> __device__ __forceinline__ void grid_boundary(const FluidArgs<R> &a, const GridArgs<R> &ga, int b) {
+__device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const GridArgs &ga, int b) {
     const GridBnd f = ga.bnd[b];
-    const GridSide<R> rec = ga.bnd_side[b];
+    const GridSide rec = ga.bnd_side[b];
     const int side = f.info & 7, axis = side >> 1;
-    R d[3][4], dp[3][4];
-    State4<R> own, ghost;
+    double d[3][4], dp[3][4];
+    State4 own, ghost;
     {
-        const Vec4<R> s = a.state[f.cell];
+        const Vec4<double> s = a.state[f.cell];
         own = {{s.rho, s.u, s.v, s.w}};
     }
     boundary_slopes(a, ga, f, rec, own.s, d);
     ghost = own;
     side_ghost(a, rec, ghost.s);
     if (rec.flags & 12) {  // the partner's slopes
-        const Vec4<R> s = a.state[rec.partner];
-        const R q[4] = {s.rho, s.u, s.v, s.w};
+        const Vec4<double> s = a.state[rec.partner];
+        const double q[4] = {s.rho, s.u, s.v, s.w};
         boundary_slopes(a, ga, ga.bnd[f.partner], ga.bnd_side[f.partner], q, dp);
     } else {
 #pragma unroll
         for (int q = 0; q < 3; q++)
 #pragma unroll
-            for (int m = 0; m < 4; m++) dp[q][m] = R(0);
+            for (int m = 0; m < 4; m++) dp[q][m] = 0.0;
     }
     // into the frame: components (n, t1, t2) = (axis, the other two in order), n outward
-    const R sn = (side & 1) ? R(1) : R(-1);
-    auto turn = [&](R x, R y, R z, R (&o)[3]) {
+    const double sn = (side & 1) ? 1.0 : -1.0;
+    auto turn = [&](double x, double y, double z, double (&o)[3]) {
         o[0] = sn * (axis == 0 ? x : (axis == 1 ? y : z));
         o[1] = axis == 0 ? y : x;
         o[2] = axis == 2 ? y : z;
     };
-    auto turned = [&](const R (&v)[4]) {
-        State4<R> o;
+    auto turned = [&](const double (&v)[4]) {
+        State4 o;
         o.s[0] = v[0];
-        R t[3];
+        double t[3];
         turn(v[1], v[2], v[3], t);
         o.s[1] = t[0]; o.s[2] = t[1]; o.s[3] = t[2];
         return o;
     };
-    R e[3][4], ep[3][4];  // differences along n, t1, t2 with turned components
-    auto turn_slopes = [&](const R (&v)[3][4], R (&o)[3][4]) {
-        const State4<R> x = turned(v[0]), y = turned(v[1]), z = turned(v[2]);
+    double e[3][4], ep[3][4];  // differences along n, t1, t2 with turned components
+    auto turn_slopes = [&](const double (&v)[3][4], double (&o)[3][4]) {
+        const State4 x = turned(v[0]), y = turned(v[1]), z = turned(v[2]);
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-            R t[3];
+            double t[3];
             turn(x.s[m], y.s[m], z.s[m], t);
             o[0][m] = t[0]; o[1][m] = t[1]; o[2][m] = t[2];
         }
     };
     turn_slopes(d, e);
     turn_slopes(dp, ep);
-    const State4<R> S1 = turned(own.s), S2 = turned(ghost.s), V = turned({rec.val.rho, rec.val.u, rec.val.v, rec.val.w});
-    const GridWeights<R> &g = ga.cw;
-    const R rho0 = rho0_of(a);
-    constexpr R sc = sizeof(R) == 8 ? R(3) : R(1);
+    const State4 S1 = turned(own.s), S2 = turned(ghost.s), V = turned({rec.val.rho, rec.val.u, rec.val.v, rec.val.w});
+    const GridWeights &g = ga.cw;
     const bool first = (f.info & 1024) != 0;
-    R p[4], a1[4], a2[4], ad1[3] = {R(0), R(0), R(0)}, ad2[3] = {R(0), R(0), R(0)};
-    R b1[4], c1[4], b2[4], c2[4];
+    double p[4], a1[4], a2[4];
+    double b1[4], c1[4], b2[4], c2[4];
 #pragma unroll
     for (int m = 0; m < 4; m++) {
         const bool dir = (rec.flags & (m == 0 ? 1 : 2)) != 0;
         const bool per = (rec.flags & (m == 0 ? 4 : 8)) != 0;
-        const R Dn = dir ? ga.bnd_k * (S2.s[m] - S1.s[m]) : (per ? ep[0][m] : R(0));  // ghost's differences
-        b2[m] = dir ? R(0) : (per ? ep[1][m] : e[1][m]);
-        c2[m] = dir ? R(0) : (per ? ep[2][m] : e[2][m]);
-        const R wD = g.w * Dn;
+        const double Dn = dir ? ga.bnd_k * (S2.s[m] - S1.s[m]) : (per ? ep[0][m] : 0.0);  // ghost's differences
+        b2[m] = dir ? 0.0 : (per ? ep[1][m] : e[1][m]);
+        c2[m] = dir ? 0.0 : (per ? ep[2][m] : e[2][m]);
+        const double wD = g.w * Dn;
         const bool set = (rec.flags & (m == 0 ? 1 : 16)) != 0;
-        const R h = g.h * (e[0][m] - Dn), hd = R(0.5) * (S1.s[m] - S2.s[m]);
+        const double h = g.h * (e[0][m] - Dn), hd = 0.5 * (S1.s[m] - S2.s[m]);
         p[m] = first ? S1.s[m] - (hd - h) : (set ? V.s[m] : S1.s[m] + wD);
         a1[m] = first ? S1.s[m] : p[m] - wD;
         a2[m] = first ? S2.s[m] : p[m] + wD;
         b1[m] = first ? e[1][m] : b2[m];
         c1[m] = first ? e[2][m] : c2[m];
-        if constexpr (sizeof(R) == 4) {
-            if (m > 0) {
-                ad1[m - 1] = first ? hd - h : -wD;
-                ad2[m - 1] = first ? -(hd + h) : wD;
-            }
-        }
     }
-    const R v1[3] = {sc * a1[1], sc * a1[2], sc * a1[3]}, v2[3] = {sc * a2[1], sc * a2[2], sc * a2[3]};
-    const R pv[3] = {sc * p[1], sc * p[2], sc * p[3]};
-    const SideSums<R> o = uniform_side<R, 0, 1>(a1[0], v1, b1, c1, g, ad1, rho0);
-    const SideSums<R> n = uniform_side<R, 0, -1>(a2[0], v2, b2, c2, g, ad2, rho0);
+    const double v1[3] = {3.0 * a1[1], 3.0 * a1[2], 3.0 * a1[3]}, v2[3] = {3.0 * a2[1], 3.0 * a2[2], 3.0 * a2[3]};
+    const double pv[3] = {3.0 * p[1], 3.0 * p[2], 3.0 * p[3]};
+    const SideSums o = uniform_side<0, 1>(a1[0], v1, b1, c1, g);
+    const SideSums n = uniform_side<0, -1>(a2[0], v2, b2, c2, g);
 #pragma unroll
     for (int m = 0; m < 4; m++) { b1[m] = b1[m] + b2[m]; c1[m] = c1[m] + c2[m]; }
-    const Vec4<R> t = face_flux<R, 0>(a, g, p[0], pv, b1, c1, o, n, relaxation(a, R(1), ga.dt));
-    const R fn = sn * t.u;
-    Vec4<R> out;
+    const Vec4<double> t = face_flux<0>(g, p[0], pv, b1, c1, o, n, relaxation(a, 1.0, ga.dt));
+    const double fn = sn * t.u;
+    Vec4<double> out;
     out.rho = t.rho * ga.area;
     out.u = (axis == 0 ? fn : t.v) * ga.area;
     out.v = (axis == 1 ? fn : (axis == 0 ? t.v : t.w)) * ga.area;
@@ -448,10 +371,9 @@ template <typename R> __device__ __forceinline__ void grid_boundary(const FluidA
     a.flux[a.ni + b] = out;
 }
 
-template <typename R, int BLOCKS>
-__global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidArgs<R> a, GridArgs<R> ga) {
+__global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_step(FluidArgs<double> a, GridArgs ga) {
     extern __shared__ __align__(16) unsigned char raw[];
-    constexpr int H = Half<R>::n, TB = kUniformThreads;
+    constexpr int H = 2, TB = kUniformThreads;  // H 16-byte pieces of a state record
     pdl_trigger();
     const int bnd = bnd_before(ga, blockIdx.x);
     if (bnd_before(ga, blockIdx.x + 1) > bnd) {
@@ -462,13 +384,13 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
     const GridTile t = ga.tiles[blockIdx.x - bnd];
     const GridInst gi = ga.inst[t.inst];
     const int Q = ga.plane_stride;
-    Planes<R> pl;
-    pl.h = reinterpret_cast<typename Half<R>::type *>(raw);
+    Planes pl;
+    pl.h = reinterpret_cast<double2 *>(raw);
     pl.Q = Q;
     double *sum = reinterpret_cast<double *>(pl.h + (size_t)kSlots * H * Q);  // [4][TB] the columns' sums
-    GridSide<R> *stage = reinterpret_cast<GridSide<R> *>(sum + 4 * TB);       // [stage_max] ghosts' records
-    R *vis = reinterpret_cast<R *>(stage + ga.stage_max);                     // [3][Q]
-    R *fx = vis + 3 * Q, *fy = fx + 4 * TB, *below = fy + 4 * TB;             // [4][TB]: the plane's fluxes, states two planes down
+    GridSide *stage = reinterpret_cast<GridSide *>(sum + 4 * TB);       // [stage_max] ghosts' records
+    double *vis = reinterpret_cast<double *>(stage + ga.stage_max);                     // [3][Q]
+    double *fx = vis + 3 * Q, *fy = fx + 4 * TB, *below = fy + 4 * TB;             // [4][TB]: the plane's fluxes, states two planes down
     const int tid = threadIdx.x, W = t.w + 3;
     const int nxy = gi.nx * gi.ny;
     const int z_end = t.z0 + t.d;
@@ -516,8 +438,8 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
             const int p = tid + q * TB;
             const int c = load_c[q] + nxy * kc;
             if (set) {  // the ghost of cell c across the grid's first or last plane
-                const Vec4<R> own = a.state[c];
-                R s[4] = {own.rho, own.u, own.v, own.w};
+                const Vec4<double> own = a.state[c];
+                double s[4] = {own.rho, own.u, own.v, own.w};
                 side_ghost(a, ga.side[gi.side0[side] + load_c[q] - gi.cell0], s);
                 pl.put(base + p, s);
             } else {
@@ -525,7 +447,7 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
 #pragma unroll
                 for (int e = 0; e < H; e++) copy16(pl.h + base + e * Q + p, src + 16 * e);
             }
-            if (k > 0) copy_small<sizeof(R)>(vis + ((k - 1) % 3) * Q + p, a.visc_factor + load_c[q] + nxy * (k - 1));
+            if (k > 0) copy8(vis + ((k - 1) % 3) * Q + p, a.visc_factor + load_c[q] + nxy * (k - 1));
         }
         if (ghost_at >= 0 && side < 0) {
             const char *src = reinterpret_cast<const char *>(a.state + ghost_c + nxy * k);
@@ -534,16 +456,16 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
             if (ghost_set && staged) {
                 const char *rec = reinterpret_cast<const char *>(ga.side + ghost_rec + (size_t)ghost_step * k);
 #pragma unroll
-                for (int e = 0; e < (int)(sizeof(GridSide<R>) / 16); e++)
+                for (int e = 0; e < (int)(sizeof(GridSide) / 16); e++)
                     copy16(reinterpret_cast<char *>(stage + tid) + 16 * e, rec + 16 * e);
             }
         }
     };
     // this thread's copies have arrived; its ghost of plane k is set where it is not zero-gradient
     auto landed = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
-    auto set_ghost = [&](int k, const GridSide<R> &rec) {
+    auto set_ghost = [&](int k, const GridSide &rec) {
         const int at = H * (k & (kSlots - 1)) * Q + ghost_at;
-        R s[4];
+        double s[4];
         pl.get(at, s);
         side_ghost(a, rec, s);
         pl.put(at, s);
@@ -554,13 +476,13 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
     const int gx = t.x0 + lx, gy = t.y0 + ly;
     const int at = (ly + 2) * W + lx + 2;
     const int c00 = gi.cell0 + gx + gi.nx * gy;
-    const R tau1 = relaxation(a, R(1), ga.dt);  // at a viscosity factor of 1
+    const double tau1 = relaxation(a, 1.0, ga.dt);  // at a viscosity factor of 1
     const size_t n = (size_t)a.nc;
 
     for (int k = t.z0 - 1; k <= t.z0 + 1; k++) bring(k, false);
     if (own && t.z0 > 0) {  // two planes down: the plane's cell, or the ghost of the first plane's
-        const Vec4<R> q = a.state[c00 + nxy * max(t.z0 - 2, 0)];
-        R s[4] = {q.rho, q.u, q.v, q.w};
+        const Vec4<double> q = a.state[c00 + nxy * max(t.z0 - 2, 0)];
+        double s[4] = {q.rho, q.u, q.v, q.w};
         if (t.z0 == 1 && (gi.active & 16)) side_ghost(a, ga.side[gi.side0[4] + c00 - gi.cell0], s);
 #pragma unroll
         for (int m = 0; m < 4; m++) below[m * TB + tid] = s[m];
@@ -579,11 +501,11 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
         const int pm = o * ((k - 1) & (kSlots - 1)), pk = o * (k & (kSlots - 1)), pp = o * ((k + 1) & (kSlots - 1));
         if (k + 1 < z_end) bring(k + 2, true);  // over plane k - 2, last read before the barrier
         const int c = c00 + nxy * k;
-        CellSlopes<R> cell;
+        CellSlopes cell;
         if (own) {
             pl.get(pk + at, cell.s);
-            auto diff = [&](int m0, int p1, R (&d)[4]) {
-                R q0[4], q1[4];
+            auto diff = [&](int m0, int p1, double (&d)[4]) {
+                double q0[4], q1[4];
                 pl.get(m0, q0);
                 pl.get(p1, q1);
 #pragma unroll
@@ -593,40 +515,40 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
             diff(pk + at - W, pk + at + W, cell.d[1]);
             diff(pm + at, pp + at, cell.d[2]);
             ga.prev[c] = {cell.s[1], cell.s[2], cell.s[3], cell.s[0]};
-            const R *vis0 = vis + (k % 3) * Q + at;
+            const double *vis0 = vis + (k % 3) * Q + at;
             if (gx > 0) {
                 const int l = pk + at - 1;
-                const Vec4<R> v = uniform_flux<R, 0>(a, ga, pl, cell, l, pl.at(l - 1), l - W, l + W, pm + at - 1,
+                const Vec4<double> v = uniform_flux<0>(ga, pl, cell, l, pl.at(l - 1), l - W, l + W, pm + at - 1,
                                                      pp + at - 1, tau1 * vis0[-1]);
-                R *f = fx + tid;
+                double *f = fx + tid;
                 f[0] = v.rho; f[TB] = v.u; f[2 * TB] = v.v; f[3 * TB] = v.w;
                 if (lx == 0) ga.edge[c] = v;
             }
             if (gy > 0) {
                 const int l = pk + at - W;
-                const Vec4<R> v = uniform_flux<R, 1>(a, ga, pl, cell, l, pl.at(l - W), l - 1, l + 1, pm + at - W,
+                const Vec4<double> v = uniform_flux<1>(ga, pl, cell, l, pl.at(l - W), l - 1, l + 1, pm + at - W,
                                                      pp + at - W, tau1 * vis0[-W]);
-                R *f = fy + tid;
+                double *f = fy + tid;
                 f[0] = v.rho; f[TB] = v.u; f[2 * TB] = v.v; f[3 * TB] = v.w;
                 if (ly == 0) ga.edge[n + c] = v;
             }
         }
         __syncthreads();
         if (own) {
-            Vec4<R> z{};
+            Vec4<double> z{};
             if (k > 0) {
                 const int l = pm + at;
-                State4<R> two;  // of plane k - 2
+                State4 two;  // of plane k - 2
 #pragma unroll
                 for (int m = 0; m < 4; m++) two.s[m] = below[m * TB + tid];
-                z = uniform_flux<R, 2>(a, ga, pl, cell, l, two, l - 1, l + 1, l - W, l + W, tau1 * vis[((k - 1) % 3) * Q + at]);
+                z = uniform_flux<2>(ga, pl, cell, l, two, l - 1, l + 1, l - W, l + W, tau1 * vis[((k - 1) % 3) * Q + at]);
                 if (k == t.z0) ga.edge[2 * n + c] = z;
             }
-            R lo[4];
+            double lo[4];
             pl.get(pm + at, lo);
 #pragma unroll
             for (int m = 0; m < 4; m++) below[m * TB + tid] = lo[m];
-            const R zl[4] = {z.rho, z.u, z.v, z.w};
+            const double zl[4] = {z.rho, z.u, z.v, z.w};
             double below_sum[4];
 #pragma unroll
             for (int m = 0; m < 4; m++) {
@@ -649,26 +571,19 @@ __global__ void __launch_bounds__(kUniformThreads, BLOCKS) k_uniform_step(FluidA
 
 }  // namespace
 
-template <typename R> size_t grid_smem_bytes(const GridArgs<R> &ga) {
-    return sizeof(R) * ((kSlots * 4 + 3) * (size_t)ga.plane_stride + 12 * (size_t)kUniformThreads) +
-           32 * (size_t)kUniformThreads + ga.stage_max * sizeof(GridSide<R>);
+size_t grid_smem_bytes(const GridArgs &ga) {
+    return sizeof(double) * ((kSlots * 4 + 3) * (size_t)ga.plane_stride + 12 * (size_t)kUniformThreads) +
+           32 * (size_t)kUniformThreads + ga.stage_max * sizeof(GridSide);
 }
 // The limit is the kernel's, shared by every handle: always the largest.
-template <typename R> cudaError_t grid_prepare() {
-    return cudaFuncSetAttribute(k_uniform_step<R, GridShape<R>::blocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+cudaError_t grid_prepare() {
+    return cudaFuncSetAttribute(k_uniform_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
 }
 static_assert(sizeof(double) * ((kSlots * 4 + 3) * kUniformPlaneMax + 12 * kUniformThreads) +
-                      kUniformThreads * (32 + sizeof(GridSide<double>)) <= 64 * 1024,
+                      kUniformThreads * (32 + sizeof(GridSide)) <= 64 * 1024,
               "a tile's shared memory");
-template <typename R> void launch_grid_step(const FluidArgs<R> &a, const GridArgs<R> &ga, cudaStream_t s) {
-    k_uniform_step<R, GridShape<R>::blocks>
-        <<<ga.bnd_blocks + ga.n_tiles, kUniformThreads, grid_smem_bytes(ga), s>>>(a, ga);
+void launch_grid_step(const FluidArgs<double> &a, const GridArgs &ga, cudaStream_t s) {
+    k_uniform_step<<<ga.bnd_blocks + ga.n_tiles, kUniformThreads, grid_smem_bytes(ga), s>>>(a, ga);
 }
-template size_t grid_smem_bytes<double>(const GridArgs<double> &);
-template size_t grid_smem_bytes<float>(const GridArgs<float> &);
-template cudaError_t grid_prepare<double>();
-template cudaError_t grid_prepare<float>();
-template void launch_grid_step<double>(const FluidArgs<double> &, const GridArgs<double> &, cudaStream_t);
-template void launch_grid_step<float>(const FluidArgs<float> &, const GridArgs<float> &, cudaStream_t);
 
 }  // namespace lbfs

@@ -9,6 +9,10 @@
 // it); a periodic partner is a boundary cell; and gamma is 1.  The generator's uniform
 // meshes and their ensembles meet this; it is checked face by face and cell by
 // cell at create, and any other mesh keeps the separate kernels.
+//
+// FP64 handles only.  An FP32 form of the pass was bound by instruction issue: alone
+// a handle gained by it (32^3 duct 14.2 -> 12.0 us a step, 64^3 34 -> 31.5), but three
+// handles of 57x45x33 cells in turn lost (112 -> 122 us for ten steps).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,9 +23,8 @@
 
 namespace lbfs {
 
-// Blocks per SM the kernel is compiled for: FP64 four of 128 registers, FP32 six of 80.
-template <typename R> struct GridShape { static constexpr int blocks = sizeof(R) == 8 ? 4 : 6; };
 constexpr int kUniformThreads = 128;   // a column each
+constexpr int kUniformBlocks = 4;      // blocks an SM, 128 registers a thread
 constexpr int kUniformPlaneMax = 230;  // cells of a tile's plane with two more below and one above along x and y
 
 struct GridTile {
@@ -36,8 +39,8 @@ struct GridInst {
 // The ghost of one boundary face as its cell's gradients need it: val the
 // Dirichlet values (velocity profiles of types 9 and 10 evaluated), flags which
 // components take them (the others copy the cell), or the periodic partner's.
-template <typename R> struct alignas(16) GridSide {
-    Vec4<R> val;
+struct GridSide {
+    Vec4<double> val;
     // bit 0: rho Dirichlet, 1: velocity Dirichlet, 2: rho periodic, 3: velocity periodic, 4: the face takes
     // the velocity val itself (type 1)
     int flags, partner;
@@ -51,31 +54,31 @@ struct alignas(16) GridBnd {
 };
 
 // Multiples of the slope weight w = dt x gradient weight: 3 w, 3 w^2, w / 2, 3 w / 2, 3 w^2 / 4.
-template <typename R> struct GridWeights {
-    R w, w3, ww3, h, h3, hh3;
+struct GridWeights {
+    double w, w3, ww3, h, h3, hh3;
 };
 
-template <typename R> struct GridArgs {
+struct GridArgs {
     int n_tiles, bnd_blocks;
     int plane_stride;              // cells of the largest tile's plane
     int stage_max;                 // threads that may hold a ghost's record
     const GridTile *tiles;
     const GridInst *inst;
-    const GridSide<R> *side;       // the boundary faces of every side of every instance
+    const GridSide *side;       // the boundary faces of every side of every instance
     const GridBnd *bnd;            // [nb]
-    const GridSide<R> *bnd_side;   // [nb] the boundary faces' records in their own order
-    R bnd_k;                       // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
-    GridWeights<R> cw;
-    R area, dt;                    // of every interior face
-    Vec4<R> *prev;                 // [nc + nb] the state the last step started from
+    const GridSide *bnd_side;   // [nb] the boundary faces' records in their own order
+    double bnd_k;                       // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
+    GridWeights cw;
+    double area, dt;                    // of every interior face
+    Vec4<double> *prev;                 // [nc + nb] the state the last step started from
     double4 *res;                  // [nc] sums of the interior face fluxes per unit area, those in edge left out
-    Vec4<R> *edge;                 // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes
+    Vec4<double> *edge;                 // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes
     const unsigned char *sides;    // [nc] bit 0: the cell has boundary faces; bits 1, 2, 3: its upper x, y, z flux is in edge
 };
 
-template <typename R> size_t grid_smem_bytes(const GridArgs<R> &ga);
-template <typename R> cudaError_t grid_prepare();
+size_t grid_smem_bytes(const GridArgs &ga);
+cudaError_t grid_prepare();
 // boundary face fluxes and the cells' interior sums of one step
-template <typename R> void launch_grid_step(const FluidArgs<R> &a, const GridArgs<R> &ga, cudaStream_t s);
+void launch_grid_step(const FluidArgs<double> &a, const GridArgs &ga, cudaStream_t s);
 
 }  // namespace lbfs

@@ -57,13 +57,12 @@ struct lbfs_solver {
     // tiles of the face kernel (interior faces ordered by owner within each axis), one table per flux
     // block size 64 / 128 / 256: tiles_h[b] = first face of each axis owned by tile t (3 ints per
     // tile, n_tiles + 1 rows), tile_maxnb[b][t] = largest neighbour of the faces of tiles <= t
-    // fused fluid step of structured grids (lbfs_fused.h): grid64 / grid32 hold its plan when `fused`.
+    // fused fluid step of structured grids (lbfs_fused.h, FP64 handles): its plan when `fused`.
     // separate: steps take the separate kernels all the same (the adjoint's recording, which reads
     // every step's gradients).  fields_stale: the last step left no gradients, fluxes or ghosts; they
     // are formed from the state it started from when asked for.
     bool fused = false, separate = false, fields_stale = false;
-    GridArgs<double> grid64{};
-    GridArgs<float> grid32{};
+    GridArgs grid{};
     cudaGraphExec_t graph_separate = nullptr;
     bool tiled = false;
     std::vector<int> tiles_h[3], tile_maxnb[3];
@@ -98,7 +97,7 @@ struct lbfs_solver {
         long long taken = 0;  // by them
         bool failed = false;
     };
-    StepRun run, run_separate;
+    StepRun run;
     // lbfs_step_until: one graph whose while node repeats the step and a convergence check
     cudaGraphExec_t loop_graph = nullptr;
     bool loop_unavailable = false;  // the loop graph could not be built (steps go one at a time)
@@ -152,10 +151,8 @@ bool dynamic_dt(const lbfs_params &p) { return p.time_stepping != 0 && p.time_st
 // The cached graphs of a step hold the launch shape, the stream and the kernel arguments: dropped
 // whenever one of those changes.
 void drop_step_graphs(lbfs_solver *s) {
-    for (lbfs_solver::StepRun *r : {&s->run, &s->run_separate}) {
-        if (r->graph) cudaGraphExecDestroy(r->graph);
-        *r = lbfs_solver::StepRun{};
-    }
+    if (s->run.graph) cudaGraphExecDestroy(s->run.graph);
+    s->run = lbfs_solver::StepRun{};
     if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; s->graph_steps = 0; }
     if (s->graph_separate) { cudaGraphExecDestroy(s->graph_separate); s->graph_separate = nullptr; }
     if (s->loop_graph) { cudaGraphExecDestroy(s->loop_graph); s->loop_graph = nullptr; }
@@ -170,9 +167,6 @@ struct DevBuf {
 template <typename R> FluidArgs<R> &fluid(lbfs_solver *s);
 template <> FluidArgs<double> &fluid<double>(lbfs_solver *s) { return s->f64; }
 template <> FluidArgs<float> &fluid<float>(lbfs_solver *s) { return s->f32; }
-template <typename R> GridArgs<R> &grid(lbfs_solver *s);
-template <> GridArgs<double> &grid<double>(lbfs_solver *s) { return s->grid64; }
-template <> GridArgs<float> &grid<float>(lbfs_solver *s) { return s->grid32; }
 
 int check_mesh(const lbfs_mesh_desc *m) {
     if (!m) return set_error(LBFS_ERR_ARG, "mesh descriptor is null");
@@ -213,9 +207,9 @@ int check_mesh(const lbfs_mesh_desc *m) {
     return LBFS_OK;
 }
 
-template <typename R>
-int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>> &lsw,
-              const std::vector<AxisFace<R>> &axf, const std::vector<GenFace<R>> &gen, const std::vector<BcRec<R>> &bcr);
+int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<double>> &lsw,
+              const std::vector<AxisFace<double>> &axf, const std::vector<GenFace<double>> &gen,
+              const std::vector<BcRec<double>> &bcr);
 
 template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     FluidArgs<R> &a = fluid<R>(s);
@@ -512,7 +506,8 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     a.n_membranes = 0;
     a.instances = nullptr;
     a.cell_instance = nullptr;
-    return plan_grid<R>(s, m, lsw, axf, gen, bcr);
+    if constexpr (sizeof(R) == 8) return plan_grid(s, m, lsw, axf, gen, bcr);
+    else return LBFS_OK;
 }
 
 // Tiles of an instance's grid for the fused step: columns of w x h cells walked
@@ -548,16 +543,13 @@ TileShape tile_shape(int nx, int ny) {
 // The fused step's plan: the conditions of lbfs_fused.h over every face and
 // cell, the geometry by direction, and the tiles.  Leaves s->fused false where a
 // condition fails (LBFS_SEPARATE_KERNELS set: always; a diagnostic switch).
-template <typename R>
-int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>> &lsw,
-              const std::vector<AxisFace<R>> &axf, const std::vector<GenFace<R>> &gen, const std::vector<BcRec<R>> &bcr) {
-    FluidArgs<R> &a = fluid<R>(s);
-    GridArgs<R> &ga = grid<R>(s);
+int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<double>> &lsw,
+              const std::vector<AxisFace<double>> &axf, const std::vector<GenFace<double>> &gen,
+              const std::vector<BcRec<double>> &bcr) {
+    FluidArgs<double> &a = s->f64;
+    GridArgs &ga = s->grid;
     s->fused = false;
     if (!a.axis_aligned || a.ni == 0 || std::getenv("LBFS_SEPARATE_KERNELS")) return LBFS_OK;
-    // FP32 keeps the separate kernels: bound by instruction issue in both forms, the fused pass took 22 us
-    // against their 21 at 64^3 (two ducts of 57 x 45 x 33 side by side: 3 % more)
-    if (s->fp32) return LBFS_OK;
     const int nc = a.nc, ni = a.ni, nb = a.nb;
     // the instances' grids, and each cell's place in its grid
     std::vector<GridInst> inst;
@@ -624,16 +616,16 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
         sides[o] = 1;
     }
     // the ghosts as the gradients take them (ghost_state)
-    std::vector<GridSide<R>> side(nb), bnd_side(nb);
+    std::vector<GridSide> side(nb), bnd_side(nb);
     std::vector<GridBnd> bnd(nb);
     std::vector<int> face_of(nc, -1);  // a boundary face of the cell
     for (size_t e = 0; e < side.size(); e++) {
         const int b = side_bc[e], rt = m->bc_rho_type[b], vt = m->bc_vel_type[b], ghost = nc + b;
         const double *v = m->bc_values + 4 * (size_t)b;
-        const R gy = (R)m->cell_centroid[3 * (size_t)ghost + 1], gz = (R)m->cell_centroid[3 * (size_t)ghost + 2];
-        GridSide<R> q{};
-        q.val = {(R)v[0], (R)v[1], (R)v[2], (R)(v[3] - (double)a.rho0)};
-        if (vt == 9) q.val.u = (R)(16 * (double)q.val.u * (a.H2 + gy) * (a.H2 - gy) * (a.H2 + gz) * (a.H2 - gz) / a.H4);
+        const double gy = m->cell_centroid[3 * (size_t)ghost + 1], gz = m->cell_centroid[3 * (size_t)ghost + 2];
+        GridSide q{};
+        q.val = {v[0], v[1], v[2], v[3]};
+        if (vt == 9) q.val.u = 16 * q.val.u * (a.H2 + gy) * (a.H2 - gy) * (a.H2 + gz) * (a.H2 - gz) / a.H4;
         else if (vt == 10) q.val.u = gy * q.val.u;
         q.flags = (rt == 1 ? 1 : 0) | (vt == 1 || vt == 9 || vt == 10 ? 2 : 0) | (rt == 3 ? 4 : 0) | (vt == 3 ? 8 : 0) |
                   (vt == 1 ? 16 : 0);
@@ -663,25 +655,25 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
         if (bnd[b].partner < 0) return LBFS_OK;
     }
     // every boundary face like the interior ones, its ghost straight across it
-    if (a.gamma_inv != R(1) || a.recon_q != R(1)) return LBFS_OK;
+    if (a.gamma_inv != 1.0 || a.recon_q != 1.0) return LBFS_OK;
     for (int b = 0; b < nb; b++) {
-        const GenFace<R> &f = gen[b];
-        const BcRec<R> &r = bcr[b];
+        const GenFace<double> &f = gen[b];
+        const BcRec<double> &r = bcr[b];
         const int ax = side_of[b] / 2;
-        const R sn = (side_of[b] & 1) ? R(1) : R(-1);
-        const R nv[3] = {f.nx, f.ny, f.nz}, t1[3] = {f.t1x, f.t1y, f.t1z}, t2[3] = {f.t2x, f.t2y, f.t2z};
-        const R dn[3] = {r.dnx, r.dny, r.dnz}, mv[3] = {r.mx, r.my, r.mz};
+        const double sn = (side_of[b] & 1) ? 1.0 : -1.0;
+        const double nv[3] = {f.nx, f.ny, f.nz}, t1[3] = {f.t1x, f.t1y, f.t1z}, t2[3] = {f.t2x, f.t2y, f.t2z};
+        const double dn[3] = {r.dnx, r.dny, r.dnz}, mv[3] = {r.mx, r.my, r.mz};
         if (f.area != axf[0].area || f.dt != axf[0].dt || r.dmag != bcr[0].dmag) return LBFS_OK;
         for (int q = 0; q < 3; q++) {
-            const R e = q == ax ? sn : R(0);
-            if (nv[q] != e || dn[q] != e || t1[q] != -f.dt * e || t2[q] != f.dt * e || mv[q] != (q == ax ? R(0) : R(1)))
+            const double e = q == ax ? sn : 0.0;
+            if (nv[q] != e || dn[q] != e || t1[q] != -f.dt * e || t2[q] != f.dt * e || mv[q] != (q == ax ? 0.0 : 1.0))
                 return LBFS_OK;
         }
-        if (f.bc_branch == R(0)) bnd[b].info |= 1024;
+        if (f.bc_branch == 0.0) bnd[b].info |= 1024;
     }
     // every gradient stencil is the six neighbours, weighted along their axes alone by one magnitude
     // (ref: a lower neighbour's weight)
-    R ref = R(0);
+    double ref = 0.0;
     for (int c = 0; c < nc; c++) {
         int seen = 0;
         for (int q = 0; q < 6; q++) {
@@ -695,10 +687,10 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
             }
             if (d == 6 || (seen >> d & 1)) return LBFS_OK;
             seen |= 1 << d;
-            const R *v = lsw[c].w + 3 * q;
+            const double *v = lsw[c].w + 3 * q;
             if (c == 0 && q == 0) ref = (d & 1) ? -v[d / 2] : v[d / 2];
             for (int r = 0; r < 3; r++)
-                if (v[r] != (r == d / 2 ? ((d & 1) ? -ref : ref) : R(0))) return LBFS_OK;
+                if (v[r] != (r == d / 2 ? ((d & 1) ? -ref : ref) : 0.0)) return LBFS_OK;
         }
     }
     // every interior face has one area and dt and lies dt from both centres
@@ -706,12 +698,12 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
     ga.dt = axf[0].dt;
     for (int f = 0; f < ni; f++)
         if (axf[f].area != ga.area || axf[f].dt != ga.dt || axf[f].t1 != -ga.dt || axf[f].t2 != ga.dt) return LBFS_OK;
-    const R c = -ref * ga.dt;
-    ga.cw = {c, R(3) * c, R(3) * c * c, R(0.5) * c, R(1.5) * c, R(0.75) * c * c};
-    ga.bnd_k = nb > 0 ? ga.dt / (bcr[0].dmag * c) : R(0);
+    const double c = -ref * ga.dt;
+    ga.cw = {c, 3.0 * c, 3.0 * c * c, 0.5 * c, 1.5 * c, 0.75 * c * c};
+    ga.bnd_k = nb > 0 ? ga.dt / (bcr[0].dmag * c) : 0.0;
     int rc;
     // the tiles, with one walk length d for all instances.  A block's time is d planes and a start of 1.2
-    // (clock stamps inside the kernel), a plane's about 3000 cycles and 1300 (FP64) or 1100 (FP32) for each
+    // (clock stamps inside the kernel), a plane's about 3000 cycles and 1300 for each
     // block on its SM.  Grids of at most one wave: the longest block at that occupancy; larger ones: the
     // blocks' throughput and a third of a block for the last wave.  64^3 FP64: 45 us at the chosen d = 4,
     // 47 at 3, 54 at 8; 128^3: 203 at 8, 206 at 4, 213 at 16.
@@ -721,8 +713,8 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
         if (t.w == 0) return LBFS_OK;
         shape.push_back(t);
     }
-    const int per_sm = GridShape<R>::blocks;
-    auto plane_time = [](int blocks) { return 3000.0 + (sizeof(R) == 8 ? 1300.0 : 1100.0) * blocks; };
+    const int per_sm = kUniformBlocks;
+    auto plane_time = [](int blocks) { return 3000.0 + 1300.0 * blocks; };
     int depth = 1;
     double best = 1e300;
     for (int d = 1; d <= 64; d++) {
@@ -766,12 +758,12 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
     }
     GridTile *d_tiles;
     GridInst *d_inst;
-    GridSide<R> *d_side;
+    GridSide *d_side;
     GridBnd *d_bnd;
-    GridSide<R> *d_bside;
+    GridSide *d_bside;
     unsigned char *d_sides;
     double4 *d_res;
-    Vec4<R> *d_prev;
+    Vec4<double> *d_prev;
     if ((rc = s->upload(&d_tiles, tiles)) || (rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) ||
         (rc = s->upload(&d_bnd, bnd)) || (rc = s->upload(&d_bside, bnd_side)) ||
         (rc = s->upload(&d_sides, sides)) || (rc = s->alloc(&d_res, nc)) || (rc = s->alloc(&d_prev, (size_t)nc + nb)))
@@ -797,7 +789,7 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<R>>
     ga.bnd_blocks = (nb + kUniformThreads - 1) / kUniformThreads;
     ga.plane_stride = P;
     ga.stage_max = G;
-    if (grid_prepare<R>() != cudaSuccess) {
+    if (grid_prepare() != cudaSuccess) {
         cudaGetLastError();
         return LBFS_OK;
     }
@@ -1412,21 +1404,21 @@ int fork_behind_launch(lbfs_solver *s) {
 // gradient kernel to follow here: behind the pass, whose blocks hold every
 // register of an SM until they end, the chain came late (us per step, behind /
 // beside: 44.6 / 36.5 on 48^3 with 162 nodes, 64.8 / 55.5 at 64^3 with 642).
-template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
-    const GridArgs<R> &ga = grid<R>(s);
-    FluidArgs<R> a = fluid<R>(s);
+int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
+    const GridArgs &ga = s->grid;
+    FluidArgs<double> a = s->f64;
     a.grid_res = ga.res;
     a.grid_sides = ga.sides;
     int n = 0;
     for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = false;
     if (s->profiling) LBFS_CUDA(record_event(s->ev_phase[5][0], s->stream));
     if (a.time_stepping != 0 && a.time_stepping != LBFS_DT_CONSTANT) {
-        launch_fluid_cfl<R>(a, s->stream);
+        launch_fluid_cfl<double>(a, s->stream);
         n += 1;
     }
     auto pass = [&]() {
         PhaseMark m(s, 2, s->stream);
-        launch_grid_step<R>(a, ga, s->stream);
+        launch_grid_step(a, ga, s->stream);
         n += 1;
     };
     if (s->n_membranes == 0) {
@@ -1449,7 +1441,7 @@ template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, i
         pass();
         LBFS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_join, 0));
     }
-    { PhaseMark m(s, 3, s->stream); launch_fluid_update<R>(a, s->stream, !s->kernel_events); }
+    { PhaseMark m(s, 3, s->stream); launch_fluid_update<double>(a, s->stream, !s->kernel_events); }
     n += 1;
     if (s->profiling) {
         LBFS_CUDA(record_event(s->ev_phase[5][1], s->stream));
@@ -1461,7 +1453,7 @@ template <typename R> int enqueue_fused_step(lbfs_solver *s, bool visc_update, i
 }
 
 template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *launches) {
-    if (s->fused && !s->separate) return enqueue_fused_step<R>(s, visc_update, launches);
+    if (s->fused && !s->separate) return enqueue_fused_step(s, visc_update, launches);
     FluidArgs<R> &a = fluid<R>(s);
     int n = 0;
     for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = false;
@@ -1534,20 +1526,15 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
 
 // Gradients, face fluxes and ghosts of the last fused step, formed by the
 // separate kernels from the state it started from; on the handle's stream.
-template <typename R> int form_fields(lbfs_solver *s) {
-    FluidArgs<R> a = fluid<R>(s);
-    a.state = grid<R>(s).prev;
-    launch_fluid_gradients<R>(a, s->stream);
-    launch_fluid_flux<R>(a, s->stream);
-    LBFS_CUDA(cudaGetLastError());
-    LBFS_CUDA(cudaMemcpyAsync(fluid<R>(s).state + s->nc, a.state + s->nc, sizeof(Vec4<R>) * (size_t)s->nb,
-                              cudaMemcpyDeviceToDevice, s->stream));
-    return LBFS_OK;
-}
 int ensure_fields(lbfs_solver *s) {
     if (!s->fields_stale) return LBFS_OK;
-    int rc = s->fp32 ? form_fields<float>(s) : form_fields<double>(s);
-    if (rc) return rc;
+    FluidArgs<double> a = s->f64;
+    a.state = s->grid.prev;
+    launch_fluid_gradients<double>(a, s->stream);
+    launch_fluid_flux<double>(a, s->stream);
+    LBFS_CUDA(cudaGetLastError());
+    LBFS_CUDA(cudaMemcpyAsync(s->f64.state + s->nc, a.state + s->nc, sizeof(Vec4<double>) * (size_t)s->nb,
+                              cudaMemcpyDeviceToDevice, s->stream));
     s->fields_stale = false;
     return LBFS_OK;
 }
@@ -1810,7 +1797,8 @@ int build_step_graph(lbfs_solver *s, int steps, cudaGraphExec_t *graph) {
 constexpr int kRunSteps = 16;
 constexpr long long kRunAfter = 256;
 
-void plan_step_run(lbfs_solver *s, lbfs_solver::StepRun *r, int n_steps) {
+void plan_step_run(lbfs_solver *s, int n_steps) {
+    lbfs_solver::StepRun *r = &s->run;
     const int asked = std::min(n_steps, kRunSteps);
     if (asked != r->asked) {
         r->asked = asked;
@@ -1840,10 +1828,10 @@ extern "C" int lbfs_step_graph(lbfs_solver *s, int32_t n_steps) {
         s->graph_steps = 1;
         for (int p = 0; p < kPhases; p++) s->graph_phase_recorded[p] = s->phase_recorded[p];
     }
-    lbfs_solver::StepRun &run = s->separate ? s->run_separate : s->run;
-    plan_step_run(s, &run, n_steps);
+    if (!s->separate) plan_step_run(s, n_steps);
+    const lbfs_solver::StepRun &run = s->run;
     for (int k = 0; k < n_steps; k++) {
-        bool together = run.graph && !s->profiling && n_steps - k >= run.steps;
+        bool together = run.graph && !s->separate && !s->profiling && n_steps - k >= run.steps;
         for (int q = 0; together && q < run.steps; q++) together = !visc_due(s, s->t + q) && !wrap_due(s, s->t + q);
         if (together) {
             LBFS_CUDA(cudaGraphLaunch(run.graph, s->stream));
