@@ -27,7 +27,7 @@ namespace lbfs {
 namespace {
 
 __device__ __forceinline__ double relaxation(const FluidArgs<double> &a, double vf, double dt) {
-    return (a.testcase == 8) ? 0.0 : (a.vi3.0 * vf * 3.0 / dt * a.gamma_inv);
+    return (a.testcase == 8) ? 0.0 : (a.visc * vf * 3.0 / dt * a.gamma_inv);
 }
 
 // The ghost of a cell (state s: rho, u, v, w) across a side with record gs, in place of s.
