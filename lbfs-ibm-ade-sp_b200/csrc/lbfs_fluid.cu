@@ -178,10 +178,12 @@ template <typename R> __device__ __forceinline__ void until_check(const FluidArg
     cudaGraphSetConditional(a.until.handle, (!converged && !diverged && c < u->limit) ? 1u : 0u);
 }
 
-// GRID: behind the fused step, whose cell sums over the interior faces it
+// FUSED: behind the fused step, whose cell sums over the interior faces it
 // reads (32 B instead of six fluxes of 32 / 16 B).  It subtracts the upper faces
 // that other tiles formed, z, x, y, scales the sum and adds the boundary faces.
-template <typename R, int TB, bool GRID>
+// MIXED: grids of several spacings, or cells that keep the separate kernels.
+enum Sums { GATHER, FUSED, MIXED };
+template <typename R, int TB, int SUMS>
 __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
     __shared__ double sh[4][TB / 32];
     __shared__ bool last_block;
@@ -221,17 +223,19 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
         const double iv = a.inv_volume_uniform ? a.inv_volume_all : __ldg(a.cell_inv_volume + i);
         double4 t = a.t1[i];  // in flight beside the sums (1 to 2 % of the step when loaded where it is used)
         double r[4] = {0, 0, 0, 0};  // rho, u, v, w
-        if constexpr (GRID) {
+        const unsigned sides = SUMS != GATHER ? a.grid_sides[i] : (unsigned)kSeparateCell;
+        if (SUMS == FUSED || (SUMS == MIXED && !(sides & kSeparateCell))) {
             const double4 q = a.grid_res[i];
             r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
-            const unsigned sides = a.grid_sides[i];
+            int sy = a.grid_stride[0], sz = a.grid_stride[1];
+            double area = a.grid_area;
+            if (SUMS == MIXED || ((sides & 14u) && sy == 0)) {
+                const GridCells g = a.grid_cells[__ldg(a.grid_instance + i)];
+                sy = g.sy;
+                sz = g.sz;
+                area = g.area;
+            }
             if (sides & 14u) {  // upper faces that another tile formed: z first, as a walk subtracts it
-                int sy = a.grid_stride[0], sz = a.grid_stride[1];
-                if (sy == 0) {
-                    const int2 q = a.grid_strides[__ldg(a.grid_instance + i)];
-                    sy = q.x;
-                    sz = q.y;
-                }
 #pragma unroll
                 for (int e = 0; e < 3; e++) {
                     const int d = (e + 2) % 3;
@@ -242,7 +246,7 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
                     for (int m = 0; m < 4; m++) r[m] = r[m] - fv[m];
                 }
             }
-            const double ia = iv * a.grid_area;
+            const double ia = iv * (SUMS == MIXED ? area : a.grid_area);
 #pragma unroll
             for (int m = 0; m < 4; m++) r[m] = __dmul_rn(r[m], ia);  // not contracted with what follows, whatever that is
             if (sides & 1u) {
@@ -528,17 +532,17 @@ template <typename R> void launch_fluid_flux(const FluidArgs<R> &a, cudaStream_t
     launch_fluid_flux_axis<R>(a, s);
     launch_fluid_flux_general<R>(a, s);
 }
-template <typename R, bool GRID> void launch_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
+template <typename R, int SUMS> void launch_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
     const int tb = a.tb_update, g = k3_grid(a);
-    if (tb == 128) launch_maybe_pdl(k_cell_update<R, 128, GRID>, g, 128, s, pdl, a);
-    else if (tb == 512) launch_maybe_pdl(k_cell_update<R, 512, GRID>, g, 512, s, pdl, a);
-    else launch_maybe_pdl(k_cell_update<R, 256, GRID>, g, 256, s, pdl, a);
+    if (tb == 128) launch_maybe_pdl(k_cell_update<R, 128, SUMS>, g, 128, s, pdl, a);
+    else if (tb == 512) launch_maybe_pdl(k_cell_update<R, 512, SUMS>, g, 512, s, pdl, a);
+    else launch_maybe_pdl(k_cell_update<R, 256, SUMS>, g, 256, s, pdl, a);
 }
 template <typename R> void launch_fluid_update(const FluidArgs<R> &a, cudaStream_t s, bool pdl) {
     if constexpr (sizeof(R) == 8) {
-        if (a.grid_res) return launch_update<R, true>(a, s, pdl);
+        if (a.grid_res) return a.grid_mixed ? launch_update<R, MIXED>(a, s, pdl) : launch_update<R, FUSED>(a, s, pdl);
     }
-    launch_update<R, false>(a, s, pdl);
+    launch_update<R, GATHER>(a, s, pdl);
 }
 
 template <typename R> void launch_fluid_cfl(const FluidArgs<R> &a, cudaStream_t s) {

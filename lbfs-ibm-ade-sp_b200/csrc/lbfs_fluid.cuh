@@ -187,6 +187,13 @@ struct UntilArgs {
     double ref_rho, ref_mom;
 };
 
+// Strides along y and z of an instance of the fused step and its face area.
+struct GridCells {
+    int sy, sz;
+    double area;
+};
+constexpr int kSeparateCell = 128;
+
 template <typename R> struct FluidArgs {
     int nc, nf, ni, nb, nfx, nfy, nfz, axis_aligned;
     int cone;  // general faces in three ranges, every normal within its axis' cone, n_A - |n_B| - |n_C| > 0.001 dt
@@ -251,15 +258,17 @@ template <typename R> struct FluidArgs {
     // leaves out, sum over the faces of -+ rho0/3 n area / volume (null when
     // every cell closes, where it vanishes)
     const double *closure;       // [3 nc]
-    // after the fused step of structured grids (lbfs_fused.h): the cells' sums over their interior
-    // faces and which cells have boundary faces (null after the separate kernels)
+    // after the fused step of structured grids (lbfs_fused.h): the cells' sums over their interior faces
+    // (null after the separate kernels).  grid_sides: bit 0: the cell has boundary faces; bits 1, 2, 3: its
+    // upper x, y, z flux is in grid_edge (GridArgs::edge); kSeparateCell: the cell keeps the separate kernels
     const double4 *grid_res;     // [nc] (rho, u, v, w)
-    const unsigned char *grid_sides;  // [nc] GridArgs::sides
-    const Vec4<R> *grid_edge;    // GridArgs::edge, with the face area and the strides along y and z
-    double grid_area;
-    int grid_stride[2];          // of the one instance; 0: grid_strides[grid_instance[cell]]
-    const int2 *grid_strides;
-    const int *grid_instance;
+    const unsigned char *grid_sides;  // [nc]
+    const Vec4<R> *grid_edge;
+    int grid_mixed;              // grids of several spacings, or instances that keep the separate kernels
+    double grid_area;            // face area and strides along y and z of the one instance (strides 0: grid_cells)
+    int grid_stride[2];
+    const GridCells *grid_cells; // [instances]
+    const int *grid_instance;    // [nc]
     double4 *t1;                 // [nc] (u, v, w, rho) conservative accumulator, FP64
     double *res_out;             // [4*nc] residuals kept for parity checks (null = not stored)
     // IBM patches (one per membrane), grouped by ensemble instance

@@ -368,7 +368,7 @@ __device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const 
     out.u = (axis == 0 ? fn : t.v) * ga.area;
     out.v = (axis == 1 ? fn : (axis == 0 ? t.v : t.w)) * ga.area;
     out.w = (axis == 2 ? fn : t.w) * ga.area;
-    a.flux[a.ni + b] = out;
+    a.flux[a.ni + f.face] = out;
 }
 
 __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_step(FluidArgs<double> a, GridArgs ga) {
@@ -377,8 +377,8 @@ __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_ste
     pdl_trigger();
     const int bnd = bnd_before(ga, blockIdx.x);
     if (bnd_before(ga, blockIdx.x + 1) > bnd) {
-        const int b = bnd * TB + threadIdx.x;
-        if (b < a.nb) grid_boundary(a, ga, b);
+        const int b = ga.bnd0 + bnd * TB + threadIdx.x;
+        if (b < ga.bnd1) grid_boundary(a, ga, b);
         return;
     }
     const GridTile t = ga.tiles[blockIdx.x - bnd];

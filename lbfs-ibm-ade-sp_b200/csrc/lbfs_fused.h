@@ -6,9 +6,10 @@
 // boundary face; a cell's gradient stencil is its six neighbours (or ghosts), each
 // with a weight along its axis alone and of one magnitude; every face has one area
 // and one dt and lies dt from both centres (a boundary face's ghost straight across
-// it); a periodic partner is a boundary cell; and gamma is 1.  The generator's uniform
-// meshes and their ensembles meet this; it is checked face by face and cell by
-// cell at create, and any other mesh keeps the separate kernels.
+// it); a periodic partner is a boundary cell; and gamma is 1.  Cells and faces are in
+// the generator's order.  Its uniform meshes and their ensembles meet this; it is
+// checked face by face and cell by cell at create, instance by instance, and any
+// other instance keeps the separate kernels.
 //
 // FP64 handles only.  An FP32 form of the pass was bound by instruction issue: alone
 // a handle gained by it (32^3 duct 14.2 -> 12.0 us a step, 64^3 34 -> 31.5), but three
@@ -48,9 +49,9 @@ struct GridSide {
 // One boundary face: its cell, the cell's strides along y and z, info -- its side d,
 // up to two more missing sides of the cell << 3 and << 6 (7: none) with their
 // boundary faces in more, bit 10: the interior branch (an instance's first ghost);
-// partner: a boundary face of the periodic partner cell.
+// partner: a boundary face of the periodic partner cell; face: its index among the mesh's boundary faces.
 struct alignas(16) GridBnd {
-    int cell, sy, sz, info, more[2], partner, pad;
+    int cell, sy, sz, info, more[2], partner, face;
 };
 
 // Multiples of the slope weight w = dt x gradient weight: 3 w, 3 w^2, w / 2, 3 w / 2, 3 w^2 / 4.
@@ -60,20 +61,20 @@ struct GridWeights {
 
 struct GridArgs {
     int n_tiles, bnd_blocks;
+    int bnd0, bnd1;                // boundary faces of this launch
     int plane_stride;              // cells of the largest tile's plane
     int stage_max;                 // threads that may hold a ghost's record
     const GridTile *tiles;
     const GridInst *inst;
-    const GridSide *side;       // the boundary faces of every side of every instance
-    const GridBnd *bnd;            // [nb]
-    const GridSide *bnd_side;   // [nb] the boundary faces' records in their own order
-    double bnd_k;                       // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
+    const GridSide *side;          // the boundary faces of every side of every instance
+    const GridBnd *bnd;            // the boundary faces, launch by launch
+    const GridSide *bnd_side;      // their records in that order
+    double bnd_k;                  // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
     GridWeights cw;
-    double area, dt;                    // of every interior face
-    Vec4<double> *prev;                 // [nc + nb] the state the last step started from
+    double area, dt;               // of every interior face
+    Vec4<double> *prev;            // [nc + nb] the state the last step started from
     double4 *res;                  // [nc] sums of the interior face fluxes per unit area, those in edge left out
-    Vec4<double> *edge;                 // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes
-    const unsigned char *sides;    // [nc] bit 0: the cell has boundary faces; bits 1, 2, 3: its upper x, y, z flux is in edge
+    Vec4<double> *edge;            // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes
 };
 
 size_t grid_smem_bytes(const GridArgs &ga);

@@ -57,12 +57,19 @@ struct lbfs_solver {
     // tiles of the face kernel (interior faces ordered by owner within each axis), one table per flux
     // block size 64 / 128 / 256: tiles_h[b] = first face of each axis owned by tile t (3 ints per
     // tile, n_tiles + 1 rows), tile_maxnb[b][t] = largest neighbour of the faces of tiles <= t
-    // fused fluid step of structured grids (lbfs_fused.h, FP64 handles): its plan when `fused`.
+    // fused fluid step of structured grids (lbfs_fused.h, FP64 handles): its launches, one per set of face
+    // constants, when `fused`, and the instances that keep the separate kernels (rest).
     // separate: steps take the separate kernels all the same (the adjoint's recording, which reads
     // every step's gradients).  fields_stale: the last step left no gradients, fluxes or ghosts; they
     // are formed from the state it started from when asked for.
     bool fused = false, separate = false, fields_stale = false;
-    GridArgs grid{};
+    std::vector<GridArgs> passes;
+    const unsigned char *grid_sides = nullptr;
+    struct Rest {
+        bool any = false;
+        int cell0 = 0, cell1 = 0;  // their cells and faces, with those of the grids between them
+        FaceRanges faces{};
+    } rest;
     cudaGraphExec_t graph_separate = nullptr;
     bool tiled = false;
     std::vector<int> tiles_h[3], tile_maxnb[3];
@@ -207,9 +214,21 @@ int check_mesh(const lbfs_mesh_desc *m) {
     return LBFS_OK;
 }
 
-int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<double>> &lsw,
-              const std::vector<AxisFace<double>> &axf, const std::vector<GenFace<double>> &gen,
-              const std::vector<BcRec<double>> &bcr);
+// The mesh as setup_fluid formed it: folded weights (code null) or each cell's codes into tab, whose
+// vectors lie along one axis (-1: not) with one value.
+struct GridMesh {
+    const std::vector<LsW<double>> &lsw;
+    const std::vector<AxisFace<double>> &axf;
+    const std::vector<GenFace<double>> &gen;
+    const std::vector<BcRec<double>> &bcr;
+    const unsigned *code;
+    struct Code {
+        int axis;
+        double value;
+    } tab[8];
+};
+
+int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm);
 
 template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     FluidArgs<R> &a = fluid<R>(s);
@@ -506,8 +525,16 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     a.n_membranes = 0;
     a.instances = nullptr;
     a.cell_instance = nullptr;
-    if constexpr (sizeof(R) == 8) return plan_grid(s, m, lsw, axf, gen, bcr);
-    else return LBFS_OK;
+    if constexpr (sizeof(R) == 8) {
+        GridMesh gm{lsw, axf, gen, bcr, coded ? lcode.data() : nullptr, {}};
+        for (int k = 0; k < n_tab; k++) {
+            const double *v = a.lsw_tab[k];
+            const int ax = v[0] != 0.0 ? 0 : (v[1] != 0.0 ? 1 : 2);
+            gm.tab[k] = {v[(ax + 1) % 3] == 0.0 && v[(ax + 2) % 3] == 0.0 ? ax : -1, v[ax]};
+        }
+        return plan_grid(s, m, gm);
+    }
+    return LBFS_OK;
 }
 
 // Tiles of an instance's grid for the fused step: columns of w x h cells walked
@@ -540,188 +567,277 @@ TileShape tile_shape(int nx, int ny) {
     return best;
 }
 
-// The fused step's plan: the conditions of lbfs_fused.h over every face and
-// cell, the geometry by direction, and the tiles.  Leaves s->fused false where a
-// condition fails (LBFS_SEPARATE_KERNELS set: always; a diagnostic switch).
-int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<double>> &lsw,
-              const std::vector<AxisFace<double>> &axf, const std::vector<GenFace<double>> &gen,
-              const std::vector<BcRec<double>> &bcr) {
-    FluidArgs<double> &a = s->f64;
-    GridArgs &ga = s->grid;
-    s->fused = false;
-    if (!a.axis_aligned || a.ni == 0 || std::getenv("LBFS_SEPARATE_KERNELS")) return LBFS_OK;
-    const int nc = a.nc, ni = a.ni, nb = a.nb;
-    // the instances' grids, and each cell's place in its grid
-    std::vector<GridInst> inst;
-    std::vector<int> place(nc);  // 6 bits: sides on which the cell has no neighbour; instance above
-    long long side_total = 0;
+// ---- the plan of the fused step (lbfs_fused.h) -------------------------------
+
+// One instance as the plan sees it: its grid, its faces (grouped by instance within each range) and,
+// where the conditions hold, the constants of its faces.
+struct GridCheck {
+    GridInst g{};
+    int face[3][2], bnd[2];  // its interior faces along each axis and its boundary faces
+    double area = 0, dt = 0, weight = 0, dmag = 0;
+    bool fits = false;
+};
+
+// First face of every instance in [f0, f1) (and f1), whose faces are grouped by instance; false where they are not.
+bool faces_by_instance(const lbfs_solver *s, const int *owner, int f0, int f1, std::vector<int> &first) {
+    first.clear();
+    int f = f0;
     for (const lbfs_grid_desc &g : s->grids) {
-        if (!(g.delta_x > 0)) return LBFS_OK;
-        long long n[3];
-        for (int d = 0; d < 3; d++) {
-            n[d] = std::llround(g.length[d] / g.delta_x);
-            if (n[d] < 1 || n[d] > nc) return LBFS_OK;
-        }
-        if (n[0] * n[1] > nc || n[0] * n[1] * n[2] != g.n_cells) return LBFS_OK;
-        GridInst q{};
-        q.cell0 = g.cell0; q.nx = (int)n[0]; q.ny = (int)n[1]; q.nz = (int)n[2];
-        const long long area[3] = {n[1] * n[2], n[0] * n[2], n[0] * n[1]};
-        for (int d = 0; d < 6; d++) {
-            q.side0[d] = (int)side_total;
-            side_total += area[d / 2];
-        }
-        int c = q.cell0;
-        for (int k = 0; k < q.nz; k++)
-            for (int j = 0; j < q.ny; j++)
-                for (int i = 0; i < q.nx; i++, c++)
-                    place[c] = (i == 0) | (i == q.nx - 1) << 1 | (j == 0) << 2 | (j == q.ny - 1) << 3 | (k == 0) << 4 |
-                               (k == q.nz - 1) << 5 | (int)inst.size() << 6;
-        inst.push_back(q);
+        first.push_back(f);
+        while (f < f1 && owner[f] >= g.cell0 && owner[f] < g.cell0 + g.n_cells) f++;
     }
-    if (side_total != nb) return LBFS_OK;  // every missing side has one boundary face
-    auto stride = [&](int c, int ax) {
-        const GridInst &q = inst[place[c] >> 6];
-        return ax == 0 ? 1 : (ax == 1 ? q.nx : q.nx * q.ny);
-    };
-    // every interior face joins a cell to its neighbour along one axis
-    std::vector<int> low_face(3 * (size_t)nc, -1);
-    for (int f = 0; f < ni; f++) {
-        const int o = m->owner[f], n = m->neighbour[f];
-        int ax = 0;
-        while (ax < 3 && !(n - o == stride(o, ax) && !(place[o] >> (2 * ax + 1) & 1) && !(place[n] >> (2 * ax) & 1))) ax++;
-        if (ax == 3 || (place[o] >> 6) != (place[n] >> 6) || low_face[(size_t)ax * nc + n] >= 0) return LBFS_OK;
-        if (ax != ((f < a.nfx) ? 0 : ((f < a.nfx + a.nfy) ? 1 : 2))) return LBFS_OK;
-        low_face[(size_t)ax * nc + n] = f;
+    first.push_back(f);
+    return f == f1;
+}
+
+// Side of its grid that a boundary face is on, by the outward normal's largest component.
+int boundary_side(const lbfs_mesh_desc *m, int f) {
+    const double *n = m->face_normal + 3 * (size_t)f;
+    int ax = 0;
+    for (int d = 1; d < 3; d++)
+        if (std::fabs(n[d]) > std::fabs(n[ax])) ax = d;
+    return 2 * ax + (n[ax] > 0 ? 1 : 0);
+}
+
+// Sides of its grid on which cell l = i + nx (j + ny k) has no neighbour.
+int missing_sides(const GridInst &g, int i, int j, int k) {
+    return (i == 0) | (i == g.nx - 1) << 1 | (j == 0) << 2 | (j == g.ny - 1) << 3 | (k == 0) << 4 | (k == g.nz - 1) << 5;
+}
+
+// The conditions of lbfs_fused.h on one instance.  The cells and faces are walked in the order that a
+// grid numbers them in, so that each entry is compared with the one expected (at 128^3 the tables and
+// searches of a check in any order took 200 ms).
+bool grid_fits(lbfs_solver *s, const lbfs_mesh_desc *m, const lbfs_grid_desc &gd, const GridMesh &gm, GridCheck &q) {
+    const int nc = s->nc, ni = s->ni;
+    GridInst &g = q.g;
+    if (!(gd.delta_x > 0)) return false;
+    long long n[3];
+    for (int d = 0; d < 3; d++) {
+        n[d] = std::llround(gd.length[d] / gd.delta_x);
+        if (n[d] < 2 || n[d] > gd.n_cells) return false;  // one cell thick: sides that face each other
     }
-    for (int ax = 0; ax < 3; ax++)
-        for (int c = 0; c < nc; c++)
-            if ((low_face[(size_t)ax * nc + c] < 0) != ((place[c] >> (2 * ax) & 1) != 0)) return LBFS_OK;
-    // the boundary face of every missing side, by the outward normal's largest component
-    std::vector<int> side_bc(nb, -1), side_of(nb);
-    std::vector<unsigned char> sides(nc, 0);
-    for (int b = 0; b < nb; b++) {
-        const int f = ni + b, o = m->owner[f];
-        const double *n = m->face_normal + 3 * (size_t)f;
-        int ax = 0;
-        for (int d = 1; d < 3; d++)
-            if (std::fabs(n[d]) > std::fabs(n[ax])) ax = d;
-        const int d = 2 * ax + (n[ax] > 0 ? 1 : 0);
-        if (!(place[o] >> d & 1)) return LBFS_OK;
-        const GridInst &q = inst[place[o] >> 6];
-        const int l = o - q.cell0, i = l % q.nx, j = (l / q.nx) % q.ny, k = l / (q.nx * q.ny);
-        int &slot = side_bc[q.side0[d] + (ax == 0 ? j + q.ny * k : (ax == 1 ? i + q.nx * k : i + q.nx * j))];
-        if (slot >= 0) return LBFS_OK;
-        slot = b;
-        side_of[b] = d;
-        sides[o] = 1;
+    if (n[0] * n[1] > gd.n_cells || n[0] * n[1] * n[2] != gd.n_cells) return false;
+    g.cell0 = gd.cell0; g.nx = (int)n[0]; g.ny = (int)n[1]; g.nz = (int)n[2];
+    const int dim[3] = {g.nx, g.ny, g.nz}, step[3] = {1, g.nx, g.nx * g.ny};
+    if (q.bnd[1] - q.bnd[0] != 2 * (n[1] * n[2] + n[0] * n[2] + n[0] * n[1])) return false;
+    // interior faces: each cell and its upper neighbour along the axis; one area and dt, dt from both centres
+    q.area = gm.axf[q.face[0][0]].area;
+    q.dt = gm.axf[q.face[0][0]].dt;
+    for (int ax = 0; ax < 3; ax++) {
+        if (q.face[ax][1] - q.face[ax][0] != (dim[ax] - 1) * (gd.n_cells / dim[ax])) return false;
+        const int end[3] = {dim[0] - (ax == 0), dim[1] - (ax == 1), dim[2] - (ax == 2)};
+        int f = q.face[ax][0];
+        for (int k = 0; k < end[2]; k++)
+            for (int j = 0; j < end[1]; j++) {
+                int c = g.cell0 + g.nx * (j + g.ny * k);
+                for (int i = 0; i < end[0]; i++, c++, f++) {
+                    const AxisFace<double> &x = gm.axf[f];
+                    if (m->owner[f] != c || m->neighbour[f] != c + step[ax] || x.area != q.area || x.dt != q.dt ||
+                        x.t1 != -q.dt || x.t2 != q.dt)
+                        return false;
+                }
+            }
     }
-    // the ghosts as the gradients take them (ghost_state)
-    std::vector<GridSide> side(nb), bnd_side(nb);
-    std::vector<GridBnd> bnd(nb);
-    std::vector<int> face_of(nc, -1);  // a boundary face of the cell
-    for (size_t e = 0; e < side.size(); e++) {
-        const int b = side_bc[e], rt = m->bc_rho_type[b], vt = m->bc_vel_type[b], ghost = nc + b;
-        const double *v = m->bc_values + 4 * (size_t)b;
-        const double gy = m->cell_centroid[3 * (size_t)ghost + 1], gz = m->cell_centroid[3 * (size_t)ghost + 2];
-        GridSide q{};
-        q.val = {v[0], v[1], v[2], v[3]};
-        if (vt == 9) q.val.u = 16 * q.val.u * (a.H2 + gy) * (a.H2 - gy) * (a.H2 + gz) * (a.H2 - gz) / a.H4;
-        else if (vt == 10) q.val.u = gy * q.val.u;
-        q.flags = (rt == 1 ? 1 : 0) | (vt == 1 || vt == 9 || vt == 10 ? 2 : 0) | (rt == 3 ? 4 : 0) | (vt == 3 ? 8 : 0) |
-                  (vt == 1 ? 16 : 0);
-        q.partner = rt == 3 || vt == 3 ? m->periodic_node[b] : 0;
-        side[e] = q;
-        if (q.flags) inst[place[m->owner[ni + b]] >> 6].active |= 1 << side_of[b];
-        bnd_side[b] = q;
-        // its cell's other missing sides
-        const int o = m->owner[ni + b], l = o - inst[place[o] >> 6].cell0;
-        const GridInst &g = inst[place[o] >> 6];
-        const int i = l % g.nx, j = (l / g.nx) % g.ny, k = l / (g.nx * g.ny);
-        GridBnd &r = bnd[b];
-        r = {o, g.nx, g.nx * g.ny, side_of[b], {0, 0}, 0, 0};
-        int others = 0;
-        for (int d = 0; d < 6; d++) {
-            if (d == side_of[b] || !(place[o] >> d & 1)) continue;
-            if (others == 2) return LBFS_OK;  // a grid one cell thick
-            r.info |= d << (3 + 3 * others);
-            r.more[others++] = side_bc[g.side0[d] + (d < 2 ? j + g.ny * k : (d < 4 ? i + g.nx * k : i + g.nx * j))];
-        }
-        for (; others < 2; others++) r.info |= 7 << (3 + 3 * others);
-        face_of[o] = b;
-    }
-    for (int b = 0; b < nb; b++) {
-        if (!(bnd_side[b].flags & 12)) continue;
-        bnd[b].partner = face_of[bnd_side[b].partner];
-        if (bnd[b].partner < 0) return LBFS_OK;
-    }
-    // every boundary face like the interior ones, its ghost straight across it
-    if (a.gamma_inv != 1.0 || a.recon_q != 1.0) return LBFS_OK;
-    for (int b = 0; b < nb; b++) {
-        const GenFace<double> &f = gen[b];
-        const BcRec<double> &r = bcr[b];
-        const int ax = side_of[b] / 2;
-        const double sn = (side_of[b] & 1) ? 1.0 : -1.0;
+    // boundary faces: one on every missing side, like the interior ones, the ghost straight across
+    std::vector<char> seen(gd.n_cells, 0);
+    q.dmag = gm.bcr[q.bnd[0]].dmag;
+    for (int b = q.bnd[0]; b < q.bnd[1]; b++) {
+        const int o = m->owner[ni + b], l = o - g.cell0, d = boundary_side(m, ni + b), ax = d / 2;
+        if (!(missing_sides(g, l % g.nx, (l / g.nx) % g.ny, l / step[2]) >> d & 1) || (seen[l] >> d & 1)) return false;
+        seen[l] |= (char)(1 << d);
+        const GenFace<double> &f = gm.gen[b];
+        const BcRec<double> &r = gm.bcr[b];
+        const double sn = (d & 1) ? 1.0 : -1.0;
         const double nv[3] = {f.nx, f.ny, f.nz}, t1[3] = {f.t1x, f.t1y, f.t1z}, t2[3] = {f.t2x, f.t2y, f.t2z};
         const double dn[3] = {r.dnx, r.dny, r.dnz}, mv[3] = {r.mx, r.my, r.mz};
-        if (f.area != axf[0].area || f.dt != axf[0].dt || r.dmag != bcr[0].dmag) return LBFS_OK;
-        for (int q = 0; q < 3; q++) {
-            const double e = q == ax ? sn : 0.0;
-            if (nv[q] != e || dn[q] != e || t1[q] != -f.dt * e || t2[q] != f.dt * e || mv[q] != (q == ax ? 0.0 : 1.0))
-                return LBFS_OK;
+        if (f.area != q.area || f.dt != q.dt || r.dmag != q.dmag) return false;
+        for (int e = 0; e < 3; e++) {
+            const double x = e == ax ? sn : 0.0;
+            if (nv[e] != x || dn[e] != x || t1[e] != -f.dt * x || t2[e] != f.dt * x || mv[e] != (e == ax ? 0.0 : 1.0))
+                return false;
         }
-        if (f.bc_branch == 0.0) bnd[b].info |= 1024;
+        if (m->bc_rho_type[b] == 3 || m->bc_vel_type[b] == 3) {
+            const int p = m->periodic_node[b] - g.cell0;  // a boundary cell of this grid
+            if (p < 0 || p >= gd.n_cells || !missing_sides(g, p % g.nx, (p / g.nx) % g.ny, p / step[2])) return false;
+        }
     }
-    // every gradient stencil is the six neighbours, weighted along their axes alone by one magnitude
-    // (ref: a lower neighbour's weight)
-    double ref = 0.0;
-    for (int c = 0; c < nc; c++) {
-        int seen = 0;
-        for (int q = 0; q < 6; q++) {
-            const int j = m->gradient_stencil[6 * (size_t)c + q];
-            int d = 0;
-            if (j >= nc) {
-                if (m->owner[ni + j - nc] != c) return LBFS_OK;
-                d = side_of[j - nc];
-            } else {
-                while (d < 6 && !(!(place[c] >> d & 1) && j - c == ((d & 1) ? stride(c, d / 2) : -stride(c, d / 2)))) d++;
+    // gradient stencils: the six neighbours, weighted along their axes alone by one magnitude (weight: a lower
+    // neighbour's)
+    int c = g.cell0;
+    for (int k = 0; k < g.nz; k++)
+        for (int j = 0; j < g.ny; j++)
+            for (int i = 0; i < g.nx; i++, c++) {
+                const int miss = missing_sides(g, i, j, k);
+                const int *st = m->gradient_stencil + 6 * (size_t)c;
+                int have = 0;
+                for (int e = 0; e < 6; e++) {
+                    int d;
+                    if (st[e] >= nc) {
+                        const int b = st[e] - nc;
+                        if (m->owner[ni + b] != c) return false;
+                        d = boundary_side(m, ni + b);
+                    } else {
+                        const int x = st[e] - c, y = x < 0 ? -x : x;
+                        d = (y == 1 ? 0 : (y == step[1] ? 2 : (y == step[2] ? 4 : 6))) + (x > 0 ? 1 : 0);
+                        if (d > 5 || (miss >> d & 1)) return false;
+                    }
+                    if (have >> d & 1) return false;
+                    have |= 1 << d;
+                    const double *v = gm.lsw[c].w + 3 * e;
+                    if (c == g.cell0 && e == 0) q.weight = (d & 1) ? -v[d / 2] : v[d / 2];
+                    if (gm.code) {  // the weight vectors' table instead of 144 B a cell
+                        const GridMesh::Code &t = gm.tab[gm.code[c] >> (3 * e) & 7u];
+                        if (t.axis != d / 2 || t.value != ((d & 1) ? -q.weight : q.weight)) return false;
+                    } else {
+                        for (int r = 0; r < 3; r++)
+                            if (v[r] != (r == d / 2 ? ((d & 1) ? -q.weight : q.weight) : 0.0)) return false;
+                    }
+                }
             }
-            if (d == 6 || (seen >> d & 1)) return LBFS_OK;
-            seen |= 1 << d;
-            const double *v = lsw[c].w + 3 * q;
-            if (c == 0 && q == 0) ref = (d & 1) ? -v[d / 2] : v[d / 2];
-            for (int r = 0; r < 3; r++)
-                if (v[r] != (r == d / 2 ? ((d & 1) ? -ref : ref) : 0.0)) return LBFS_OK;
-        }
+    q.fits = true;
+    return true;
+}
+
+// The fused step's plan: which instances take the pass (each by itself, so that an instance of an
+// ensemble steps as it does in a handle of its own), one launch per set of face constants, the ghosts,
+// and the tiles.  Instances that do not keep the separate kernels.  Leaves s->fused false where none
+// does (LBFS_SEPARATE_KERNELS set: always; a diagnostic switch).
+int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
+    FluidArgs<double> &a = s->f64;
+    s->fused = false;
+    if (!a.axis_aligned || a.ni == 0 || std::getenv("LBFS_SEPARATE_KERNELS")) return LBFS_OK;
+    if (a.gamma_inv != 1.0 || a.recon_q != 1.0) return LBFS_OK;
+    const int nc = a.nc, ni = a.ni, nb = a.nb, n_inst = (int)s->grids.size();
+    const int start[4] = {0, a.nfx, a.nfx + a.nfy, ni};
+    std::vector<int> first[4];
+    for (int ax = 0; ax < 3; ax++)
+        if (!faces_by_instance(s, m->owner, start[ax], start[ax + 1], first[ax])) return LBFS_OK;
+    if (!faces_by_instance(s, m->owner, ni, ni + nb, first[3])) return LBFS_OK;
+    std::vector<GridCheck> check(n_inst);
+    int fits = 0;
+    for (int k = 0; k < n_inst; k++) {
+        GridCheck &q = check[k];
+        for (int ax = 0; ax < 3; ax++)
+            for (int e = 0; e < 2; e++) q.face[ax][e] = first[ax][k + e];
+        for (int e = 0; e < 2; e++) q.bnd[e] = first[3][k + e] - ni;
+        fits += grid_fits(s, m, s->grids[k], gm, q);
     }
-    // every interior face has one area and dt and lies dt from both centres
-    ga.area = axf[0].area;
-    ga.dt = axf[0].dt;
-    for (int f = 0; f < ni; f++)
-        if (axf[f].area != ga.area || axf[f].dt != ga.dt || axf[f].t1 != -ga.dt || axf[f].t2 != ga.dt) return LBFS_OK;
-    const double c = -ref * ga.dt;
-    ga.cw = {c, 3.0 * c, 3.0 * c * c, 0.5 * c, 1.5 * c, 0.75 * c * c};
-    ga.bnd_k = nb > 0 ? ga.dt / (bcr[0].dmag * c) : 0.0;
-    int rc;
+    if (fits == 0) return LBFS_OK;
+    // the instances that keep the separate kernels must not read beyond themselves: the others leave no gradients
+    s->rest = lbfs_solver::Rest{};
+    for (int k = 0; k < n_inst; k++) {
+        const GridCheck &q = check[k];
+        if (q.fits) continue;
+        const int c0 = s->grids[k].cell0, c1 = c0 + s->grids[k].n_cells;
+        auto inside = [&](int j) { return j < nc ? j >= c0 && j < c1 : j - nc >= q.bnd[0] && j - nc < q.bnd[1]; };
+        for (int ax = 0; ax < 3; ax++)
+            for (int f = q.face[ax][0]; f < q.face[ax][1]; f++)
+                if (!inside(m->neighbour[f])) return LBFS_OK;
+        for (size_t e = 6 * (size_t)c0; e < 6 * (size_t)c1; e++)
+            if (!inside(m->gradient_stencil[e])) return LBFS_OK;
+        for (int b = q.bnd[0]; b < q.bnd[1]; b++)
+            if ((m->bc_rho_type[b] == 3 || m->bc_vel_type[b] == 3) && !inside(m->periodic_node[b])) return LBFS_OK;
+        lbfs_solver::Rest &r = s->rest;  // their cells and faces, with those of the instances between them
+        if (!r.any) {
+            r.any = true;
+            r.cell0 = c0;
+            for (int ax = 0; ax < 3; ax++) r.faces.start[ax] = q.face[ax][0];
+        }
+        r.cell1 = c1;
+        for (int ax = 0; ax < 3; ax++) r.faces.count[ax] = q.face[ax][1] - r.faces.start[ax];
+    }
+    // one launch per set of face constants
+    std::vector<std::vector<int>> sets;
+    for (int k = 0; k < n_inst; k++) {
+        if (!check[k].fits) continue;
+        size_t e = 0;
+        auto same = [&](const GridCheck &x, const GridCheck &y) {
+            return x.area == y.area && x.dt == y.dt && x.weight == y.weight && x.dmag == y.dmag;
+        };
+        while (e < sets.size() && !same(check[sets[e][0]], check[k])) e++;
+        if (e == sets.size()) sets.emplace_back();
+        sets[e].push_back(k);
+    }
+    // the boundary faces in the order of the launches: place[b] their place in it
+    std::vector<int> place(nb, -1);
+    int placed = 0, sided = 0;
+    for (const std::vector<int> &set : sets)
+        for (int k : set) {
+            GridInst &g = check[k].g;
+            const int area[3] = {g.ny * g.nz, g.nx * g.nz, g.nx * g.ny};
+            for (int d = 0; d < 6; d++) {
+                g.side0[d] = sided;
+                sided += area[d / 2];
+            }
+            for (int b = check[k].bnd[0]; b < check[k].bnd[1]; b++) place[b] = placed++;
+        }
+    // the ghosts as the gradients take them (ghost_state), by side and in the launches' order
+    std::vector<GridSide> side(sided), bnd_side(placed);
+    std::vector<GridBnd> bnd(placed);
+    std::vector<int> side_bc(sided, -1), face_of(nc, -1);  // boundary face of a side's place; one of a cell's
+    std::vector<unsigned char> sides(nc, (unsigned char)(s->rest.any ? kSeparateCell : 0));
+    for (int pass = 0; pass < 2; pass++)
+        for (GridCheck &q : check) {
+            if (!q.fits) continue;
+            GridInst &g = q.g;
+            auto at = [&](int d, int i, int j, int k) {
+                return g.side0[d] + (d < 2 ? j + g.ny * k : (d < 4 ? i + g.nx * k : i + g.nx * j));
+            };
+            if (pass == 0) std::fill_n(sides.begin() + g.cell0, (size_t)g.nx * g.ny * g.nz, (unsigned char)0);
+            for (int b = q.bnd[0]; b < q.bnd[1]; b++) {
+                const int o = m->owner[ni + b], l = o - g.cell0, i = l % g.nx, j = (l / g.nx) % g.ny, k = l / (g.nx * g.ny);
+                const int own_side = boundary_side(m, ni + b);
+                if (pass == 0) {
+                    side_bc[at(own_side, i, j, k)] = b;
+                    face_of[o] = b;
+                    continue;
+                }
+                const int rt = m->bc_rho_type[b], vt = m->bc_vel_type[b], ghost = nc + b;
+                const double *v = m->bc_values + 4 * (size_t)b;
+                const double gy = m->cell_centroid[3 * (size_t)ghost + 1], gz = m->cell_centroid[3 * (size_t)ghost + 2];
+                GridSide e{};
+                e.val = {v[0], v[1], v[2], v[3]};
+                if (vt == 9) e.val.u = 16 * e.val.u * (a.H2 + gy) * (a.H2 - gy) * (a.H2 + gz) * (a.H2 - gz) / a.H4;
+                else if (vt == 10) e.val.u = gy * e.val.u;
+                e.flags = (rt == 1 ? 1 : 0) | (vt == 1 || vt == 9 || vt == 10 ? 2 : 0) | (rt == 3 ? 4 : 0) |
+                          (vt == 3 ? 8 : 0) | (vt == 1 ? 16 : 0);
+                const bool periodic = rt == 3 || vt == 3;
+                e.partner = periodic ? m->periodic_node[b] : 0;
+                if (e.flags) g.active |= 1 << own_side;
+                side[at(own_side, i, j, k)] = bnd_side[place[b]] = e;
+                sides[o] = 1;
+                GridBnd &r = bnd[place[b]];
+                r = {o, g.nx, g.nx * g.ny, own_side, {0, 0}, periodic ? place[face_of[e.partner]] : 0, b};
+                const int miss = missing_sides(g, i, j, k);
+                int others = 0;  // its cell's other missing sides
+                for (int d = 0; d < 6; d++) {
+                    if (d == own_side || !(miss >> d & 1)) continue;
+                    r.info |= d << (3 + 3 * others);
+                    r.more[others++] = place[side_bc[at(d, i, j, k)]];
+                }
+                for (; others < 2; others++) r.info |= 7 << (3 + 3 * others);
+                if (gm.gen[b].bc_branch == 0.0) r.info |= 1024;
+            }
+        }
     // the tiles, with one walk length d for all instances.  A block's time is d planes and a start of 1.2
     // (clock stamps inside the kernel), a plane's about 3000 cycles and 1300 for each
     // block on its SM.  Grids of at most one wave: the longest block at that occupancy; larger ones: the
     // blocks' throughput and a third of a block for the last wave.  64^3 FP64: 45 us at the chosen d = 4,
     // 47 at 3, 54 at 8; 128^3: 203 at 8, 206 at 4, 213 at 16.
-    std::vector<TileShape> shape;
-    for (const GridInst &q : inst) {
-        const TileShape t = tile_shape(q.nx, q.ny);
-        if (t.w == 0) return LBFS_OK;
-        shape.push_back(t);
-    }
+    std::vector<TileShape> shape(n_inst);
+    for (int k = 0; k < n_inst; k++)
+        if (check[k].fits) shape[k] = tile_shape(check[k].g.nx, check[k].g.ny);
     const int per_sm = kUniformBlocks;
     auto plane_time = [](int blocks) { return 3000.0 + 1300.0 * blocks; };
     int depth = 1;
     double best = 1e300;
     for (int d = 1; d <= 64; d++) {
         double planes = 0.0, longest = 0.0, blocks = 0.0;
-        for (size_t q = 0; q < inst.size(); q++) {
-            const int walks = (inst[q].nz + d - 1) / d, even = (inst[q].nz + walks - 1) / walks;
-            const double n = (double)((inst[q].nx + shape[q].w - 1) / shape[q].w) * ((inst[q].ny + shape[q].h - 1) / shape[q].h) * walks;
+        for (int k = 0; k < n_inst; k++) {
+            if (!check[k].fits) continue;
+            const GridInst &g = check[k].g;
+            const int walks = (g.nz + d - 1) / d, even = (g.nz + walks - 1) / walks;
+            const double n = (double)((g.nx + shape[k].w - 1) / shape[k].w) * ((g.ny + shape[k].h - 1) / shape[k].h) * walks;
             blocks += n;
             planes += n * (even + 1.2);
             longest = std::max(longest, even + 1.2);
@@ -734,61 +850,86 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const std::vector<LsW<dou
             depth = d;
         }
     }
-    std::vector<GridTile> tiles;
-    int P = 0, G = 0;
-    for (size_t q = 0; q < inst.size(); q++) {
-        const GridInst &g = inst[q];
-        const int w0 = shape[q].w, h0 = shape[q].h, walks = (g.nz + depth - 1) / depth, dz = (g.nz + walks - 1) / walks;
-        for (int z = 0; z < g.nz; z += dz)
-            for (int y = 0; y < g.ny; y += h0)
-                for (int x = 0; x < g.nx; x += w0) {
-                    const GridTile t = {x, y, z, std::min(w0, g.nx - x), std::min(h0, g.ny - y), std::min(dz, g.nz - z), (int)q, 0};
-                    tiles.push_back(t);
-                    for (int k = t.z0; k < t.z0 + t.d; k++)  // upper faces that other tiles form
-                        for (int j = t.y0; j < t.y0 + t.h; j++)
-                            for (int i = t.x0; i < t.x0 + t.w; i++) {
-                                const int e = (i == t.x0 + t.w - 1 && i < g.nx - 1) << 1 |
-                                              (j == t.y0 + t.h - 1 && j < g.ny - 1) << 2 |
-                                              (k == t.z0 + t.d - 1 && k < g.nz - 1) << 3;
-                                if (e) sides[g.cell0 + i + g.nx * (j + g.ny * k)] |= (unsigned char)e;
-                            }
-                    P = std::max(P, (t.w + 3) * (t.h + 3));
-                    G = std::max(G, 2 * (t.w + t.h + 4));
-                }
+    // what the launches share
+    int rc;
+    GridArgs all{};
+    std::vector<GridInst> inst(n_inst);
+    std::vector<GridCells> cells(n_inst);
+    for (int k = 0; k < n_inst; k++) {
+        inst[k] = check[k].g;
+        cells[k] = {check[k].g.nx, check[k].g.nx * check[k].g.ny, check[k].area};
     }
-    GridTile *d_tiles;
     GridInst *d_inst;
-    GridSide *d_side;
+    GridSide *d_side, *d_bside;
     GridBnd *d_bnd;
-    GridSide *d_bside;
-    unsigned char *d_sides;
-    double4 *d_res;
-    Vec4<double> *d_prev;
-    if ((rc = s->upload(&d_tiles, tiles)) || (rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) ||
-        (rc = s->upload(&d_bnd, bnd)) || (rc = s->upload(&d_bside, bnd_side)) ||
-        (rc = s->upload(&d_sides, sides)) || (rc = s->alloc(&d_res, nc)) || (rc = s->alloc(&d_prev, (size_t)nc + nb)))
+    if ((rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) || (rc = s->upload(&d_bnd, bnd)) ||
+        (rc = s->upload(&d_bside, bnd_side)) || (rc = s->alloc(&all.res, nc)) ||
+        (rc = s->alloc(&all.prev, (size_t)nc + nb)) || (rc = s->alloc(&all.edge, 3 * (size_t)nc)))
         return rc;
-    if ((rc = s->alloc(&ga.edge, 3 * (size_t)nc))) return rc;
-    a.grid_edge = ga.edge;
-    a.grid_area = (double)ga.area;
-    a.grid_stride[0] = inst.size() == 1 ? inst[0].nx : 0;
-    a.grid_stride[1] = inst.size() == 1 ? inst[0].nx * inst[0].ny : 0;
-    if (inst.size() > 1) {
-        std::vector<int2> st;
+    all.inst = d_inst; all.side = d_side; all.bnd = d_bnd; all.bnd_side = d_bside;
+    s->passes.clear();
+    int faces = 0;
+    for (const std::vector<int> &set : sets) {
+        GridArgs ga = all;
+        const GridCheck &one = check[set[0]];
+        ga.area = one.area;
+        ga.dt = one.dt;
+        const double c = -one.weight * one.dt;
+        ga.cw = {c, 3.0 * c, 3.0 * c * c, 0.5 * c, 1.5 * c, 0.75 * c * c};
+        ga.bnd_k = one.dt / (one.dmag * c);
+        std::vector<GridTile> tiles;
+        ga.bnd0 = faces;
+        for (int q : set) {
+            const GridInst &g = check[q].g;
+            const int walks = (g.nz + depth - 1) / depth, dz = (g.nz + walks - 1) / walks;
+            for (int z = 0; z < g.nz; z += dz)
+                for (int y = 0; y < g.ny; y += shape[q].h)
+                    for (int x = 0; x < g.nx; x += shape[q].w) {
+                        const GridTile t = {x, y, z, std::min(shape[q].w, g.nx - x), std::min(shape[q].h, g.ny - y),
+                                            std::min(dz, g.nz - z), q, 0};
+                        tiles.push_back(t);
+                        // upper faces that other tiles form
+                        const int i1 = t.x0 + t.w - 1, j1 = t.y0 + t.h - 1, k1 = t.z0 + t.d - 1;
+                        auto mark = [&](int i0, int j0, int k0, int bit) {
+                            for (int k = k0; k <= k1; k++)
+                                for (int j = j0; j <= j1; j++)
+                                    for (int i = i0; i <= i1; i++)
+                                        sides[g.cell0 + i + g.nx * (j + g.ny * k)] |= (unsigned char)(1 << bit);
+                        };
+                        if (i1 < g.nx - 1) mark(i1, t.y0, t.z0, 1);
+                        if (j1 < g.ny - 1) mark(t.x0, j1, t.z0, 2);
+                        if (k1 < g.nz - 1) mark(t.x0, t.y0, k1, 3);
+                        ga.plane_stride = std::max(ga.plane_stride, (t.w + 3) * (t.h + 3));
+                        ga.stage_max = std::max(ga.stage_max, 2 * (t.w + t.h + 4));
+                    }
+            faces += check[q].bnd[1] - check[q].bnd[0];
+        }
+        ga.bnd1 = faces;
+        ga.bnd_blocks = (ga.bnd1 - ga.bnd0 + kUniformThreads - 1) / kUniformThreads;
+        ga.n_tiles = (int)tiles.size();
+        GridTile *d_tiles;
+        if ((rc = s->upload(&d_tiles, tiles))) return rc;
+        ga.tiles = d_tiles;
+        s->passes.push_back(ga);
+    }
+    unsigned char *d_sides;
+    if ((rc = s->upload(&d_sides, sides))) return rc;
+    s->grid_sides = d_sides;
+    a.grid_edge = all.edge;
+    const bool one_grid = n_inst == 1, one_kind = sets.size() == 1 && !s->rest.any;
+    a.grid_mixed = !one_kind;
+    a.grid_area = check[sets[0][0]].area;
+    a.grid_stride[0] = one_grid ? inst[0].nx : 0;
+    a.grid_stride[1] = one_grid ? inst[0].nx * inst[0].ny : 0;
+    if (!one_grid) {
         std::vector<int> which(nc);
-        for (const GridInst &q : inst) st.push_back(make_int2(q.nx, q.nx * q.ny));
-        for (int i = 0; i < nc; i++) which[i] = place[i] >> 6;
-        int2 *d_st;
+        for (int k = 0; k < n_inst; k++) std::fill_n(which.begin() + s->grids[k].cell0, s->grids[k].n_cells, k);
+        GridCells *d_cells;
         int *d_which;
-        if ((rc = s->upload(&d_st, st)) || (rc = s->upload(&d_which, which))) return rc;
-        a.grid_strides = d_st;
+        if ((rc = s->upload(&d_cells, cells)) || (rc = s->upload(&d_which, which))) return rc;
+        a.grid_cells = d_cells;
         a.grid_instance = d_which;
     }
-    ga.tiles = d_tiles; ga.inst = d_inst; ga.side = d_side; ga.bnd = d_bnd; ga.bnd_side = d_bside; ga.sides = d_sides; ga.res = d_res; ga.prev = d_prev;
-    ga.n_tiles = (int)tiles.size();
-    ga.bnd_blocks = (nb + kUniformThreads - 1) / kUniformThreads;
-    ga.plane_stride = P;
-    ga.stage_max = G;
     if (grid_prepare() != cudaSuccess) {
         cudaGetLastError();
         return LBFS_OK;
@@ -1214,7 +1355,7 @@ void set_chunks(lbfs_solver *s, int K) {
     const std::vector<int> &mx = s->tile_maxnb[tb == 64 ? 0 : (tb == 256 ? 2 : 1)];
     // fused step: fluid pass and update; else gradients and interior fluxes (K each), boundary fluxes,
     // update; membrane kernels; CFL
-    s->launches_per_step = (s->fused ? 2 : 2 * K + 2) + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
+    s->launches_per_step = (s->fused ? (int)s->passes.size() + 1 + (s->rest.any ? 3 : 0) : 2 * K + 2) + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
     s->chunk_cell.assign(K + 1, 0);
     s->chunk_faces.assign(K, FaceRanges{});
     for (int c = 0; c <= K; c++) s->chunk_cell[c] = (int)((long long)s->nc * c / K);
@@ -1405,10 +1546,9 @@ int fork_behind_launch(lbfs_solver *s) {
 // register of an SM until they end, the chain came late (us per step, behind /
 // beside: 44.6 / 36.5 on 48^3 with 162 nodes, 64.8 / 55.5 at 64^3 with 642).
 int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
-    const GridArgs &ga = s->grid;
     FluidArgs<double> a = s->f64;
-    a.grid_res = ga.res;
-    a.grid_sides = ga.sides;
+    a.grid_res = s->passes[0].res;
+    a.grid_sides = s->grid_sides;
     int n = 0;
     for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = false;
     if (s->profiling) LBFS_CUDA(record_event(s->ev_phase[5][0], s->stream));
@@ -1416,18 +1556,31 @@ int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
         launch_fluid_cfl<double>(a, s->stream);
         n += 1;
     }
-    auto pass = [&]() {
+    auto pass = [&]() -> int {
         PhaseMark m(s, 2, s->stream);
-        launch_grid_step(a, ga, s->stream);
-        n += 1;
+        if (s->rest.any) {  // the instances between take part, before the pass writes their fluxes and its copy of the state
+            const size_t c0 = (size_t)s->rest.cell0, count = (size_t)(s->rest.cell1 - s->rest.cell0);
+            launch_fluid_gradients_range<double>(a, s->rest.cell0, s->rest.cell1, s->stream);
+            launch_fluid_flux_axis_ranges<double>(a, s->rest.faces, s->stream);
+            launch_fluid_flux_general<double>(a, s->stream);
+            LBFS_CUDA(cudaMemcpyAsync(s->passes[0].prev + c0, a.state + c0, sizeof(Vec4<double>) * count,
+                                      cudaMemcpyDeviceToDevice, s->stream));
+            n += 3;
+        }
+        for (const GridArgs &ga : s->passes) {
+            launch_grid_step(a, ga, s->stream);
+            n += 1;
+        }
+        return LBFS_OK;
     };
+    int rc = LBFS_OK;
     if (s->n_membranes == 0) {
-        pass();
+        rc = pass();
     } else if (visc_update) {
         { PhaseMark m(s, 0, s->stream); n += launch_membrane(s->ma, s->stream); }
         { PhaseMark m(s, 4, s->stream); launch_interior_viscosity(s->va, s->stream); }
-        n += 2;
-        pass();
+        n += 1;
+        rc = pass();
     } else {
         cudaGraphNode_t advect = nullptr;
         LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
@@ -1437,10 +1590,11 @@ int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
             n += launch_membrane(s->ma, s->stream2, s->stream3, s->ev_advected, s->ev_sorted, false, &advect);
         }
         LBFS_CUDA(cudaEventRecord(s->ev_join, s->stream2));
-        if (int rc = order_behind_advect(s, advect)) return rc;
-        pass();
+        if ((rc = order_behind_advect(s, advect))) return rc;
+        rc = pass();
         LBFS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_join, 0));
     }
+    if (rc) return rc;
     { PhaseMark m(s, 3, s->stream); launch_fluid_update<double>(a, s->stream, !s->kernel_events); }
     n += 1;
     if (s->profiling) {
@@ -1529,7 +1683,7 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
 int ensure_fields(lbfs_solver *s) {
     if (!s->fields_stale) return LBFS_OK;
     FluidArgs<double> a = s->f64;
-    a.state = s->grid.prev;
+    a.state = s->passes[0].prev;
     launch_fluid_gradients<double>(a, s->stream);
     launch_fluid_flux<double>(a, s->stream);
     LBFS_CUDA(cudaGetLastError());

@@ -10,7 +10,7 @@ area and volume is no power of two, so that another place of the scaling shows i
 import numpy as np
 import pytest
 
-from lbfs_b200 import GpuSolver, StepParams, build_uniform_mesh
+from lbfs_b200 import GpuSolver, StepParams, _abi, build_uniform_mesh
 from lbfs_b200.ensemble import concatenate
 from lbfs_b200.slabs import SlabSolver, build_slab_mesh, slab_bounds, step_local
 
@@ -74,3 +74,41 @@ def test_slabs_equal_the_whole_mesh(spacing):
         for a, b in zip(s.owned_state(), want):
             assert np.array_equal(a, b[z0 * n * n:z1 * n * n])
         s.solver.close()
+
+
+def _plateau(n):
+    m = build_uniform_mesh(*(2.0 * k for k in n), 1.0, visc=PARAMS.visc, mesh_type=4, plateau_width=5.0, plateau_slope=0.3)
+    m.set_boundaries(BCS)
+    return m
+
+
+@pytest.mark.parametrize("kinds", ["2 1.5", "1.5 2 1", "p 2", "2 p 1.5 p", "p 1.5 p"])
+def test_instances_of_different_meshes_equal_handles_of_their_own(kinds):
+    """Grids of different spacings and rectilinear ones (p) in one handle: each instance takes the kernels,
+    and the constants, that it takes alone; the gradient, flux and ghost fields too."""
+    meshes = [_plateau((14 + k, 12, 10)) if s == "p" else _box((13, 17 + k, 12), float(s)) for k, s in enumerate(kinds.split())]
+    states = [_state(m.n_cells, 20 + k) for k, m in enumerate(meshes)]
+    e = concatenate(meshes)
+
+    def run(mesh, state):
+        with GpuSolver(mesh, PARAMS) as s:
+            s.set_state(*state)
+            s.step(3, graph=True)
+            s.step(2)
+            s.keep_residuals(True)
+            s.step(1)
+            assert s.status() == 0
+            return s.state(), s.field(_abi.LBFS_FIELD_RESIDUAL).reshape(-1, 4), \
+                s.field(_abi.LBFS_FIELD_GRADIENTS).reshape(-1, 12), s.field(_abi.LBFS_FIELD_GHOST).reshape(-1, 4)
+
+    state, res, grad, ghost = run(e, [np.concatenate(q) for q in zip(*states)])
+    b0 = 0
+    for k, (m, st) in enumerate(zip(meshes, states)):
+        own = run(m, st)
+        for a, b in zip(state, own[0]):
+            assert np.array_equal(e.split(a)[k], b), k
+        assert np.array_equal(e.split(res)[k], own[1]), k
+        assert np.array_equal(e.split(grad)[k], own[2][:m.n_cells]), k
+        assert np.array_equal(ghost[b0:b0 + m.n_bc], own[3]), k
+        assert np.array_equal(grad[e.n_cells + b0:e.n_cells + b0 + m.n_bc], own[2][m.n_cells:]), k
+        b0 += m.n_bc
