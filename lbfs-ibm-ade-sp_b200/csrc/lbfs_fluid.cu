@@ -360,10 +360,12 @@ __global__ void __launch_bounds__(TB) k_cell_update(FluidArgs<R> a) {
 #pragma unroll
             for (int w = 0; w < TB / 32; w++) v += sh[lane][w];
             a.partials[4 * blockIdx.x + lane] = v;
-            __threadfence();
         }
         __syncwarp();
-        if (lane == 0) last_block = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+        if (lane == 0) {  // the fence behind the barrier: it orders all four lanes' sums (and the flags) before the ticket
+            __threadfence();
+            last_block = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+        }
     }
     __syncthreads();
     if (last_block) {
