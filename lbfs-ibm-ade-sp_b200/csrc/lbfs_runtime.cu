@@ -61,8 +61,8 @@ struct lbfs_solver {
     // constants, when `fused`, and the instances that keep the separate kernels (rest).
     // separate: steps take the separate kernels all the same (the adjoint's recording, which reads
     // every step's gradients).  fields_stale: the last step left no gradients, fluxes or ghosts; they
-    // are formed from the state it started from when asked for.
-    bool fused = false, separate = false, fields_stale = false;
+    // are formed from the state it started from (prev, where prev_last) when asked for.
+    bool fused = false, separate = false, fields_stale = false, prev_last = false;
     std::vector<GridArgs> passes;
     const unsigned char *grid_sides = nullptr;
     struct Rest {
@@ -1693,7 +1693,7 @@ int ensure_fields(lbfs_solver *s) {
     return LBFS_OK;
 }
 // after one or more steps
-void note_steps(lbfs_solver *s) { s->fields_stale = s->fused && !s->separate; }
+void note_steps(lbfs_solver *s) { s->fields_stale = s->prev_last = s->fused && !s->separate; }
 
 int enqueue(lbfs_solver *s, bool visc_update, int *launches) {
     return s->fp32 ? enqueue_step<float>(s, visc_update, launches) : enqueue_step<double>(s, visc_update, launches);
@@ -1951,6 +1951,15 @@ int build_step_graph(lbfs_solver *s, int steps, cudaGraphExec_t *graph) {
 constexpr int kRunSteps = 16;
 constexpr long long kRunAfter = 256;
 
+int make_step_run(lbfs_solver *s, int steps) {
+    cudaGraphExec_t g = nullptr;
+    if (int rc = build_step_graph(s, steps, &g)) return rc;
+    if (s->run.graph) cudaGraphExecDestroy(s->run.graph);
+    s->run.graph = g;
+    s->run.steps = steps;
+    return LBFS_OK;
+}
+
 void plan_step_run(lbfs_solver *s, int n_steps) {
     lbfs_solver::StepRun *r = &s->run;
     const int asked = std::min(n_steps, kRunSteps);
@@ -1961,15 +1970,10 @@ void plan_step_run(lbfs_solver *s, int n_steps) {
     if (asked < 2 || asked == r->steps || r->failed || s->profiling || (r->taken += n_steps) <= kRunAfter) return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;  // the caller may be capturing this call
     if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return;
-    cudaGraphExec_t g = nullptr;
-    if (build_step_graph(s, asked, &g) != LBFS_OK) {  // one step at a time as before
+    if (make_step_run(s, asked) != LBFS_OK) {  // one step at a time as before
         cudaGetLastError();
         r->failed = true;
-        return;
     }
-    if (r->graph) cudaGraphExecDestroy(r->graph);
-    r->graph = g;
-    r->steps = asked;
 }
 }  // namespace
 
@@ -3167,12 +3171,13 @@ namespace {
 // steps (graph replays, CUDA events on the handle's stream) from the same
 // saved state: the kernels run with the contention of a real step (the
 // membrane chain beside the fluid kernels), which isolated kernel timings
-// miss.  The state (the checkpoint parts, the counter and the status word)
-// is put back afterwards.
+// miss.  Steps go several to a graph, as long runs take them, made before the
+// timed region.  The state (the checkpoint parts, the counter and the status
+// word) is put back afterwards, and what the fused step's fields are formed from.
 int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) {
-    if (int r = ensure_fields(s)) return r;  // of the caller's last step
     LBFS_CUDA(cudaStreamSynchronize(s->stream));
-    const std::vector<CkPart> parts = ck_parts(s);
+    std::vector<CkPart> parts = ck_parts(s);
+    if (s->prev_last) parts.push_back({s->passes[0].prev, sizeof(Vec4<double>) * (size_t)s->nc});
     size_t total = 0;
     for (const CkPart &p : parts) total += p.bytes;
     DevBuf snap;
@@ -3201,6 +3206,7 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
         s->t = t0;
         drop_graph(s);
         if ((r = lbfs_step_graph(s, 2))) return r;  // capture + warm
+        if (reps > 1 && !s->profiling && (r = make_step_run(s, std::min(reps, kRunSteps)))) return r;
         LBFS_CUDA(cudaEventRecord(e0, s->stream));
         if ((r = lbfs_step_graph(s, reps))) return r;
         LBFS_CUDA(cudaEventRecord(e1, s->stream));
@@ -3219,15 +3225,17 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
         std::vector<int> values;
     };
     const bool membranes = s->n_membranes > 0;
+    const bool separate = !s->fused || s->rest.any;  // the separate kernels run: the knobs of theirs that have an effect
+    auto theirs = [&](std::vector<int> values) { return separate ? values : std::vector<int>{}; };
     const std::vector<Knob> knobs = {
-        {&lbfs_launch_shape::gradient_threads, {128, 256, 512}},
-        {&lbfs_launch_shape::flux_threads, {64, 128, 256}},
-        {&lbfs_launch_shape::general_flux_threads, {64, 128, 256}},
+        {&lbfs_launch_shape::gradient_threads, theirs({128, 256, 512})},
+        {&lbfs_launch_shape::flux_threads, theirs({64, 128, 256})},
+        {&lbfs_launch_shape::general_flux_threads, theirs({64, 128, 256})},
         {&lbfs_launch_shape::update_threads, {128, 256, 512}},
         {&lbfs_launch_shape::update_blocks, {148 * 2, 148 * 4, 148 * 8, 148 * 16}},
         {&lbfs_launch_shape::spread_blocks,
          membranes ? std::vector<int>{148, 296, 592, 1184, 2368} : std::vector<int>{}},
-        {&lbfs_launch_shape::flux_chunks, s->chunkable ? std::vector<int>{1, 2, 4, 8} : std::vector<int>{}},
+        {&lbfs_launch_shape::flux_chunks, s->chunkable && !s->fused ? std::vector<int>{1, 2, 4, 8} : std::vector<int>{}},
     };
     lbfs_launch_shape cur = fp32 ? args_to_shape<float>(s) : args_to_shape<double>(s);
     double best = 0;
@@ -3256,6 +3264,7 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
         const lbfs_launch_shape base = cur;
         for (int cl : clusters) {
             for (int after = 0; !rc && after < 2; after++) {
+                if (s->fused && after != base.membrane_after_k1) continue;  // no gradient launch to follow
                 if (cl == base.membrane_cluster && after == base.membrane_after_k1) continue;
                 lbfs_launch_shape trial = base;
                 trial.membrane_cluster = cl;
@@ -3275,7 +3284,6 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
     const int r2 = copy_all(false);
     if (!rc) rc = r2;
     s->t = t0;
-    if (s->fused) s->fields_stale = false;
     drop_graph(s);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -242,3 +242,35 @@ def test_spread_form_does_not_change_bits(stencil):
         n = len(own[1])
         assert np.array_equal(nodes[first:first + n], own[1]) and np.array_equal(force[first:first + n], own[2]), k
         first += n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+def test_autotune_keeps_fields_and_idle_knobs(precision):
+    """The gradient, flux and ghost fields after tuning are those of the step before it on handles that
+    form them on request (FP64, uniform), and there the tuner leaves the block sizes and chunks of kernels
+    that do not run as they were.  More repetitions than steps of a graph, so that both forms are timed."""
+    from lbfs_b200 import GpuSolver, _abi, cases
+    c = cases.shear_rbc(n=24, level=2, radius_cells=4.0, precision=precision)
+    which = (_abi.LBFS_FIELD_GRADIENTS, _abi.LBFS_FIELD_FACE_FLUX, _abi.LBFS_FIELD_GHOST)
+    idle = ("gradient_threads", "flux_threads", "general_flux_threads", "flux_chunks", "membrane_after_k1")
+    for formed in (False, True):  # before tuning, or only after it
+        with GpuSolver(c.mesh, c.params, c.membranes) as s, GpuSolver(c.mesh, c.params, c.membranes) as ref:
+            for h in (s, ref):
+                h.set_state(c.rho, c.u, c.v, c.w)
+                h.step(3, graph=True)
+            before = [ref.field(w) for w in which]
+            shape = s.launch_shape()
+            if formed:
+                assert all(np.array_equal(a, s.field(w)) for a, w in zip(before, which))
+            s.autotune(reps=18)
+            if precision == 0:
+                assert all(np.array_equal(a, s.field(w)) for a, w in zip(before, which))
+                assert all(s.launch_shape()[k] == shape[k] for k in idle)
+            for a, b in zip(s.state(), ref.state()):
+                assert np.array_equal(a, b)
+            # the fields of the next step, of which tuning left no trace
+            ref.set_launch_shape(**{k: v for k, v in s.launch_shape().items() if k != "step_us"})
+            for h in (s, ref):
+                h.step(1, graph=True)
+            assert all(np.array_equal(s.field(w), ref.field(w)) for w in which)
