@@ -14,12 +14,14 @@ namespace lbfs {
 
 // ------------------------------------------------------------------ K1 ----
 
-template <typename R, int TB>
-__global__ void __launch_bounds__(TB, TB == 128 ? 5 : 1) k_cell_gradients(FluidArgs<R> a, int begin, int end) {
+// REST: the cells beside those of the fused step (kSeparateCell); they also keep their state in prev.
+template <typename R, int TB, bool REST>
+__global__ void __launch_bounds__(TB, TB == 128 ? 5 : 1) k_cell_gradients(FluidArgs<R> a, int begin, int end, Vec4<R> *prev) {
     pdl_trigger();  // the interior-face kernel may be scheduled behind the last wave
     const int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end) return;
+    if (i >= end || (REST && !(a.grid_sides[i] & kSeparateCell))) return;
     const Vec4<R> own = a.state[i];
+    if constexpr (REST) prev[i] = own;
     GradRec<R> gr;
     cell_gradient(a, i, own, gr.g);
     reinterpret_cast<GradRec<R> *>(a.grad)[i] = gr;
@@ -31,13 +33,15 @@ __global__ void __launch_bounds__(TB, TB == 128 ? 5 : 1) k_cell_gradients(FluidA
 // Interior faces of an axis-aligned mesh: faces [0, nfx) x, [nfx, nfx+nfy) y,
 // the rest z; warps never mix axes except at the two range boundaries.
 // TB threads per block, 640 / TB blocks per SM (at most 102 registers a thread).
-template <typename R, int TB>
+// REST: the faces of the cells beside those of the fused step.
+template <typename R, int TB, bool REST>
 __global__ void __launch_bounds__(TB, 640 / TB) k_face_flux(FluidArgs<R> a, FaceRanges r) {
     int t = blockIdx.x * blockDim.x + threadIdx.x, f;
     if (t < r.count[0]) f = r.start[0] + t;
     else if ((t -= r.count[0]) < r.count[1]) f = r.start[1] + t;
     else if ((t -= r.count[1]) < r.count[2]) f = r.start[2] + t;
     else return;
+    if (REST && !(a.grid_sides[__ldg(a.face_cells + f).x] & kSeparateCell)) return;
     Vec4<R> out;
     if (f < a.nfx) out = axis_face_flux<R, 0>(a, f);
     else if (f < a.nfx + a.nfy) out = axis_face_flux<R, 1>(a, f);
@@ -97,11 +101,11 @@ __global__ void __launch_bounds__(TB, (sizeof(R) == 4 ? 1024 : 512) / TB) k_face
 
 // Boundary faces (always) and the interior faces of meshes that are not axis
 // aligned: the general-normal reconstruction.  `first` is ni (axis-aligned
-// meshes) or 0.
-template <typename R, int TB>
+// meshes) or 0.  REST: those of the cells beside the fused step's.
+template <typename R, int TB, bool REST>
 __global__ void __launch_bounds__(TB) k_face_flux_general(FluidArgs<R> a, int first) {
     const int f = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= a.nf) return;
+    if (f >= a.nf || (REST && !(a.grid_sides[__ldg(a.face_cells + f).x] & kSeparateCell))) return;
     a.flux[f] = general_face_flux<R, -1>(a, f, f >= a.ni);
 }
 
@@ -433,9 +437,17 @@ template <typename R> int k3_grid(const FluidArgs<R> &a) {
 template <typename R> void launch_fluid_gradients_range(const FluidArgs<R> &a, int begin, int end, cudaStream_t s) {
     if (end <= begin) return;
     const int tb = a.tb_grad, g = (end - begin + tb - 1) / tb;
-    if (tb == 128) k_cell_gradients<R, 128><<<g, 128, 0, s>>>(a, begin, end);
-    else if (tb == 512) k_cell_gradients<R, 512><<<g, 512, 0, s>>>(a, begin, end);
-    else k_cell_gradients<R, 256><<<g, 256, 0, s>>>(a, begin, end);
+    if (tb == 128) k_cell_gradients<R, 128, false><<<g, 128, 0, s>>>(a, begin, end, nullptr);
+    else if (tb == 512) k_cell_gradients<R, 512, false><<<g, 512, 0, s>>>(a, begin, end, nullptr);
+    else k_cell_gradients<R, 256, false><<<g, 256, 0, s>>>(a, begin, end, nullptr);
+}
+// Gradients and fluxes of the cells beside those of the fused step: cells [begin, end) and faces r hold them
+// all, with those of the grids between them, whose threads leave at once.
+void launch_fluid_rest(const FluidArgs<double> &a, int begin, int end, const FaceRanges &r, Vec4<double> *prev, cudaStream_t s) {
+    const int n = r.count[0] + r.count[1] + r.count[2];
+    k_cell_gradients<double, 128, true><<<(end - begin + 127) / 128, 128, 0, s>>>(a, begin, end, prev);
+    if (n > 0) k_face_flux<double, 128, true><<<(n + 127) / 128, 128, 0, s>>>(a, r);
+    if (a.nb > 0) k_face_flux_general<double, 128, true><<<(a.nb + 127) / 128, 128, 0, s>>>(a, a.ni);
 }
 template <typename R> void launch_fluid_gradients(const FluidArgs<R> &a, cudaStream_t s) {
     launch_fluid_gradients_range<R>(a, 0, a.nc, s);
@@ -444,9 +456,9 @@ template <typename R> void launch_fluid_flux_axis_ranges(const FluidArgs<R> &a, 
     const int n = r.count[0] + r.count[1] + r.count[2];
     if (!a.axis_aligned || n == 0) return;
     const int tb = a.tb_flux, g = (n + tb - 1) / tb;
-    if (tb == 64) k_face_flux<R, 64><<<g, 64, 0, s>>>(a, r);
-    else if (tb == 256) k_face_flux<R, 256><<<g, 256, 0, s>>>(a, r);
-    else k_face_flux<R, 128><<<g, 128, 0, s>>>(a, r);
+    if (tb == 64) k_face_flux<R, 64, false><<<g, 64, 0, s>>>(a, r);
+    else if (tb == 256) k_face_flux<R, 256, false><<<g, 256, 0, s>>>(a, r);
+    else k_face_flux<R, 128, false><<<g, 128, 0, s>>>(a, r);
 }
 // A launch with the programmatic-serialization attribute when `pdl` (the
 // kernel directly behind the kernel whose output it reads, on the same stream).
@@ -503,7 +515,7 @@ template <typename R> void launch_fluid_flux_axis(const FluidArgs<R> &a, cudaStr
 // instantiated with per-node priorities).
 template <typename R, int TB> void launch_general(const FluidArgs<R> &a, int first, int g, cudaStream_t s, bool hi) {
     if (!hi) {
-        k_face_flux_general<R, TB><<<g, TB, 0, s>>>(a, first);
+        k_face_flux_general<R, TB, false><<<g, TB, 0, s>>>(a, first);
         return;
     }
     int lo = 0, top = 0;
@@ -517,7 +529,7 @@ template <typename R, int TB> void launch_general(const FluidArgs<R> &a, int fir
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_face_flux_general<R, TB>, a, first);
+    cudaLaunchKernelEx(&cfg, k_face_flux_general<R, TB, false>, a, first);
 }
 template <typename R> void launch_fluid_flux_general(const FluidArgs<R> &a, cudaStream_t s) {
     // boundary faces only when the interior faces have a kernel of their own (axis faces, or tiles)

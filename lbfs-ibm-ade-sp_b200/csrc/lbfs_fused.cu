@@ -208,10 +208,9 @@ __device__ __forceinline__ Vec4<double> face_flux(const GridWeights &g, double p
 // the lower cell at lo, its lower neighbour's state lm and its neighbours lbm, lbp
 // along B and lcm, lcp along C.
 template <int A>
-__device__ __forceinline__ Vec4<double> uniform_flux(const GridArgs &ga, const Planes &pl, const CellSlopes &hi, int lo,
+__device__ __forceinline__ Vec4<double> uniform_flux(const GridWeights &g, const Planes &pl, const CellSlopes &hi, int lo,
                                                      const State4 &lm, int lbm, int lbp, int lcm, int lcp, double tau) {
     constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
-    const GridWeights &g = ga.cw;
     double s1[4], p0, p[3];
     pl.get(lo, s1);
     {
@@ -284,8 +283,8 @@ __device__ __forceinline__ void boundary_slopes(const FluidArgs<double> &a, cons
     }
 }
 
-__device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const GridArgs &ga, int b) {
-    const GridBnd f = ga.bnd[b];
+__device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const GridArgs &ga, const GridSet &gs,
+                                              const GridBnd &f, int b) {
     const GridSide rec = ga.bnd_side[b];
     const int side = f.info & 7, axis = side >> 1;
     double d[3][4], dp[3][4];
@@ -335,7 +334,7 @@ __device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const 
     turn_slopes(d, e);
     turn_slopes(dp, ep);
     const State4 S1 = turned(own.s), S2 = turned(ghost.s), V = turned({rec.val.rho, rec.val.u, rec.val.v, rec.val.w});
-    const GridWeights &g = ga.cw;
+    const GridWeights &g = gs.cw;
     const bool first = (f.info & 1024) != 0;
     double p[4], a1[4], a2[4];
     double b1[4], c1[4], b2[4], c2[4];
@@ -343,7 +342,7 @@ __device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const 
     for (int m = 0; m < 4; m++) {
         const bool dir = (rec.flags & (m == 0 ? 1 : 2)) != 0;
         const bool per = (rec.flags & (m == 0 ? 4 : 8)) != 0;
-        const double Dn = dir ? ga.bnd_k * (S2.s[m] - S1.s[m]) : (per ? ep[0][m] : 0.0);  // ghost's differences
+        const double Dn = dir ? gs.bnd_k * (S2.s[m] - S1.s[m]) : (per ? ep[0][m] : 0.0);  // ghost's differences
         b2[m] = dir ? 0.0 : (per ? ep[1][m] : e[1][m]);
         c2[m] = dir ? 0.0 : (per ? ep[2][m] : e[2][m]);
         const double wD = g.w * Dn;
@@ -361,28 +360,34 @@ __device__ __forceinline__ void grid_boundary(const FluidArgs<double> &a, const 
     const SideSums n = uniform_side<0, -1>(a2[0], v2, b2, c2, g);
 #pragma unroll
     for (int m = 0; m < 4; m++) { b1[m] = b1[m] + b2[m]; c1[m] = c1[m] + c2[m]; }
-    const Vec4<double> t = face_flux<0>(g, p[0], pv, b1, c1, o, n, relaxation(a, 1.0, ga.dt));
+    const Vec4<double> t = face_flux<0>(g, p[0], pv, b1, c1, o, n, relaxation(a, 1.0, gs.dt));
     const double fn = sn * t.u;
     Vec4<double> out;
-    out.rho = t.rho * ga.area;
-    out.u = (axis == 0 ? fn : t.v) * ga.area;
-    out.v = (axis == 1 ? fn : (axis == 0 ? t.v : t.w)) * ga.area;
-    out.w = (axis == 2 ? fn : t.w) * ga.area;
+    out.rho = t.rho * gs.area;
+    out.u = (axis == 0 ? fn : t.v) * gs.area;
+    out.v = (axis == 1 ? fn : (axis == 0 ? t.v : t.w)) * gs.area;
+    out.w = (axis == 2 ? fn : t.w) * gs.area;
     a.flux[a.ni + f.face] = out;
 }
 
+// SETS: grids of several spacings, whose constants a block loads (one spacing: kernel parameters).
+template <bool SETS>
 __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_step(FluidArgs<double> a, GridArgs ga) {
     extern __shared__ __align__(16) unsigned char raw[];
     constexpr int H = 2, TB = kUniformThreads;  // H 16-byte pieces of a state record
     pdl_trigger();
     const int bnd = bnd_before(ga, blockIdx.x);
     if (bnd_before(ga, blockIdx.x + 1) > bnd) {
-        const int b = ga.bnd0 + bnd * TB + threadIdx.x;
-        if (b < ga.bnd1) grid_boundary(a, ga, b);
+        const int b = bnd * TB + threadIdx.x;
+        if (b >= ga.n_bnd) return;
+        const GridBnd f = ga.bnd[b];
+        if constexpr (SETS) grid_boundary(a, ga, ga.sets[f.info >> 11], f, b);
+        else grid_boundary(a, ga, ga.set, f, b);
         return;
     }
     const GridTile t = ga.tiles[blockIdx.x - bnd];
     const GridInst gi = ga.inst[t.inst];
+    const GridSet &gs = SETS ? ga.sets[t.set] : ga.set;
     const int Q = ga.plane_stride;
     Planes pl;
     pl.h = reinterpret_cast<double2 *>(raw);
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_ste
     const int gx = t.x0 + lx, gy = t.y0 + ly;
     const int at = (ly + 2) * W + lx + 2;
     const int c00 = gi.cell0 + gx + gi.nx * gy;
-    const double tau1 = relaxation(a, 1.0, ga.dt);  // at a viscosity factor of 1
+    const double tau1 = relaxation(a, 1.0, gs.dt);  // at a viscosity factor of 1
     const size_t n = (size_t)a.nc;
 
     for (int k = t.z0 - 1; k <= t.z0 + 1; k++) bring(k, false);
@@ -518,7 +523,7 @@ __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_ste
             const double *vis0 = vis + (k % 3) * Q + at;
             if (gx > 0) {
                 const int l = pk + at - 1;
-                const Vec4<double> v = uniform_flux<0>(ga, pl, cell, l, pl.at(l - 1), l - W, l + W, pm + at - 1,
+                const Vec4<double> v = uniform_flux<0>(gs.cw, pl, cell, l, pl.at(l - 1), l - W, l + W, pm + at - 1,
                                                      pp + at - 1, tau1 * vis0[-1]);
                 double *f = fx + tid;
                 f[0] = v.rho; f[TB] = v.u; f[2 * TB] = v.v; f[3 * TB] = v.w;
@@ -526,7 +531,7 @@ __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_ste
             }
             if (gy > 0) {
                 const int l = pk + at - W;
-                const Vec4<double> v = uniform_flux<1>(ga, pl, cell, l, pl.at(l - W), l - 1, l + 1, pm + at - W,
+                const Vec4<double> v = uniform_flux<1>(gs.cw, pl, cell, l, pl.at(l - W), l - 1, l + 1, pm + at - W,
                                                      pp + at - W, tau1 * vis0[-W]);
                 double *f = fy + tid;
                 f[0] = v.rho; f[TB] = v.u; f[2 * TB] = v.v; f[3 * TB] = v.w;
@@ -541,7 +546,7 @@ __global__ void __launch_bounds__(kUniformThreads, kUniformBlocks) k_uniform_ste
                 State4 two;  // of plane k - 2
 #pragma unroll
                 for (int m = 0; m < 4; m++) two.s[m] = below[m * TB + tid];
-                z = uniform_flux<2>(ga, pl, cell, l, two, l - 1, l + 1, l - W, l + W, tau1 * vis[((k - 1) % 3) * Q + at]);
+                z = uniform_flux<2>(gs.cw, pl, cell, l, two, l - 1, l + 1, l - W, l + W, tau1 * vis[((k - 1) % 3) * Q + at]);
                 if (k == t.z0) ga.edge[2 * n + c] = z;
             }
             double lo[4];
@@ -577,13 +582,17 @@ size_t grid_smem_bytes(const GridArgs &ga) {
 }
 // The limit is the kernel's, shared by every handle: always the largest.
 cudaError_t grid_prepare() {
-    return cudaFuncSetAttribute(k_uniform_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(k_uniform_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_uniform_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
 }
 static_assert(sizeof(double) * ((kSlots * 4 + 3) * kUniformPlaneMax + 12 * kUniformThreads) +
                       kUniformThreads * (32 + sizeof(GridSide)) <= 64 * 1024,
               "a tile's shared memory");
 void launch_grid_step(const FluidArgs<double> &a, const GridArgs &ga, cudaStream_t s) {
-    k_uniform_step<<<ga.bnd_blocks + ga.n_tiles, kUniformThreads, grid_smem_bytes(ga), s>>>(a, ga);
+    const int blocks = ga.bnd_blocks + ga.n_tiles;
+    if (ga.n_sets > 1) k_uniform_step<true><<<blocks, kUniformThreads, grid_smem_bytes(ga), s>>>(a, ga);
+    else k_uniform_step<false><<<blocks, kUniformThreads, grid_smem_bytes(ga), s>>>(a, ga);
 }
 
 }  // namespace lbfs

@@ -29,7 +29,7 @@ constexpr int kUniformBlocks = 4;      // blocks an SM, 128 registers a thread
 constexpr int kUniformPlaneMax = 230;  // cells of a tile's plane with two more below and one above along x and y
 
 struct GridTile {
-    int x0, y0, z0, w, h, d, inst, pad;  // columns [x0, x0 + w) x [y0, y0 + h), planes [z0, z0 + d)
+    int x0, y0, z0, w, h, d, inst, set;  // columns [x0, x0 + w) x [y0, y0 + h), planes [z0, z0 + d); its GridSet
 };
 struct GridInst {
     int cell0, nx, ny, nz;
@@ -48,7 +48,8 @@ struct GridSide {
 };
 // One boundary face: its cell, the cell's strides along y and z, info -- its side d,
 // up to two more missing sides of the cell << 3 and << 6 (7: none) with their
-// boundary faces in more, bit 10: the interior branch (an instance's first ghost);
+// boundary faces in more, bit 10: the interior branch (an instance's first ghost), its
+// GridSet << 11;
 // partner: a boundary face of the periodic partner cell; face: its index among the mesh's boundary faces.
 struct alignas(16) GridBnd {
     int cell, sy, sz, info, more[2], partner, face;
@@ -59,19 +60,25 @@ struct GridWeights {
     double w, w3, ww3, h, h3, hh3;
 };
 
+// What the faces of grids of one spacing share.
+struct GridSet {
+    double bnd_k;                  // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
+    GridWeights cw;
+    double area, dt;               // of every interior face
+};
+
 struct GridArgs {
-    int n_tiles, bnd_blocks;
-    int bnd0, bnd1;                // boundary faces of this launch
+    int n_tiles, n_bnd, bnd_blocks;
+    int n_sets;
     int plane_stride;              // cells of the largest tile's plane
     int stage_max;                 // threads that may hold a ghost's record
     const GridTile *tiles;
     const GridInst *inst;
     const GridSide *side;          // the boundary faces of every side of every instance
-    const GridBnd *bnd;            // the boundary faces, launch by launch
-    const GridSide *bnd_side;      // their records in that order
-    double bnd_k;                  // dt / (owner-ghost distance x w): a Dirichlet ghost's slope in differences
-    GridWeights cw;
-    double area, dt;               // of every interior face
+    const GridBnd *bnd;            // [n_bnd] the boundary faces
+    const GridSide *bnd_side;      // [n_bnd] their records in that order
+    GridSet set;                   // of all grids (n_sets 1)
+    const GridSet *sets;           // else one each
     Vec4<double> *prev;            // [nc + nb] the state the last step started from
     double4 *res;                  // [nc] sums of the interior face fluxes per unit area, those in edge left out
     Vec4<double> *edge;            // [3][nc] low fluxes per unit area of the tiles' first columns, rows and planes

@@ -19,6 +19,7 @@ constexpr int kK3BlocksLimit = LBFS_MAX_UPDATE_BLOCKS;  // partial-sum slots all
 template <typename R> void launch_fluid_gradients(const FluidArgs<R> &a, cudaStream_t s);
 // K1 over cells [begin, end) and K2 over up to three axis face ranges (the pipelined form)
 template <typename R> void launch_fluid_gradients_range(const FluidArgs<R> &a, int begin, int end, cudaStream_t s);
+void launch_fluid_rest(const FluidArgs<double> &a, int begin, int end, const FaceRanges &r, Vec4<double> *prev, cudaStream_t s);
 template <typename R> void launch_fluid_flux_axis_ranges(const FluidArgs<R> &a, const FaceRanges &r, cudaStream_t s);
 // K2 over the faces owned by tiles [tile0, tile1) of a.flux_tiles (axis-aligned meshes whose faces are
 // ordered by owner within each axis)

@@ -57,14 +57,13 @@ struct lbfs_solver {
     // tiles of the face kernel (interior faces ordered by owner within each axis), one table per flux
     // block size 64 / 128 / 256: tiles_h[b] = first face of each axis owned by tile t (3 ints per
     // tile, n_tiles + 1 rows), tile_maxnb[b][t] = largest neighbour of the faces of tiles <= t
-    // fused fluid step of structured grids (lbfs_fused.h, FP64 handles): its launches, one per set of face
-    // constants, when `fused`, and the instances that keep the separate kernels (rest).
+    // fused fluid step of structured grids (lbfs_fused.h, FP64 handles): its plan when `fused`, and the
+    // instances that keep the separate kernels (rest).
     // separate: steps take the separate kernels all the same (the adjoint's recording, which reads
     // every step's gradients).  fields_stale: the last step left no gradients, fluxes or ghosts; they
     // are formed from the state it started from (prev, where prev_last) when asked for.
     bool fused = false, separate = false, fields_stale = false, prev_last = false;
-    std::vector<GridArgs> passes;
-    const unsigned char *grid_sides = nullptr;
+    GridArgs grid{};
     struct Rest {
         bool any = false;
         int cell0 = 0, cell1 = 0;  // their cells and faces, with those of the grids between them
@@ -575,6 +574,7 @@ struct GridCheck {
     GridInst g{};
     int face[3][2], bnd[2];  // its interior faces along each axis and its boundary faces
     double area = 0, dt = 0, weight = 0, dmag = 0;
+    int set = 0;
     bool fits = false;
 };
 
@@ -699,7 +699,7 @@ bool grid_fits(lbfs_solver *s, const lbfs_mesh_desc *m, const lbfs_grid_desc &gd
 }
 
 // The fused step's plan: which instances take the pass (each by itself, so that an instance of an
-// ensemble steps as it does in a handle of its own), one launch per set of face constants, the ghosts,
+// ensemble steps as it does in a handle of its own), the faces' constants of each spacing, the ghosts,
 // and the tiles.  Instances that do not keep the separate kernels.  Leaves s->fused false where none
 // does (LBFS_SEPARATE_KERNELS set: always; a diagnostic switch).
 int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
@@ -746,32 +746,35 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
         r.cell1 = c1;
         for (int ax = 0; ax < 3; ax++) r.faces.count[ax] = q.face[ax][1] - r.faces.start[ax];
     }
-    // one launch per set of face constants
-    std::vector<std::vector<int>> sets;
+    // the sets of face constants
+    std::vector<GridSet> sets;
+    std::vector<int> one;  // an instance of each
     for (int k = 0; k < n_inst; k++) {
-        if (!check[k].fits) continue;
-        size_t e = 0;
-        auto same = [&](const GridCheck &x, const GridCheck &y) {
-            return x.area == y.area && x.dt == y.dt && x.weight == y.weight && x.dmag == y.dmag;
+        GridCheck &q = check[k];
+        if (!q.fits) continue;
+        auto same = [&](const GridCheck &x) {
+            return x.area == q.area && x.dt == q.dt && x.weight == q.weight && x.dmag == q.dmag;
         };
-        while (e < sets.size() && !same(check[sets[e][0]], check[k])) e++;
-        if (e == sets.size()) sets.emplace_back();
-        sets[e].push_back(k);
+        while (q.set < (int)one.size() && !same(check[one[q.set]])) q.set++;
+        if (q.set < (int)one.size()) continue;
+        const double c = -q.weight * q.dt;
+        sets.push_back({q.dt / (q.dmag * c), {c, 3.0 * c, 3.0 * c * c, 0.5 * c, 1.5 * c, 0.75 * c * c}, q.area, q.dt});
+        one.push_back(k);
     }
-    // the boundary faces in the order of the launches: place[b] their place in it
+    // the boundary faces of the pass: place[b] their place among them
     std::vector<int> place(nb, -1);
     int placed = 0, sided = 0;
-    for (const std::vector<int> &set : sets)
-        for (int k : set) {
-            GridInst &g = check[k].g;
-            const int area[3] = {g.ny * g.nz, g.nx * g.nz, g.nx * g.ny};
-            for (int d = 0; d < 6; d++) {
-                g.side0[d] = sided;
-                sided += area[d / 2];
-            }
-            for (int b = check[k].bnd[0]; b < check[k].bnd[1]; b++) place[b] = placed++;
+    for (GridCheck &q : check) {
+        if (!q.fits) continue;
+        GridInst &g = q.g;
+        const int area[3] = {g.ny * g.nz, g.nx * g.nz, g.nx * g.ny};
+        for (int d = 0; d < 6; d++) {
+            g.side0[d] = sided;
+            sided += area[d / 2];
         }
-    // the ghosts as the gradients take them (ghost_state), by side and in the launches' order
+        for (int b = q.bnd[0]; b < q.bnd[1]; b++) place[b] = placed++;
+    }
+    // the ghosts as the gradients take them (ghost_state), by side and by face
     std::vector<GridSide> side(sided), bnd_side(placed);
     std::vector<GridBnd> bnd(placed);
     std::vector<int> side_bc(sided, -1), face_of(nc, -1);  // boundary face of a side's place; one of a cell's
@@ -816,7 +819,7 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
                     r.more[others++] = place[side_bc[at(d, i, j, k)]];
                 }
                 for (; others < 2; others++) r.info |= 7 << (3 + 3 * others);
-                if (gm.gen[b].bc_branch == 0.0) r.info |= 1024;
+                r.info |= (gm.gen[b].bc_branch == 0.0 ? 1024 : 0) | q.set << 11;
             }
         }
     // the tiles, with one walk length d for all instances.  A block's time is d planes and a start of 1.2
@@ -850,78 +853,64 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
             depth = d;
         }
     }
-    // what the launches share
     int rc;
-    GridArgs all{};
+    GridArgs &ga = s->grid;
+    ga = GridArgs{};
     std::vector<GridInst> inst(n_inst);
     std::vector<GridCells> cells(n_inst);
-    for (int k = 0; k < n_inst; k++) {
-        inst[k] = check[k].g;
-        cells[k] = {check[k].g.nx, check[k].g.nx * check[k].g.ny, check[k].area};
+    std::vector<GridTile> tiles;
+    for (int q = 0; q < n_inst; q++) {
+        const GridInst &g = check[q].g;
+        inst[q] = g;
+        cells[q] = {g.nx, g.nx * g.ny, check[q].area};
+        if (!check[q].fits) continue;
+        const int walks = (g.nz + depth - 1) / depth, dz = (g.nz + walks - 1) / walks;
+        for (int z = 0; z < g.nz; z += dz)
+            for (int y = 0; y < g.ny; y += shape[q].h)
+                for (int x = 0; x < g.nx; x += shape[q].w) {
+                    const GridTile t = {x, y, z, std::min(shape[q].w, g.nx - x), std::min(shape[q].h, g.ny - y),
+                                        std::min(dz, g.nz - z), q, check[q].set};
+                    tiles.push_back(t);
+                    // upper faces that other tiles form
+                    const int i1 = t.x0 + t.w - 1, j1 = t.y0 + t.h - 1, k1 = t.z0 + t.d - 1;
+                    auto mark = [&](int i0, int j0, int k0, int bit) {
+                        for (int k = k0; k <= k1; k++)
+                            for (int j = j0; j <= j1; j++)
+                                for (int i = i0; i <= i1; i++)
+                                    sides[g.cell0 + i + g.nx * (j + g.ny * k)] |= (unsigned char)(1 << bit);
+                    };
+                    if (i1 < g.nx - 1) mark(i1, t.y0, t.z0, 1);
+                    if (j1 < g.ny - 1) mark(t.x0, j1, t.z0, 2);
+                    if (k1 < g.nz - 1) mark(t.x0, t.y0, k1, 3);
+                    ga.plane_stride = std::max(ga.plane_stride, (t.w + 3) * (t.h + 3));
+                    ga.stage_max = std::max(ga.stage_max, 2 * (t.w + t.h + 4));
+                }
     }
+    GridTile *d_tiles;
     GridInst *d_inst;
     GridSide *d_side, *d_bside;
     GridBnd *d_bnd;
-    if ((rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) || (rc = s->upload(&d_bnd, bnd)) ||
-        (rc = s->upload(&d_bside, bnd_side)) || (rc = s->alloc(&all.res, nc)) ||
-        (rc = s->alloc(&all.prev, (size_t)nc + nb)) || (rc = s->alloc(&all.edge, 3 * (size_t)nc)))
-        return rc;
-    all.inst = d_inst; all.side = d_side; all.bnd = d_bnd; all.bnd_side = d_bside;
-    s->passes.clear();
-    int faces = 0;
-    for (const std::vector<int> &set : sets) {
-        GridArgs ga = all;
-        const GridCheck &one = check[set[0]];
-        ga.area = one.area;
-        ga.dt = one.dt;
-        const double c = -one.weight * one.dt;
-        ga.cw = {c, 3.0 * c, 3.0 * c * c, 0.5 * c, 1.5 * c, 0.75 * c * c};
-        ga.bnd_k = one.dt / (one.dmag * c);
-        std::vector<GridTile> tiles;
-        ga.bnd0 = faces;
-        for (int q : set) {
-            const GridInst &g = check[q].g;
-            const int walks = (g.nz + depth - 1) / depth, dz = (g.nz + walks - 1) / walks;
-            for (int z = 0; z < g.nz; z += dz)
-                for (int y = 0; y < g.ny; y += shape[q].h)
-                    for (int x = 0; x < g.nx; x += shape[q].w) {
-                        const GridTile t = {x, y, z, std::min(shape[q].w, g.nx - x), std::min(shape[q].h, g.ny - y),
-                                            std::min(dz, g.nz - z), q, 0};
-                        tiles.push_back(t);
-                        // upper faces that other tiles form
-                        const int i1 = t.x0 + t.w - 1, j1 = t.y0 + t.h - 1, k1 = t.z0 + t.d - 1;
-                        auto mark = [&](int i0, int j0, int k0, int bit) {
-                            for (int k = k0; k <= k1; k++)
-                                for (int j = j0; j <= j1; j++)
-                                    for (int i = i0; i <= i1; i++)
-                                        sides[g.cell0 + i + g.nx * (j + g.ny * k)] |= (unsigned char)(1 << bit);
-                        };
-                        if (i1 < g.nx - 1) mark(i1, t.y0, t.z0, 1);
-                        if (j1 < g.ny - 1) mark(t.x0, j1, t.z0, 2);
-                        if (k1 < g.nz - 1) mark(t.x0, t.y0, k1, 3);
-                        ga.plane_stride = std::max(ga.plane_stride, (t.w + 3) * (t.h + 3));
-                        ga.stage_max = std::max(ga.stage_max, 2 * (t.w + t.h + 4));
-                    }
-            faces += check[q].bnd[1] - check[q].bnd[0];
-        }
-        ga.bnd1 = faces;
-        ga.bnd_blocks = (ga.bnd1 - ga.bnd0 + kUniformThreads - 1) / kUniformThreads;
-        ga.n_tiles = (int)tiles.size();
-        GridTile *d_tiles;
-        if ((rc = s->upload(&d_tiles, tiles))) return rc;
-        ga.tiles = d_tiles;
-        s->passes.push_back(ga);
-    }
+    GridSet *d_sets;
     unsigned char *d_sides;
-    if ((rc = s->upload(&d_sides, sides))) return rc;
-    s->grid_sides = d_sides;
-    a.grid_edge = all.edge;
-    const bool one_grid = n_inst == 1, one_kind = sets.size() == 1 && !s->rest.any;
-    a.grid_mixed = !one_kind;
-    a.grid_area = check[sets[0][0]].area;
-    a.grid_stride[0] = one_grid ? inst[0].nx : 0;
-    a.grid_stride[1] = one_grid ? inst[0].nx * inst[0].ny : 0;
-    if (!one_grid) {
+    if ((rc = s->upload(&d_tiles, tiles)) || (rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) ||
+        (rc = s->upload(&d_bnd, bnd)) || (rc = s->upload(&d_bside, bnd_side)) || (rc = s->upload(&d_sets, sets)) ||
+        (rc = s->upload(&d_sides, sides)) || (rc = s->alloc(&ga.res, nc)) || (rc = s->alloc(&ga.prev, (size_t)nc + nb)) ||
+        (rc = s->alloc(&ga.edge, 3 * (size_t)nc)))
+        return rc;
+    ga.n_tiles = (int)tiles.size();
+    ga.n_bnd = placed;
+    ga.bnd_blocks = (placed + kUniformThreads - 1) / kUniformThreads;
+    ga.n_sets = (int)sets.size();
+    ga.tiles = d_tiles; ga.inst = d_inst; ga.side = d_side; ga.bnd = d_bnd; ga.bnd_side = d_bside;
+    ga.set = sets[0];
+    ga.sets = d_sets;
+    a.grid_sides = d_sides;
+    a.grid_edge = ga.edge;
+    a.grid_mixed = sets.size() > 1 || s->rest.any;
+    a.grid_area = sets[0].area;
+    a.grid_stride[0] = n_inst == 1 ? inst[0].nx : 0;
+    a.grid_stride[1] = n_inst == 1 ? inst[0].nx * inst[0].ny : 0;
+    if (n_inst > 1) {
         std::vector<int> which(nc);
         for (int k = 0; k < n_inst; k++) std::fill_n(which.begin() + s->grids[k].cell0, s->grids[k].n_cells, k);
         GridCells *d_cells;
@@ -1355,7 +1344,7 @@ void set_chunks(lbfs_solver *s, int K) {
     const std::vector<int> &mx = s->tile_maxnb[tb == 64 ? 0 : (tb == 256 ? 2 : 1)];
     // fused step: fluid pass and update; else gradients and interior fluxes (K each), boundary fluxes,
     // update; membrane kernels; CFL
-    s->launches_per_step = (s->fused ? (int)s->passes.size() + 1 + (s->rest.any ? 3 : 0) : 2 * K + 2) + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
+    s->launches_per_step = (s->fused ? (s->rest.any ? 5 : 2) : 2 * K + 2) + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
     s->chunk_cell.assign(K + 1, 0);
     s->chunk_faces.assign(K, FaceRanges{});
     for (int c = 0; c <= K; c++) s->chunk_cell[c] = (int)((long long)s->nc * c / K);
@@ -1547,8 +1536,7 @@ int fork_behind_launch(lbfs_solver *s) {
 // beside: 44.6 / 36.5 on 48^3 with 162 nodes, 64.8 / 55.5 at 64^3 with 642).
 int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
     FluidArgs<double> a = s->f64;
-    a.grid_res = s->passes[0].res;
-    a.grid_sides = s->grid_sides;
+    a.grid_res = s->grid.res;
     int n = 0;
     for (int p = 0; p < kPhases; p++) s->phase_recorded[p] = false;
     if (s->profiling) LBFS_CUDA(record_event(s->ev_phase[5][0], s->stream));
@@ -1556,21 +1544,19 @@ int enqueue_fused_step(lbfs_solver *s, bool visc_update, int *launches) {
         launch_fluid_cfl<double>(a, s->stream);
         n += 1;
     }
+    // the instances that keep the separate kernels beside the pass, on a stream of their own
     auto pass = [&]() -> int {
         PhaseMark m(s, 2, s->stream);
-        if (s->rest.any) {  // the instances between take part, before the pass writes their fluxes and its copy of the state
-            const size_t c0 = (size_t)s->rest.cell0, count = (size_t)(s->rest.cell1 - s->rest.cell0);
-            launch_fluid_gradients_range<double>(a, s->rest.cell0, s->rest.cell1, s->stream);
-            launch_fluid_flux_axis_ranges<double>(a, s->rest.faces, s->stream);
-            launch_fluid_flux_general<double>(a, s->stream);
-            LBFS_CUDA(cudaMemcpyAsync(s->passes[0].prev + c0, a.state + c0, sizeof(Vec4<double>) * count,
-                                      cudaMemcpyDeviceToDevice, s->stream));
+        if (s->rest.any) {
+            LBFS_CUDA(cudaEventRecord(s->ev_chunk[0], s->stream));
+            LBFS_CUDA(cudaStreamWaitEvent(s->stream4, s->ev_chunk[0], 0));
+            launch_fluid_rest(a, s->rest.cell0, s->rest.cell1, s->rest.faces, s->grid.prev, s->stream4);
+            LBFS_CUDA(cudaEventRecord(s->ev_flux, s->stream4));
             n += 3;
         }
-        for (const GridArgs &ga : s->passes) {
-            launch_grid_step(a, ga, s->stream);
-            n += 1;
-        }
+        launch_grid_step(a, s->grid, s->stream);
+        n += 1;
+        if (s->rest.any) LBFS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_flux, 0));
         return LBFS_OK;
     };
     int rc = LBFS_OK;
@@ -1683,7 +1669,7 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
 int ensure_fields(lbfs_solver *s) {
     if (!s->fields_stale) return LBFS_OK;
     FluidArgs<double> a = s->f64;
-    a.state = s->passes[0].prev;
+    a.state = s->grid.prev;
     launch_fluid_gradients<double>(a, s->stream);
     launch_fluid_flux<double>(a, s->stream);
     LBFS_CUDA(cudaGetLastError());
@@ -3177,7 +3163,7 @@ namespace {
 int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) {
     LBFS_CUDA(cudaStreamSynchronize(s->stream));
     std::vector<CkPart> parts = ck_parts(s);
-    if (s->prev_last) parts.push_back({s->passes[0].prev, sizeof(Vec4<double>) * (size_t)s->nc});
+    if (s->prev_last) parts.push_back({s->grid.prev, sizeof(Vec4<double>) * (size_t)s->nc});
     size_t total = 0;
     for (const CkPart &p : parts) total += p.bytes;
     DevBuf snap;
@@ -3225,8 +3211,7 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
         std::vector<int> values;
     };
     const bool membranes = s->n_membranes > 0;
-    const bool separate = !s->fused || s->rest.any;  // the separate kernels run: the knobs of theirs that have an effect
-    auto theirs = [&](std::vector<int> values) { return separate ? values : std::vector<int>{}; };
+    auto theirs = [&](std::vector<int> values) { return s->fused ? std::vector<int>{} : values; };  // the separate kernels'
     const std::vector<Knob> knobs = {
         {&lbfs_launch_shape::gradient_threads, theirs({128, 256, 512})},
         {&lbfs_launch_shape::flux_threads, theirs({64, 128, 256})},
@@ -3235,7 +3220,7 @@ int autotune_steps(lbfs_solver *s, int reps, lbfs_launch_shape *out, bool fp32) 
         {&lbfs_launch_shape::update_blocks, {148 * 2, 148 * 4, 148 * 8, 148 * 16}},
         {&lbfs_launch_shape::spread_blocks,
          membranes ? std::vector<int>{148, 296, 592, 1184, 2368} : std::vector<int>{}},
-        {&lbfs_launch_shape::flux_chunks, s->chunkable && !s->fused ? std::vector<int>{1, 2, 4, 8} : std::vector<int>{}},
+        {&lbfs_launch_shape::flux_chunks, s->chunkable ? theirs({1, 2, 4, 8}) : std::vector<int>{}},
     };
     lbfs_launch_shape cur = fp32 ? args_to_shape<float>(s) : args_to_shape<double>(s);
     double best = 0;
