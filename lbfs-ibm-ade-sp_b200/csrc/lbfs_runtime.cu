@@ -414,7 +414,7 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     int *d_rt, *d_vt, *d_per, *d_cf;
     int2 *d_stencil;
     LsRec<R> *d_ls = nullptr;
-    LsW<R> *d_lsw;
+    LsW<R> *d_lsw = nullptr;
     R *d_visc;
     Vec4<R> *d_bcv;
     BcRec<R> *d_bcr;
@@ -422,15 +422,16 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
     AxisFace<R> *d_axf = nullptr;
     GenFace<R> *d_gen;
     double *d_vol, *d_ivol;
-    if ((rc = s->upload(&d_stencil, stencil)) || (rc = s->upload(&d_lsw, lsw)) ||
-        (!ls.empty() && (rc = s->upload(&d_ls, ls))) ||
+    // (not what the kernels take from the parameters instead: 464 B a cell of a uniform FP64 mesh, half of what a
+    // handle held)
+    if ((rc = s->upload(&d_stencil, stencil)) || (!coded && (rc = s->upload(&d_lsw, lsw))) ||
+        (!ls.empty() && !a.ls_coded && (rc = s->upload(&d_ls, ls))) ||
         (rc = s->upload(&d_rt, rt)) || (rc = s->upload(&d_vt, vt)) || (rc = s->upload(&d_per, per)) ||
         (rc = s->upload(&d_bcv, bcv)) ||
         (rc = s->upload(&d_bcr, bcr)) || (rc = s->upload(&d_fcells, fcells)) || (rc = s->upload(&d_gen, gen)) ||
         (rc = s->upload(&d_cf, cf)) || (rc = s->upload(&d_vol, vol)) || (rc = s->upload(&d_ivol, inv_vol)) ||
         (rc = s->upload(&d_visc, visc)))
         return rc;
-    if (a.axis_aligned && (rc = s->upload(&d_axf, axf))) return rc;
     // one geometry per axis (bit for bit) on the generator's uniform meshes
     a.axis_uniform = 0;
     if (a.axis_aligned && ni > 0 && !generic) {
@@ -449,6 +450,7 @@ template <typename R> int setup_fluid(lbfs_solver *s, const lbfs_mesh_desc *m) {
         }
         a.axis_uniform = uniform ? 1 : 0;
     }
+    if (a.axis_aligned && !a.axis_uniform && (rc = s->upload(&d_axf, axf))) return rc;
     // K3 on the generator's structured meshes (one instance): the face table in closed form when it
     // equals the table entry for entry, and one 1 / volume when every cell has it
     a.grid_faces = 0;
@@ -894,9 +896,14 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
     unsigned char *d_sides;
     if ((rc = s->upload(&d_tiles, tiles)) || (rc = s->upload(&d_inst, inst)) || (rc = s->upload(&d_side, side)) ||
         (rc = s->upload(&d_bnd, bnd)) || (rc = s->upload(&d_bside, bnd_side)) || (rc = s->upload(&d_sets, sets)) ||
-        (rc = s->upload(&d_sides, sides)) || (rc = s->alloc(&ga.res, nc)) || (rc = s->alloc(&ga.prev, (size_t)nc + nb)) ||
-        (rc = s->alloc(&ga.edge, 3 * (size_t)nc)))
+        (rc = s->upload(&d_sides, sides)) || (rc = s->alloc(&ga.res, nc)) || (rc = s->alloc(&ga.prev, (size_t)nc + nb)))
         return rc;
+    // the edge fluxes in the gradients' array, which is used only when the fields are formed from prev, unless
+    // other instances' gradients are there (an edge record a cell in the cell's gradient record would do for
+    // both, but costs: 128^3 2908 us for ten steps, against 2710)
+    static_assert(3 * sizeof(Vec4<double>) == sizeof(GradRec<double>), "edge fluxes in the gradients' array");
+    ga.edge = reinterpret_cast<Vec4<double> *>(a.grad);
+    if (s->rest.any && (rc = s->alloc(&ga.edge, 3 * (size_t)nc))) return rc;
     ga.n_tiles = (int)tiles.size();
     ga.n_bnd = placed;
     ga.bnd_blocks = (placed + kUniformThreads - 1) / kUniformThreads;

@@ -89,3 +89,26 @@ def test_fields_of_the_last_step_are_kept(monkeypatch):
     assert all(np.array_equal(s.field(w), t.field(w)) for w in which)
     s.close()
     t.close()
+
+
+@pytest.mark.gpu
+def test_device_memory_of_a_handle(monkeypatch):
+    """What the fused step keeps beside the separate kernels' arrays is the state the last step started
+    from and the cell sums (64 B a cell) and its tables; and a uniform mesh's weights, inverses and face
+    geometry, which the kernels take from their parameters, are not uploaded: 530 B a cell by the arrays'
+    sizes (state and accumulator 64, gradients and fluxes 192, stencil, faces and boundary lists 80,
+    volumes, viscosity, centroids and codes 52, kept state and sums 64, the rest boundary and tables),
+    where 1104 were held."""
+    import torch
+    from lbfs_b200 import cases
+    torch.cuda.init()
+    c = cases.poiseuille(96)
+    held = {}
+    for separate in (False, True):
+        _handle(c, monkeypatch, separate).close()  # the library's own contexts and modules
+        free = torch.cuda.mem_get_info()[0]
+        s = _handle(c, monkeypatch, separate)
+        held[separate] = (free - torch.cuda.mem_get_info()[0]) / c.mesh.n_cells
+        s.close()
+    assert held[False] < held[True] + 90, held
+    assert held[False] < 660, held  # allocations are rounded up to 2 MB, some 40 of them: 95 B a cell
