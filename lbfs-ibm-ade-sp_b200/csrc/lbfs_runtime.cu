@@ -855,6 +855,7 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
             depth = d;
         }
     }
+    if (const char *v = std::getenv("LBFS_GRID_WALK")) depth = std::max(1, std::atoi(v));  // a diagnostic switch
     int rc;
     GridArgs &ga = s->grid;
     ga = GridArgs{};

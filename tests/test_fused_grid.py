@@ -95,10 +95,9 @@ def test_fields_of_the_last_step_are_kept(monkeypatch):
 def test_device_memory_of_a_handle(monkeypatch):
     """What the fused step keeps beside the separate kernels' arrays is the state the last step started
     from and the cell sums (64 B a cell) and its tables; and a uniform mesh's weights, inverses and face
-    geometry, which the kernels take from their parameters, are not uploaded: 530 B a cell by the arrays'
-    sizes (state and accumulator 64, gradients and fluxes 192, stencil, faces and boundary lists 80,
-    volumes, viscosity, centroids and codes 52, kept state and sums 64, the rest boundary and tables),
-    where 1104 were held."""
+    geometry, which the kernels take from their parameters, are not uploaded: some 450 B a cell by the
+    arrays' sizes (state and accumulator 64, gradients and fluxes 192, stencil and faces 72, volumes,
+    viscosity, centroids and codes 52, kept state and sums 64, and boundary tables)."""
     import torch
     from lbfs_b200 import cases
     torch.cuda.init()
