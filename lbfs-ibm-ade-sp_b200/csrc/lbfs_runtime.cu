@@ -825,10 +825,15 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
             }
         }
     // the tiles, with one walk length d for all instances.  A block's time is d planes and a start of 1.2
-    // (clock stamps inside the kernel), a plane's about 3000 cycles and 1300 for each
-    // block on its SM.  Grids of at most one wave: the longest block at that occupancy; larger ones: the
-    // blocks' throughput and a third of a block for the last wave.  64^3 FP64: 45 us at the chosen d = 4,
-    // 47 at 3, 54 at 8; 128^3: 203 at 8, 206 at 4, 213 at 16.
+    // (clock stamps inside the kernel), a plane's about 3000 cycles and 1300 for each block on its SM.
+    // Tiles of at most one wave: the longest block at that occupancy, a tenth more where the boundary faces'
+    // blocks, of which the last tiles wait for some, are more than a wave themselves; more tiles: their
+    // throughput and a third of a block for the last wave.  us per step at the chosen walk and at others:
+    // 64^3 39.3 at 4, 44.2 / 40.3 / 46.4 at 1 / 3 / 6; 128^3 234.3 at 8, 237.4 / 228.4 / 252.8 at 4 / 11 / 32
+    // (32 without the tenth); 96^3 109.5 at 12, 136.3 / 108.8 / 126.0 at 1 / 5 / 16.  On 28 ducts of 20 to 200
+    // cells an axis the choice is 3.3 % from the best walk on average, 18 % at most (200x50x30).  Numbers
+    // nearer to those (2.4 %) choose shorter walks on small grids, which a membrane chain beside the pass
+    // pays for: 45x37x29 with a red cell 34.7 us a step at 1, 32.0 at 2.
     std::vector<TileShape> shape(n_inst);
     for (int k = 0; k < n_inst; k++)
         if (check[k].fits) shape[k] = tile_shape(check[k].g.nx, check[k].g.ny);
@@ -848,7 +853,8 @@ int plan_grid(lbfs_solver *s, const lbfs_mesh_desc *m, const GridMesh &gm) {
             longest = std::max(longest, even + 1.2);
         }
         const int on_sm = (int)std::ceil(blocks / 148.0);
-        const double t = on_sm <= per_sm ? longest * plane_time(on_sm)
+        const bool delayed = placed / kUniformThreads > 148 * per_sm;
+        const double t = on_sm <= per_sm ? longest * plane_time(on_sm) * (delayed ? 1.1 : 1.0)
                                          : planes / 148.0 * plane_time(per_sm) / per_sm + 0.35 * longest * plane_time(per_sm);
         if (t < best * (1 - 1e-9)) {
             best = t;
