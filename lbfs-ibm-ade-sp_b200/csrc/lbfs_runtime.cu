@@ -1421,12 +1421,14 @@ struct PhaseMark {
 // programmatic edge, which lets it be placed behind their last wave) and that
 // stream's last one, as without membranes.  With the membrane stream joined to
 // the handle's stream directly the update started only after the interior
-// faces had finished.  The spread of many membranes is long, though, and follows
-// the node forces at once (us per step, behind the faces / at once: 103.6 / 101.7
-// for 49 membranes on twelve grids, 378.5 / 379.9 for 16 at 128^3).
+// faces had finished.  On ensembles of many membranes, whose boundary faces are many
+// and whose spread is long, it follows the node forces at once (us per step, behind
+// the faces / at once: 104.1 / 102.2 for 49 membranes on twelve grids, 221.3 / 220.8
+// on 24; on one grid 276.2 / 284.3 for 64 at 96^3, 179.8 / 184.3 for 48 at 80^3).
 template <typename R> bool spread_with_faces(const lbfs_solver *s, const FluidArgs<R> &a) {
     const int K = a.axis_aligned ? s->flux_chunks : 1;
-    return s->n_membranes > 0 && s->n_membranes <= 32 && K <= 1 && (a.axis_aligned || a.flux_tiles) && !s->kernel_events;
+    const bool at_once = s->n_membranes > 32 && s->grids.size() > 1;
+    return s->n_membranes > 0 && !at_once && K <= 1 && (a.axis_aligned || a.flux_tiles) && !s->kernel_events;
 }
 //
 // after_k1 (may be null): enqueued right behind the gradient launch (the last
