@@ -1656,9 +1656,11 @@ template <typename R> int enqueue_step(lbfs_solver *s, bool visc_update, int *la
                 LBFS_CUDA(cudaEventRecord(s->ev_fork, s->stream));
                 LBFS_CUDA(cudaStreamWaitEvent(s->stream2, s->ev_fork, 0));
                 if ((rc = membranes())) return rc;
-                // (gradient blocks that the SMs hold at once take no one's place: 44.5 us a step without, 46.7
-                // with, on 64,000 imported cells)
-                if (s->nc > 2 * 148 * 256 && (rc = order_behind_advect(s, advect))) return rc;
+                // (where the gradients take more than two waves; us per step without / with: 48.7 / 52.7 on 48^3
+                // rectilinear cells with 642 nodes, 50.2 / 53.1 jittered with two such cells, 40.4 / 42.6 at 56^3
+                // FP32, 75.2 / 72.4 at 64^3 rectilinear)
+                const long long wave = 148LL * (a.tb_grad == 128 ? 5 * 128 : 512);
+                if (s->nc > 2 * wave && (rc = order_behind_advect(s, advect))) return rc;
                 rc = enqueue_k1_k2<R>(s, a, &n, spread_here);
             }
             if (rc) return rc;
