@@ -37,6 +37,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(ROOT, "lbfs-ibm-ade-sp_b200"))
 
 METRIC = "Mcell-updates/s"
+# FP64 lane instructions a cell of the fused pass (profiles/k_uniform_step_shear_rbc128_fp64.md: 740 at 128^3, 756 at
+# 64^3, where boundary faces are more)
+FP64_LANES_PER_CELL = 740
 IBM_NAMES = {"peskin4": "4-point Peskin IBM", "hat2": "2-point hat IBM"}
 
 
@@ -219,14 +222,14 @@ def algorithmic_bytes(mesh, phase, fp64=True):
         geo = 0 if axis_geometry_uniform(mesh) else 4 * R
         return ni * (8 + 4 * R + geo) + nb * (16 + 29 * R) + nc * (17 * R) + nb * (16 * R)
     if phase == "fluid_pass":
-        # the fused pass of uniform meshes.  Per cell: state in 4R, viscosity factor R, 1 / volume 8, the
-        # state kept 4R and the cell sums 32 out; per bc face: ids 8, geometry 12R, types/values 8 + 4R,
-        # record 9R, flux out 4R
-        return nc * (40 + 9 * R) + nb * (16 + 29 * R)
+        # the fused pass of uniform meshes, without what it hands to the update or keeps for later (cell
+        # sums, boundary fluxes, the kept state).  Per cell: state 4R, viscosity factor R; per bc face: ids
+        # 8, geometry 12R, types/values 8 + 4R, record 9R
+        return nc * (5 * R) + nb * (16 + 25 * R)
     if phase == "fluid_update":
-        # the update behind it.  Per cell: cell sums 32 and a byte in, volume 8, t1 in/out 64, state out
-        # 4R; per bc face: flux in 4R, the owner's face list 24
-        return nc * (105 + 4 * R) + nb * (24 + 4 * R)
+        # the update behind it, without what the pass handed over.  Per cell: t1 in/out 64, state out 4R,
+        # volume 8 unless one comes from the parameters; per bc face: the owner's face list 24
+        return nc * ((0 if cell_update_closed_forms(mesh)[1] else 8) + 64 + 4 * R) + nb * 24
     if phase == "gradients":
         # per cell: stencil 24, folded weights 18R (or their 3-bit codes, 4, on a mesh with at most 8
         # distinct weight vectors), state 4R, gradients out 12R;
@@ -832,7 +835,7 @@ def main():
     # roofline of the dominant fluid kernel (the membrane kernel overlaps them on a second stream).  On
     # uniform meshes gradients and fluxes are one kernel (no gradient phase is recorded)
     fused = phases["gradients"] == 0.0
-    kernels = ({"flux": ("fluid_pass", "k_uniform_step"), "update": ("fluid_update", "k_cell_update")} if fused else
+    kernels = ({"flux": ("fluid_pass", "k_uniform_step"), "update": ("fluid_update", "k_cell_update_fused")} if fused else
                {"gradients": ("gradients", "k_cell_gradients"), "flux": ("flux", "k_face_flux"),
                 "update": ("update", "k_cell_update")})
     fluid = {k: phases[k] for k in kernels}
@@ -846,6 +849,12 @@ def main():
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "peak_source": peak_kind,
                 "algorithmic_bytes_per_launch": alg, "launch_ms": fluid[dom],
                 "timing": "per-kernel CUDA events, second timed pass of K steps with K1 and K2 not pipelined"}
+    if kname == "k_uniform_step":  # issues FP64 instructions for most of its time: against that rate too
+        lanes = FP64_LANES_PER_CELL * mesh.n_cells / (fluid[dom] * 1e-3) / 1e9
+        lanes_peak = 148 * 64 * 1.965
+        roofline.update({"bound": "fp64", "fp64_lane_ginstr_s": lanes, "fp64_lane_peak_ginstr_s": lanes_peak,
+                         "fp64_frac": lanes / lanes_peak, "fp64_note": "FP64 lane instructions of the pass "
+                         "(profiles/k_uniform_step_shear_rbc128_fp64.md) over 64 lanes an SM and cycle, 148 SMs, 1965 MHz"})
     # every fluid kernel against the same HBM peak (algorithmic bytes / event-timed duration)
     kernel_roofline = {}
     for ph, (kind, kn) in kernels.items():
