@@ -696,8 +696,7 @@ bool grid_fits(lbfs_solver *s, const lbfs_mesh_desc *m, const lbfs_grid_desc &gd
                     }
                 }
             }
-    q.fits = true;
-    return true;
+    return q.fits = tile_shape(g.nx, g.ny).w > 0;
 }
 
 // The fused step's plan: which instances take the pass (each by itself, so that an instance of an
@@ -3164,6 +3163,7 @@ extern "C" int lbfs_checkpoint_load(lbfs_solver *s, const void *buf, uint64_t by
     unsigned int *flags = s->fp32 ? s->f32.flags : s->f64.flags;
     LBFS_CUDA(cudaMemcpy(flags, &h.flags, sizeof(unsigned int), cudaMemcpyHostToDevice));
     s->t = h.t;
+    s->prev_last = false;  // of another viscosity field
     return LBFS_OK;
 }
 
