@@ -278,8 +278,8 @@ int lbfs_status(lbfs_solver *s, uint32_t *flags);
 /* Timing with CUDA events, also inside the captured graph.  level 1: events
  * around each whole step; level 2: also around every kernel (or kernel group);
  * 0: off.  lbfs_get_phase_times writes the durations in ms of the last step:
- * [0] membrane kernels, [1] ghost+gradients (0 on uniform meshes, where they are
- * part of the face flux's pass), [2] face flux, [3] cell update,
+ * [0] membrane kernels, [1] ghost+gradients (0 on uniform FP64 meshes, where they
+ * are part of the face flux's pass), [2] face flux, [3] cell update,
  * [4] interior viscosity (0 when not launched or not level 2), and [5] the
  * whole step (first launch to last, on the solver's stream). */
 int lbfs_set_profiling(lbfs_solver *s, int32_t on);
@@ -310,9 +310,9 @@ typedef struct lbfs_launch_shape {
     int32_t spread_blocks;          /* grid of the IBM spread, 1 .. LBFS_MAX_SPREAD_BLOCKS */
     int32_t flux_chunks;            /* 1, 2, 4 or 8: gradients and interior-face fluxes of an axis-aligned
                                        mesh pipelined in that many chunks of cells on two streams
-                                       (0 = 1; meshes that do not allow it use 1).  Uniform meshes form
-                                       both in one kernel, whose launch this and the two block sizes
-                                       above do not change */
+                                       (0 = 1; meshes that do not allow it use 1).  Uniform FP64 meshes
+                                       form both in one kernel, whose launch this and the gradient and
+                                       flux block sizes do not change */
     int32_t membrane_cluster;       /* 8 or 16: a membrane's totals, spring and node forces as one
                                        thread-block cluster of that many CTAs; 0: three kernels.  It
                                        changes the summation order of V, A and MAD (rounding only) */

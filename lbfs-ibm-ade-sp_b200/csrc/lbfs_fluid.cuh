@@ -208,8 +208,8 @@ template <typename R> struct FluidArgs {
     R *grad;                     // [12*(nc+nb)] rho(x,y,z) u(x,y,z) v(x,y,z) w(x,y,z)
     // K1 geometry
     const int2 *stencil;         // [3*nc] (6 stencil entries per cell)
-    const LsRec<R> *ls;          // [nc] RHS and LHS^-1 (the adjoint's; null for FP32-bulk handles)
-    const LsW<R> *lsw;           // [nc] K1's folded weights
+    const LsRec<R> *ls;          // [nc] RHS and LHS^-1 (the adjoint's; null for FP32-bulk handles and with ls_coded)
+    const LsW<R> *lsw;           // [nc] K1's folded weights (null with lsw_code)
     // Meshes whose per-slot weight vectors W_q take at most 8 distinct values
     // (the generator's uniform meshes: +-1/(4 dx) along one axis, in a
     // per-cell order): each cell's six vectors as 3-bit indices into lsw_tab,
@@ -227,7 +227,7 @@ template <typename R> struct FluidArgs {
     const BcRec<R> *bc_rec;      // [nb]
     // K2 geometry
     const int2 *face_cells;      // [nf] owner, neighbour
-    const AxisFace<R> *axis_face;  // [ni] when axis_aligned
+    const AxisFace<R> *axis_face;  // [ni] when axis_aligned (null with axis_uniform)
     // axis_uniform: every interior face of an axis has the same geometry (the
     // generator's uniform meshes, also across ensemble instances of one
     // spacing), checked bit for bit at create; the interior-face kernels then

@@ -1,10 +1,10 @@
 // Host runtime behind the C ABI of include/lbfs_b200.h.
 //
 // One handle = one solver instance on one GPU: mesh geometry and membranes are
-// uploaded once, the state stays resident in HBM, and each time step is four
-// kernels (membrane kernel on a forked stream, overlapping the gradient and
-// face-flux kernels, then the cell update), optionally replayed from a CUDA
-// graph.  This replaces gpu_solver::General_Purpose_Solver_mk_i's set-up
+// uploaded once, the state stays resident in HBM, and each time step is a few
+// kernels (the membrane kernels on a forked stream, beside the fluid's pass or its
+// gradient and face-flux kernels, then the cell update), optionally replayed from
+// a CUDA graph.  This replaces gpu_solver::General_Purpose_Solver_mk_i's set-up
 // (Solver_gpu.cu:178-746) and loop body (Solver_gpu.cu:749-1046), which issue
 // 20-30 synchronising launches per step on managed memory.
 #include <cuda_runtime.h>
@@ -1355,8 +1355,8 @@ void set_chunks(lbfs_solver *s, int K) {
     const bool aa = s->fp32 ? s->f32.axis_aligned : s->f64.axis_aligned;
     const int tb = s->fp32 ? (aa ? s->f32.tb_flux : s->f32.tb_gen) : (aa ? s->f64.tb_flux : s->f64.tb_gen);
     const std::vector<int> &mx = s->tile_maxnb[tb == 64 ? 0 : (tb == 256 ? 2 : 1)];
-    // fused step: fluid pass and update; else gradients and interior fluxes (K each), boundary fluxes,
-    // update; membrane kernels; CFL
+    // fused step: fluid pass and update (and gradients, interior and boundary fluxes of instances beside it);
+    // else gradients and interior fluxes (K each), boundary fluxes, update; membrane kernels; CFL
     s->launches_per_step = (s->fused ? (s->rest.any ? 5 : 2) : 2 * K + 2) + (s->n_membranes > 0 ? (s->ma.force_cluster > 0 ? 3 : 6) : 0) + (dynamic_dt(s->params) ? 1 : 0);
     s->chunk_cell.assign(K + 1, 0);
     s->chunk_faces.assign(K, FaceRanges{});
