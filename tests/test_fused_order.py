@@ -112,3 +112,49 @@ def test_instances_of_different_meshes_equal_handles_of_their_own(kinds):
         assert np.array_equal(ghost[b0:b0 + m.n_bc], own[3]), k
         assert np.array_equal(grad[e.n_cells + b0:e.n_cells + b0 + m.n_bc], own[2][m.n_cells:]), k
         b0 += m.n_bc
+
+
+def test_a_mixed_handle_through_the_other_entry_points(monkeypatch):
+    """Uniform grids of two spacings and a rectilinear one in a handle: the device loop, eager steps, several
+    steps a graph, a restore and tuning leave the states of single graph steps; the adjoint is that of a
+    handle on the separate kernels (which it records with)."""
+    meshes = [_box((13, 17, 12), 2.0), _plateau((14, 12, 10)), _box((12, 11, 15), 1.5)]
+    e = concatenate(meshes)
+    state = [np.concatenate(q) for q in zip(*(_state(m.n_cells, 40 + k) for k, m in enumerate(meshes)))]
+
+    def handle():
+        s = GpuSolver(e, PARAMS)
+        s.set_state(*state)
+        assert s.launches_per_step() == 5  # the pass, three kernels beside it, the update
+        return s
+
+    def same(s, t):
+        return all(np.array_equal(a, b) for a, b in zip(s.state(), t.state()))
+
+    with handle() as ref, handle() as s, handle() as t:
+        for _ in range(6):
+            ref.step(1, graph=True)
+        assert s.step_until(6, 0.0)[0] == 6 and same(s, ref)
+        t.step(3)
+        blob = t.checkpoint()
+        t.step(9, graph=True)
+        t.autotune(reps=3)
+        t.restore(blob)
+        t.step(3, graph=True)
+        assert same(t, ref)
+        for _ in range(300):
+            s.step(2, graph=True)
+        for _ in range(600):
+            ref.step(1, graph=True)
+        assert same(s, ref) and s.status() == 0
+    weights = np.random.default_rng(2).uniform(-1, 1, 3 * e.n_cells)
+    out = []
+    for separate in (False, True):
+        if separate:
+            monkeypatch.setenv("LBFS_SEPARATE_KERNELS", "1")
+        with GpuSolver(e, PARAMS) as s:
+            s.set_state(*state)
+            J, grad, _ = s.adjoint(8, 4, weights=weights)
+            out.append((J, grad, s.state(), s.field(_abi.LBFS_FIELD_GRADIENTS)))
+    assert out[0][:2] == out[1][:2]
+    assert all(np.array_equal(a, b) for a, b in zip(out[0][2], out[1][2])) and np.array_equal(out[0][3], out[1][3])
